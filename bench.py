@@ -624,7 +624,7 @@ def decode_bench(world, rank, dev, dtype, batches=(1, 16, 64), context=2048, ste
     out = {"model": "qwen3-8b-arch w4 g128 random init", "tp": world, "context": context,
            "allreduce_variants": "nccl = NCCL after each row-parallel linear; peer = nqb200_gemm_allreduce "
                                  "(reduced over peer memory by the kernel that finishes the GEMM)",
-           "attention": "flash_attn paged" if eng.paged_attention is not None else "sdpa over gathered pages", "points": []}
+           "attention": "nqb200_decode_attention over the pages", "points": []}
     g = torch.Generator().manual_seed(1)
     comm = None
     if world > 1:

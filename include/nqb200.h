@@ -179,6 +179,15 @@ int nqb200_qknorm_rope_kv(void* qkv, const void* q_weight, const void* k_weight,
                           int64_t num_q_heads, int64_t num_kv_heads, int64_t head_dim, int64_t row_stride, float eps,
                           int dtype, void* stream);
 
+/* One decode step's attention over the paged cache, in one launch: what nqb200_qknorm_rope_kv does to the step's token of
+ * every sequence (qkv itself is left as it is), then softmax(scale q k) v over the ctx[b] keys of sequence b, the step's own
+ * among them.  Block i of sequence b is table[b][i]; slots[b] is the row of the step's token, positions[b] its position.
+ * Heads of 128; row_stride (elements) a multiple of 8; out is [batch, num_q_heads * 128].  No counterpart in the reference. */
+int nqb200_decode_attention(const void* qkv, int64_t row_stride, const void* q_weight, const void* k_weight, const float* cos_sin,
+                            const int64_t* positions, const int64_t* slots, void* k_cache, void* v_cache, const int32_t* table,
+                            const int32_t* ctx, int64_t table_width, int64_t block_size, void* out, int64_t batch, int64_t num_q_heads,
+                            int64_t num_kv_heads, int64_t head_dim, float scale, float eps, int dtype, void* stream);
+
 /* One-shot all-reduce (sum) over NVLink peer memory for the small [M, N] partial results of a
  * row-parallel linear.  No counterpart in the reference (it has no distributed code).
  * Set-up, once: every rank calls nqb200_comm_alloc (a cudaMalloc'd, zeroed buffer: a header of

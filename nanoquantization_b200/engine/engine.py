@@ -5,9 +5,10 @@ The reference has none of this (its only execution is a full-sequence forward fo
 models/qwen3_quantized.py:326-341); it exists so that models are measured where they are used: prefill of batched
 prompts (whole or in portions) and greedy decode steps over a cache.  A model states what it keeps per layer run
 (``cache_layout()``) and runs one step on a ``StepBatch`` (``forward_step``).  For a model that delegates attention
-(Qwen3) the engine supplies it: PyTorch's scaled_dot_product_attention per prompt at prefill; at decode flash_attn's
-paged-KV kernel when that library loads on this GPU, else scaled_dot_product_attention over the gathered pages of
-each sequence.  Other models bring kernels that read the cache and the states themselves.
+(Qwen3) the engine supplies it: PyTorch's scaled_dot_product_attention per prompt at prefill; at decode the model's own
+kernel over the pages for heads of 128, else flash_attn's when that library loads on this GPU, else
+scaled_dot_product_attention over the gathered pages of each sequence.  Other models bring kernels that read the cache and
+the states themselves.
 
 Layout: per layer run two tensors ``[num_blocks, block_size, kv_heads, head_dim]``; a sequence owns a list of blocks;
 ``row = block * block_size + offset``.  Blocks that no later query can reach (every layer attends inside chunks) are
@@ -126,6 +127,8 @@ class LayerStep:
         self.engine, self.batch, self.decode = engine, batch, decode
         self.k_cache, self.v_cache, self.state = engine.cache.k[run], engine.cache.v[run], engine.states.states[run]
         self.kv_target = (self.k_cache, self.v_cache, batch.rows)
+        # what a kernel that looks up the pages itself needs for a decode step (heads of 128; other sizes call this object)
+        self.paged_decode = (self.k_cache, self.v_cache, batch) if decode and self.k_cache is not None and self.k_cache.is_cuda else None
 
     def __call__(self, q, k, v, stored=False):
         if not stored:
@@ -271,7 +274,9 @@ class LLMEngine:
         self.blocks = BlockManager(num_blocks, block_size)
         self.scheduler = Scheduler(self.blocks, max_batch, max_prefill_tokens, prefill_portion, self.states)
         self.use_cuda_graph = use_cuda_graph
-        self.paged_attention = self._probe_flash_attn() if model.delegates_attention and block_size % 256 == 0 else None
+        self.paged_attention = None
+        if model.delegates_attention and block_size % 256 == 0 and self.layout.kv[0].head_dim != 128:
+            self.paged_attention = self._probe_flash_attn()
         self._graphs: dict[tuple[int, int], tuple] = {}
         self._warm_stream = None  # one side stream for every graph warm-up (scratch buffers are kept per stream)
         self._next_id = 0

@@ -157,7 +157,8 @@ class Qwen3QuantizedAttention(nn.Module):
                        residual: Optional[torch.Tensor] = None):
         """``x`` is ``[T, hidden]``; ``attend(q, k, v)`` stores k, v in its cache and returns ``[T, Hq, D]``
         (called with ``stored=True`` when this method already stored them through ``attend.kv_target``).
-        One launch for q/k/v (when fused), one for QK-norm + rotary embedding."""
+        One launch for q/k/v (when fused), one for QK-norm + rotary embedding; where ``attend.paged_decode`` gives the
+        caches of a decode step, that launch does the attention too."""
         T = x.shape[0]
         nq, nk = self.num_heads * self.head_dim, self.num_kv_heads * self.head_dim
         if norm is not None:  # x is the residual stream; its RMSNorm is taken inside the linear
@@ -167,6 +168,12 @@ class Qwen3QuantizedAttention(nn.Module):
         else:
             qkv = torch.cat([self.q_proj(x), self.k_proj(x), self.v_proj(x)], dim=-1)
         stored = False
+        paged = getattr(attend, "paged_decode", None) if self.head_dim == 128 else None
+        if paged is not None:  # a decode step over a paged cache: norm, rotation, K/V store and attention in one launch
+            k_cache, v_cache, batch = paged
+            o = fused.decode_attention(qkv, self.q_norm.weight, self.k_norm.weight, self.rope.cos_sin_cache, positions, self.num_heads,
+                                       self.num_kv_heads, self.head_dim, self.q_norm.eps, k_cache, v_cache, batch)
+            return self.o_proj.forward_residual(o, residual) if residual is not None else self.o_proj(o)
         if self.head_dim == 128:
             # an attend() that exposes its cache (k_cache, v_cache, slots) gets k and v stored by this launch
             kv_target = getattr(attend, "kv_target", None)
