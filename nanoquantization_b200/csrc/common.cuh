@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <stddef.h>
+#include <atomic>
 #include "nqb200.h"
 
 namespace nqb200 {
@@ -34,6 +35,22 @@ static inline int launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 bl
   cfg.attrs = attr; cfg.numAttrs = 1;
   if (cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...) != cudaSuccess) { cudaGetLastError(); return NQB200_ERR_LAUNCH; }
   return NQB200_OK;
+}
+
+// For kernels that stream weights or states through registers: the loads under way need room in the part of an SM's memory
+// that is not shared memory, and an SM that a kernel with much shared memory has left keeps its split until a kernel that
+// states another one arrives.  States a quarter as shared memory (57 KB: enough for all resident blocks of these kernels), once
+// per kernel and device.  A hint: a call is right without it.  bf16 linears of 16 tokens behind an attention with 3 x 73 KB
+// per SM: 4096 x 8192 30 us without and 14 us with it, 4096 x 12288 44 and 22, 24576 x 4096 with its gate 53 and 44.
+template <auto Kernel>
+static inline void prefer_loads() {
+  static std::atomic<uint64_t> done{0};
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) { cudaGetLastError(); return; }
+  const uint64_t bit = 1ull << dev;
+  if (done.load(std::memory_order_relaxed) & bit) return;
+  if (cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 25) != cudaSuccess) cudaGetLastError();
+  done.fetch_or(bit, std::memory_order_relaxed);
 }
 
 // How the split-K decode kernel tiles a problem; the same plan sizes the workspace.

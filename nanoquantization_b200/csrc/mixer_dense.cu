@@ -127,7 +127,12 @@ static int launch_dense(const DenseArgs& p, cudaStream_t st) {
   if (!p.x || !p.w || !p.out) return NQB200_ERR_NULL_POINTER;
   if (!aligned16(p.x) || !aligned16(p.w)) return NQB200_ERR_MISALIGNED;
   const dim3 grid((unsigned)((p.N + 15) / 16)), block(256);
-  return p.M <= 8 ? launch_overlapped(dense_decode_kernel<MODE, 1>, grid, block, 0, st, p) : launch_overlapped(dense_decode_kernel<MODE, 2>, grid, block, 0, st, p);
+  if (p.M <= 8) {
+    prefer_loads<dense_decode_kernel<MODE, 1>>();
+    return launch_overlapped(dense_decode_kernel<MODE, 1>, grid, block, 0, st, p);
+  }
+  prefer_loads<dense_decode_kernel<MODE, 2>>();
+  return launch_overlapped(dense_decode_kernel<MODE, 2>, grid, block, 0, st, p);
 }
 
 }  // namespace nqb200

@@ -135,13 +135,15 @@ static MoeDevice device_args(const MoeArgs& a) {
 }
 
 bool moe_decode_supports(int64_t tokens, int64_t N, int64_t K) { return tokens <= kMoeDecodeTokens && K % 8 == 0 && N > 0; }
-int moe_decode(const MoeArgs& a) {
-  const MoeDevice p = device_args(a);
+template <typename O, int MT>
+static int launch_moe_decode(const MoeArgs& a) {
   const int most = a.tokens * a.top < a.experts ? a.tokens * a.top : a.experts;
-  const dim3 grid((unsigned)((a.N + 15) / 16), (unsigned)most), block(256);
-  if (a.out_dtype == NQB200_F32)
-    return a.tokens <= 8 ? launch_overlapped(moe_decode_kernel<float, 1>, grid, block, 0, a.stream, p) : launch_overlapped(moe_decode_kernel<float, 2>, grid, block, 0, a.stream, p);
-  return a.tokens <= 8 ? launch_overlapped(moe_decode_kernel<bf16, 1>, grid, block, 0, a.stream, p) : launch_overlapped(moe_decode_kernel<bf16, 2>, grid, block, 0, a.stream, p);
+  prefer_loads<moe_decode_kernel<O, MT>>();
+  return launch_overlapped(moe_decode_kernel<O, MT>, dim3((unsigned)((a.N + 15) / 16), (unsigned)most), dim3(256), 0, a.stream, device_args(a));
+}
+int moe_decode(const MoeArgs& a) {
+  if (a.out_dtype == NQB200_F32) return a.tokens <= 8 ? launch_moe_decode<float, 1>(a) : launch_moe_decode<float, 2>(a);
+  return a.tokens <= 8 ? launch_moe_decode<bf16, 1>(a) : launch_moe_decode<bf16, 2>(a);
 }
 
 static int moe_simple(const MoeArgs& a) {
