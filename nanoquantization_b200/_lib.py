@@ -267,6 +267,11 @@ def require_cuda(*tensors: torch.Tensor) -> torch.device:
 _supported: dict[int, bool] = {}
 
 
+def is_b200(device: int) -> bool:
+    """Whether the device has been found to be supported."""
+    return _supported.get(device, False)
+
+
 def require_b200(dev: torch.device) -> None:
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
     ok = _supported.get(idx)
@@ -281,19 +286,23 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+def stream_of(device: int) -> int:
+    """The device's current stream, without building a ``torch.cuda.Stream`` for it."""
+    return torch._C._cuda_getCurrentRawStream(device)
+
+
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 
 
-def workspace(dev: torch.device, nbytes: int) -> torch.Tensor | None:
+def workspace(device: int, stream: int, nbytes: int) -> torch.Tensor | None:
     """Zero-filled scratch, one per (device, stream), grown on demand.  The
     kernels leave it zero-filled again, so it is only cleared when created."""
     if nbytes == 0:
         return None
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(), stream_ptr())
-    ws = _workspaces.get(key)
+    ws = _workspaces.get((device, stream))
     if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)
-        _workspaces[key] = ws
+        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=f"cuda:{device}")
+        _workspaces[device, stream] = ws
     return ws
 
 

@@ -99,8 +99,13 @@ def _w4a16(x: torch.Tensor, qweight: torch.Tensor, qscales: torch.Tensor, qzeros
     M, K = x.shape
     N = qweight.shape[1] * 8
     group_size = K // qscales.shape[0]
-    dev = _lib.require_cuda(x, qweight, qscales, qzeros)
-    _lib.require_b200(dev)
+    # A call of one token is 7 us on the device: what the host does ahead of the launch is most of it, so that the checks
+    # of an ordinary call are integers compared.  One token, 4096 x 4096: 31 -> 14 us a call.
+    device = x.get_device()
+    if device < 0 or qweight.get_device() != device or qscales.get_device() != device or qzeros.get_device() != device:
+        _lib.require_cuda(x, qweight, qscales, qzeros)  # raises, and says why
+    if not _lib.is_b200(device):
+        _lib.require_b200(x.device)
     dtype = qscales.dtype
     code = _lib.dtype_code(dtype)
     if x.dtype != dtype:  # the reference casts x to the output dtype (gemm.py:259)
@@ -112,14 +117,15 @@ def _w4a16(x: torch.Tensor, qweight: torch.Tensor, qscales: torch.Tensor, qzeros
         bias_ptr, bias_code = bias.data_ptr(), _lib.dtype_code(bias.dtype)
     n_out = N // 2 if silu_mul else N
     if out is None:
-        out = torch.empty(M, n_out, dtype=dtype, device=dev)
+        out = torch.empty((M, n_out), dtype=dtype, device=x.device)
     else:
         assert out.shape == (M, n_out) and out.dtype == dtype and out.is_contiguous()
     if M == 0:
         return out
     lib = _lib.load()
     entry = lib.nqb200_gemm_gate_up_silu if silu_mul else lib.nqb200_gemm
-    tail = (_lib.stream_ptr(),)
+    stream = _lib.stream_of(device)
+    tail = (stream,)
     ssq_out = None
     if norm is not None or residual is not None:
         f = _lib.DecodeFusion()
@@ -131,7 +137,7 @@ def _w4a16(x: torch.Tensor, qweight: torch.Tensor, qscales: torch.Tensor, qzeros
         if residual is not None:
             assert residual.shape == (M, N) and residual.dtype == dtype and residual.is_contiguous()
             tile = lib.nqb200_decode_tile_columns()
-            ssq_out = torch.empty(M, (N + tile - 1) // tile, dtype=torch.float32, device=dev)
+            ssq_out = torch.empty(M, (N + tile - 1) // tile, dtype=torch.float32, device=x.device)
             f.residual_in, f.ssq_out = residual.data_ptr(), ssq_out.data_ptr()
         entry = lib.nqb200_gemm_decode_fused
         tail = (ctypes.byref(f),) + (tuple(peer) if peer is not None else (None, 0, 0, 0, 0)) + tail
@@ -142,12 +148,12 @@ def _w4a16(x: torch.Tensor, qweight: torch.Tensor, qscales: torch.Tensor, qzeros
     nbytes = _ws_bytes_cache.get(key)
     if nbytes is None:
         nbytes = _ws_bytes_cache[key] = lib.nqb200_gemm_workspace_bytes(M, N, K, group_size, code)
-    other_device = dev.index is not None and dev.index != torch.cuda.current_device()
+    prev = torch._C._cuda_getDevice()
+    other_device = device != prev
     if other_device:
-        prev = torch.cuda.current_device()
-        torch.cuda.set_device(dev)
+        torch.cuda.set_device(device)
     try:
-        ws = _lib.workspace(dev, nbytes)
+        ws = _lib.workspace(device, stream, nbytes)
         status = entry(x.data_ptr(), qweight.data_ptr(), qscales.data_ptr(), qzeros.data_ptr(),
                        bias_ptr, bias_code, out.data_ptr(), M, N, K, group_size, code,
                        ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0, *tail)
@@ -298,15 +304,16 @@ class WQLinear_GEMM(nn.Module):
                                                         _lib.dtype_code(output_dtype), _lib.stream_ptr()))
         return q
 
-    @torch.no_grad()
     def forward(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """``[..., K] -> [..., N]``.  The reference switches kernels at 256 tokens
         (gemm.py:558-564); here one library call picks the kernel by M, and the
         bias add (gemm.py:565-566) is fused into it."""
+        # the kernel writes an output that autograd knows nothing of, whether or not gradients are on
+        if x.dim() == 2:
+            return _w4a16(x, self.qweight, self.qscales, self.qzeros, self.bias, out)
         out_shape = x.shape[:-1] + (self.out_features,)
         x = x.reshape(-1, x.shape[-1])
-        out = _w4a16(x, self.qweight, self.qscales, self.qzeros, self.bias, out)
-        return out.reshape(out_shape)
+        return _w4a16(x, self.qweight, self.qscales, self.qzeros, self.bias, out).reshape(out_shape)
 
     @torch.no_grad()
     def forward_silu_mul(self, x: torch.Tensor) -> torch.Tensor:
