@@ -192,6 +192,107 @@ __global__ void __launch_bounds__(256, 4) norm_rope_vec_kernel(bf16* proj, bf16*
   }
 }
 
+// The same where the whole head turns and is 16 L elements long: L lanes per head, each with piece c of the lower and of the
+// upper half, which are partners where pairs lie half a head apart, so that nothing but the norm's sum crosses lanes and a
+// warp works on 32 / L heads at once (the kernel above spends its time on instructions: half of its lanes idle at 128, eight
+// shuffles a head).  8192 tokens, 32 + 8 heads of
+// 128, with the cache: 96 us by the kernel that took it before, element by element, 42 us so; 5000 tokens with norms and
+// neighbouring pairs: 61 and 27 us.
+template <bool NEIGHBOURS, int L>
+__global__ void __launch_bounds__(256) rope_full_kernel(bf16* proj, bf16* k_cache, bf16* v_cache, const nqb200_rope r, const nqb200_batch bt, int64_t stride,
+                                                        int q_off, int k_off, int v_off, int span) {
+  constexpr int DIM = 16 * L, HALF = 8 * L, PER = 256 / L, U = 2;   // PER: heads of a pass; U passes under way
+  extern __shared__ __align__(16) float cs[];  // [DIM] q_norm, [DIM] k_norm, [span][HALF] cos, [span][HALF] sin
+  __shared__ size_t slot[kRopeSpan];
+  const int cos_at = 2 * DIM, sin_at = cos_at + span * HALF;
+  grid_launch_dependents();
+  if (r.q_norm)
+    for (int e = threadIdx.x; e < DIM; e += 256) { cs[e] = r.q_norm[e]; cs[DIM + e] = r.k_norm[e]; }
+  grid_dependency_wait();
+  const int b = blockIdx.y, t0 = bt.cu[b], n = bt.cu[b + 1] - t0, first = blockIdx.x * span;
+  if (first >= n) return;
+  const int tokens = min(span, n - first), heads = r.heads + r.kv_heads, items = tokens * heads;
+  bf16* rows = proj + (size_t)(t0 + first) * stride;
+  const int c = threadIdx.x % L, own = threadIdx.x / L;
+  auto token_of = [&](int it) { return (it >= heads) + (it >= 2 * heads) + (it >= 3 * heads); };
+  auto place = [&](int tk, int hd) {
+    return reinterpret_cast<uint4*>(rows + (size_t)tk * stride + (hd < r.heads ? q_off + hd * DIM : k_off + (hd - r.heads) * DIM)) + c;
+  };
+  uint4 lo[U], hi[U], nlo[U], nhi[U];
+  auto request = [&](int i0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int it = min(i0 + u * PER + own, items - 1), tk = token_of(it);
+      const uint4* p = place(tk, it - tk * heads);
+      nlo[u] = p[0];
+      nhi[u] = p[L];
+    }
+  };
+  request(0);
+  const int p0 = bt.pos0[b] + first;
+  for (int e = threadIdx.x; e < tokens * HALF; e += 256) {
+    const int tk = e / HALF, f = e % HALF;
+    sincosf((float)(p0 + tk) * r.inv_freq[f], &cs[sin_at + e], &cs[cos_at + e]);
+  }
+  if (k_cache && (int)threadIdx.x < tokens) slot[threadIdx.x] = kv_row(bt, b, p0 + threadIdx.x);
+  __syncthreads();
+  for (int i0 = 0; i0 < items; i0 += U * PER) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) { lo[u] = nlo[u]; hi[u] = nhi[u]; }
+    if (i0 + U * PER < items) request(i0 + U * PER);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int at = i0 + u * PER + own, it = min(at, items - 1), tk = token_of(it), hd = it - tk * heads;
+      float x[8], z[8];
+      unpack8(lo[u], x);
+      unpack8(hi[u], z);
+      if (r.q_norm) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += x[e] * x[e] + z[e] * z[e];
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+        const float inv = 1.f / sqrtf(ss / (float)DIM + r.eps);
+        const float4* w = reinterpret_cast<const float4*>(cs + (hd < r.heads ? 0 : DIM)) + 2 * c;
+        const float4 w0 = w[0], w1 = w[1], w2 = w[HALF / 4], w3 = w[HALF / 4 + 1];
+        const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w}, wh[8] = {w2.x, w2.y, w2.z, w2.w, w3.x, w3.y, w3.z, w3.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { x[e] = x[e] * inv * wl[e]; z[e] = z[e] * inv * wh[e]; }
+      }
+      const float4 *cp = reinterpret_cast<const float4*>(cs + cos_at + tk * HALF), *sp = reinterpret_cast<const float4*>(cs + sin_at + tk * HALF);
+      const int a0 = NEIGHBOURS ? c : 2 * c, a1 = NEIGHBOURS ? HALF / 8 + c : 2 * c + 1;
+      const float4 c0 = cp[a0], c1 = cp[a1], s0 = sp[a0], s1 = sp[a1];
+      const float cv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      float yx[8], yz[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        if (NEIGHBOURS) {   // angles 4c .. 4c + 3 turn the lower piece, HALF / 2 + 4c .. the upper one
+          const int f = e >> 1;
+          const float xo = x[e ^ 1], zo = z[e ^ 1];
+          yx[e] = x[e] * cv[f] + (e & 1 ? xo : -xo) * sv[f];
+          yz[e] = z[e] * cv[4 + f] + (e & 1 ? zo : -zo) * sv[4 + f];
+        } else {
+          yx[e] = x[e] * cv[e] - z[e] * sv[e];
+          yz[e] = z[e] * cv[e] + x[e] * sv[e];
+        }
+      }
+      if (at < items) {
+        uint4* dst = hd < r.heads || !k_cache ? place(tk, hd) : reinterpret_cast<uint4*>(k_cache + (slot[tk] * r.kv_heads + (hd - r.heads)) * DIM) + c;
+        dst[0] = pack8(yx);
+        dst[L] = pack8(yz);
+      }
+    }
+  }
+  if (k_cache) {
+    const int per = r.kv_heads * r.vdim / 8;
+    for (int e = threadIdx.x; e < tokens * per; e += 256) {
+      const int tk = e / per, q = e - tk * per;
+      reinterpret_cast<uint4*>(v_cache + slot[tk] * r.kv_heads * r.vdim)[q] = reinterpret_cast<const uint4*>(rows + (size_t)tk * stride + v_off)[q];
+    }
+  }
+}
+
+
 constexpr int kSimpleKeys = 128;   // keys per pass = threads
 constexpr int kSimpleVCols = 8;    // value columns per thread at most: vdim <= 1024
 
@@ -268,6 +369,27 @@ __global__ void __launch_bounds__(kSimpleKeys) attention_simple_kernel(const T* 
 
 using namespace nqb200;
 
+// bf16 heads in pieces of 8, where sizes and addresses allow it.
+static bool rope_pieces(const void* proj, const void* k_cache, const void* v_cache, const nqb200_rope* r, int64_t stride, int64_t q_off, int64_t k_off,
+                        int64_t v_off, int dtype) {
+  return dtype == NQB200_BF16 && r->dim % 8 == 0 && r->dim <= 256 && r->rot % (r->interleaved ? 8 : 16) == 0 && stride % 8 == 0 && q_off % 8 == 0 &&
+         k_off % 8 == 0 && aligned16(proj) && (!r->q_norm || r->k_norm) && (r->q_norm || !r->k_norm) &&
+         (!k_cache || (aligned16(k_cache) && aligned16(v_cache) && r->vdim % 8 == 0 && v_off % 8 == 0));
+}
+static int launch_rope_pieces(void* proj, void* k_cache, void* v_cache, const nqb200_rope* r, const nqb200_batch* b, int64_t stride, int64_t q_off,
+                              int64_t k_off, int64_t v_off, cudaStream_t s) {
+  auto kernel = r->interleaved ? norm_rope_vec_kernel<true> : norm_rope_vec_kernel<false>;
+  if (r->rot == r->dim) {
+    if (r->dim == 64) kernel = r->interleaved ? rope_full_kernel<true, 4> : rope_full_kernel<false, 4>;
+    if (r->dim == 128) kernel = r->interleaved ? rope_full_kernel<true, 8> : rope_full_kernel<false, 8>;
+    if (r->dim == 256) kernel = r->interleaved ? rope_full_kernel<true, 16> : rope_full_kernel<false, 16>;
+  }
+  const int span = b->max_len >= 4 * kNumSMs ? kRopeSpan : 1;
+  return launch_overlapped(kernel, dim3((unsigned)((b->max_len + span - 1) / span), (unsigned)b->batch), dim3(256),
+                           (size_t)(2 * r->dim + span * r->rot) * sizeof(float), s, (bf16*)proj, (bf16*)k_cache, (bf16*)v_cache, *r, *b, stride, (int)q_off,
+                           (int)k_off, (int)v_off, span);
+}
+
 extern "C" int nqb200_rope_store(void* proj, void* k_cache, void* v_cache, const float* inv_freq, const nqb200_batch* b, int64_t stride,
                                  int64_t q_off, int64_t k_off, int64_t v_off, int64_t heads, int64_t kv_heads, int64_t dim, int64_t vdim,
                                  int64_t rot, int dtype, void* stream) {
@@ -277,6 +399,11 @@ extern "C" int nqb200_rope_store(void* proj, void* k_cache, void* v_cache, const
   if (!mixer_dtype(dtype)) return NQB200_ERR_BAD_DTYPE;
   if (b->tokens == 0) return NQB200_OK;
   if (!proj || !k_cache || !v_cache || (rot > 0 && !inv_freq)) return NQB200_ERR_NULL_POINTER;
+  if (heads <= INT32_MAX / 256 && kv_heads <= INT32_MAX / 256 && dim <= 256 && vdim <= INT32_MAX) {
+    const nqb200_rope r = {(int32_t)heads, (int32_t)kv_heads, (int32_t)dim, (int32_t)vdim, (int32_t)rot, 0, inv_freq, nullptr, nullptr, 0.f};
+    if (rope_pieces(proj, k_cache, v_cache, &r, stride, q_off, k_off, v_off, dtype))
+      return launch_rope_pieces(proj, k_cache, v_cache, &r, b, stride, q_off, k_off, v_off, (cudaStream_t)stream);
+  }
   const dim3 grid((unsigned)b->max_len, (unsigned)b->batch), block(256);
   const size_t smem = (size_t)rot * sizeof(float);
 #define NQB200_ROPE(T)                                                                                                                   \
@@ -300,15 +427,8 @@ extern "C" int nqb200_norm_rope(void* proj, void* k_cache, void* v_cache, const 
   const dim3 grid((unsigned)b->max_len, (unsigned)b->batch), block(256);
   const size_t smem = (size_t)r->rot * sizeof(float);
   cudaStream_t s = (cudaStream_t)stream;
-  const bool pieces = dtype == NQB200_BF16 && r->dim % 8 == 0 && r->dim <= 256 && r->rot % (r->interleaved ? 8 : 16) == 0 && stride % 8 == 0 && q_off % 8 == 0 &&
-                      k_off % 8 == 0 && aligned16(proj) && (!r->q_norm || r->k_norm) && (r->q_norm || !r->k_norm) &&
-                      (!k_cache || (aligned16(k_cache) && aligned16(v_cache) && r->vdim % 8 == 0 && v_off % 8 == 0));
-  if (pieces) {
-    auto kernel = r->interleaved ? norm_rope_vec_kernel<true> : norm_rope_vec_kernel<false>;
-    const int span = b->max_len >= 4 * kNumSMs ? kRopeSpan : 1;
-    return launch_overlapped(kernel, dim3((unsigned)((b->max_len + span - 1) / span), (unsigned)b->batch), block, (size_t)(2 * r->dim + span * r->rot) * sizeof(float), s,
-                             (bf16*)proj, (bf16*)k_cache, (bf16*)v_cache, *r, *b, stride, (int)q_off, (int)k_off, (int)v_off, span);
-  }
+  if (rope_pieces(proj, k_cache, v_cache, r, stride, q_off, k_off, v_off, dtype))
+    return launch_rope_pieces(proj, k_cache, v_cache, r, b, stride, q_off, k_off, v_off, s);
   if (dtype == NQB200_F32)
     return launch_overlapped(norm_rope_kernel<float>, grid, block, smem, s, (float*)proj, (float*)k_cache, (float*)v_cache, *r, *b, stride,
                              (int)q_off, (int)k_off, (int)v_off);

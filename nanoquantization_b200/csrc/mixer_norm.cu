@@ -114,8 +114,33 @@ __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(
 __device__ __forceinline__ float4 scale4(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
 __device__ __forceinline__ void fma4(float4& d, float4 a, float4 b) { d.x += a.x * b.x; d.y += a.y * b.y; d.z += a.z * b.z; d.w += a.w * b.w; }
 
+// stream_add in pieces of four.  8192 rows of 4096 from a bfloat16 table: 74 us element by element, 36 us so;
+// 16 rows 10 and 3 us.
+template <typename T>
+__global__ void __launch_bounds__(256) stream_add_vec_kernel(float* __restrict__ x, const int64_t* __restrict__ ids, const T* __restrict__ embed,
+                                                             const float* __restrict__ step, int accumulate, int width) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  float* row = x + (size_t)blockIdx.x * width;
+  const T* e = ids ? embed + (size_t)ids[blockIdx.x] * width : nullptr;
+  for (int c0 = threadIdx.x * 4; c0 < width; c0 += 4096) {
+    float4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + 1024 * j;
+      v[j] = accumulate && c < width ? ld4(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (e && c < width) { const float4 a = load4(e + c); v[j].x += a.x; v[j].y += a.y; v[j].z += a.z; v[j].w += a.w; }
+      if (step && c < width) { const float4 a = ld4(step + c); v[j].x += a.x; v[j].y += a.y; v[j].z += a.z; v[j].w += a.w; }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c0 + 1024 * j < width) *reinterpret_cast<float4*>(row + c0 + 1024 * j) = v[j];
+  }
+}
+
 // The same for widths that are multiples of 4 and short filters: float4 accesses, and the last taps - 1 rows of h
-// stay in registers while a thread walks down the tile's tokens.
+// stay in registers while a thread walks down the tile's tokens.  Bound by memory, so both passes over x (the second comes
+// from L2) keep eight loads of a thread under way.  8192 x 4096, four taps, bfloat16: 88 us with four, 80 with eight (2.5 TB/s).
 constexpr int kConvTile = 16;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __restrict__ x, const float* __restrict__ weight,
@@ -134,9 +159,12 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __re
     if (tok < 0 || tok >= n) continue;
     const float* row = x + (size_t)(t0 + tok) * width;
     float ss = 0.f;
-    for (int c = lane * 4; c < width; c += 128) {
-      const float4 v = ld4(row + c);
-      ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    for (int c0 = lane * 4; c0 < width; c0 += 1024) {   // eight pieces of the row under way at once
+      float4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = c0 + 128 * j < width ? ld4(row + c0 + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
     }
     ss = warp_sum(ss);
     if (lane == 0) inv_s[r] = 1.f / sqrtf(ss / (float)width + eps);
@@ -159,7 +187,7 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __re
       const int src = first - HALO + j;
       win[j] = src >= 0 ? mul4(scale4(ld4(x + (size_t)(t0 + src) * width + c), inv_s[j]), w) : old[j];
     }
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 0; i < cnt; ++i) {
       const float4 h = mul4(scale4(ld4(x + (size_t)(t0 + first + i) * width + c), inv_s[HALO + i]), w);
       float4 acc = h;
@@ -454,6 +482,11 @@ extern "C" int nqb200_stream_add(float* x, const int64_t* ids, const void* embed
   if (tokens == 0) return NQB200_OK;
   if (!x || (ids && !embed)) return NQB200_ERR_NULL_POINTER;
   const dim3 grid((unsigned)tokens), block(256);
+  if (width % 4 == 0 && aligned16(x) && aligned16(step) && (!ids || aligned16(embed))) {
+    if (dtype == NQB200_F32)
+      return launch_overlapped(stream_add_vec_kernel<float>, grid, block, 0, (cudaStream_t)stream, x, ids, (const float*)embed, step, accumulate, (int)width);
+    return launch_overlapped(stream_add_vec_kernel<bf16>, grid, block, 0, (cudaStream_t)stream, x, ids, (const bf16*)embed, step, accumulate, (int)width);
+  }
   if (dtype == NQB200_F32)
     return launch_overlapped(stream_add_kernel<float>, grid, block, 0, (cudaStream_t)stream, x, ids, (const float*)embed, step, accumulate, (int)width);
   return launch_overlapped(stream_add_kernel<bf16>, grid, block, 0, (cudaStream_t)stream, x, ids, (const bf16*)embed, step, accumulate, (int)width);

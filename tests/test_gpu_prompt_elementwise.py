@@ -1,0 +1,92 @@
+"""Rotary embedding, stream addition and norm + convolution at the sizes where their vector paths begin and end, against
+float64."""
+import pytest
+import torch
+
+from nanoquantization_b200 import _lib
+from nanoquantization_b200.engine.batch import StepBatch
+from nanoquantization_b200.layers import mixers as ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _step(lens, starts, block_size=16):
+    need = [(s + n - 1) // block_size + 1 for n, s in zip(lens, starts)]
+    order = torch.randperm(sum(need), generator=torch.Generator().manual_seed(1)).tolist()
+    blocks = [[order.pop() for _ in range(n)] for n in need]
+    return StepBatch.host([[0] * n for n in lens], starts, blocks, list(range(len(lens))), max(need), block_size).to(DEV), sum(need)
+
+
+@pytest.mark.parametrize("cached,normed", [(True, True), (True, False), (False, False)])
+@pytest.mark.parametrize("neighbours", [False, True])
+@pytest.mark.parametrize("dim,rot", [(64, 64), (128, 128), (256, 256), (128, 64), (96, 96)])
+@pytest.mark.parametrize("lens,heads,kv_heads", [((1,), 1, 1), ((3, 2), 5, 2), ((595, 30), 3, 1)], ids=str)
+@torch.no_grad()
+def test_rotation(lens, heads, kv_heads, dim, rot, neighbours, cached, normed):
+    """One token, a few, and enough for four tokens per block with a remainder; whole heads that turn and parts of them."""
+    step, nblocks = _step(lens, [7] * len(lens))
+    T = sum(lens)
+    proj = torch.randn(T, (heads + 2 * kv_heads) * dim + 8, device=DEV).bfloat16()
+    want = proj.double()
+    inv = (70.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / rot)).float().to(DEV)
+    norms = [1 + 0.2 * torch.randn(dim, device=DEV) for _ in range(2)] if normed else None
+    kc, vc = (torch.full((nblocks, 16, kv_heads, dim), 5.0, device=DEV).bfloat16() for _ in range(2)) if cached else (None, None)
+    desc = _lib.RopeDesc(heads, kv_heads, dim, dim, rot, int(neighbours), inv.data_ptr(), norms[0].data_ptr() if normed else None,
+                         norms[1].data_ptr() if normed else None, 1e-6)
+    q_off, k_off, v_off = 8, 8 + heads * dim, 8 + (heads + kv_heads) * dim
+    ops.norm_rope(proj, kc, vc, desc, step, q_off, k_off, v_off)
+    a = step.positions.double()[:, None, None] * inv.double()
+
+    def turned(off, n, norm):
+        x = want[:, off:off + n * dim].view(T, n, dim)
+        if normed:
+            x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * norm.double()
+        i, j = (slice(0, rot, 2), slice(1, rot, 2)) if neighbours else (slice(0, rot // 2), slice(rot // 2, rot))
+        y = x.clone()
+        y[..., i], y[..., j] = x[..., i] * a.cos() - x[..., j] * a.sin(), x[..., j] * a.cos() + x[..., i] * a.sin()
+        return y
+    q, k = turned(q_off, heads, norms and norms[0]), turned(k_off, kv_heads, norms and norms[1])
+
+    def close(got, want):   # one rounding to bfloat16; angles of up to 600 in float, 600 * 2^-24 apart
+        assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) * 1.05
+    close(proj[:, q_off:k_off].view(T, heads, dim), q)
+    assert torch.equal(proj[:, :q_off].double(), want[:, :q_off]) and torch.equal(proj[:, v_off:].double(), want[:, v_off:])
+    if cached:
+        close(kc.view(-1, kv_heads, dim)[step.rows], k)
+        assert torch.equal(vc.view(-1, kv_heads, dim)[step.rows].double(), want[:, v_off:v_off + kv_heads * dim].view(T, kv_heads, dim))
+        assert int((kc == 5.0).flatten(2).all(-1).sum()) >= nblocks * 16 - T
+    else:
+        close(proj[:, k_off:v_off].view(T, kv_heads, dim), k)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width", [4, 100, 4096, 5000, 8200, 37])
+@torch.no_grad()
+def test_stream_add(width, dtype):
+    e, ids, v = torch.randn(9, width, device=DEV).to(dtype), torch.tensor([8, 0, 3, 3], device=DEV), torch.randn(width, device=DEV)
+    x = torch.full((4, width), float("nan"), device=DEV)
+    ops.stream_add(x, ids, e, None, False)
+    assert torch.equal(x, e.float()[ids])
+    ops.stream_add(x, ids, e, v, True)
+    assert torch.equal(x, e.float()[ids] + e.float()[ids] + v)
+
+
+@pytest.mark.parametrize("width", [4, 1020, 1028, 4096])
+@torch.no_grad()
+def test_norm_and_convolution_of_prompts(width):
+    lens = (33, 17, 2)
+    step, _ = _step(lens, [0] * 3)
+    x, w, cw = torch.randn(sum(lens), width, device=DEV), 1 + 0.2 * torch.randn(width, device=DEV), torch.randn(4, width, device=DEV)
+    state = torch.full((4, 3, width), 9.0, device=DEV)
+    got = ops.rmsnorm_conv(x, w, cw, state, step, 1e-6, torch.float32)
+    o = 0
+    for b, n in enumerate(lens):
+        h = x[o:o + n].double()
+        h = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        full = torch.cat([torch.zeros(3, width, dtype=torch.float64, device=DEV), h])
+        want = h + sum(cw.double()[j] * full[j:j + n] for j in range(4))
+        # float sums of a few terms of the size of the largest
+        assert float((got[o:o + n].double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+        assert float((state[b].double() - full[-3:]).abs().max()) <= 1e-5 * float(full.abs().max())
+        o += n
