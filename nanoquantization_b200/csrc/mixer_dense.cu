@@ -32,9 +32,12 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 }
 
 template <int MODE, int MT>
-__global__ void __launch_bounds__(256) dense_decode_kernel(const DenseArgs p) {
+__global__ void __launch_bounds__(256, MT == 1 ? 3 : 2) dense_decode_kernel(const DenseArgs p) {
   constexpr int NG = MODE == kMinGru ? 3 : MODE == kGlu ? 2 : 1;      // row groups that meet in one output
-  constexpr int U = MODE == kMinGru ? 2 : MODE == kGlu ? 4 : 8;       // k-blocks in flight per warp
+  // k-blocks in flight per warp.  Fewer of them and more CTAs per SM keep the memory busier than twice as many that the warp
+  // then works off at once while nothing is under way: decode step of 3, 8 and 16 sequences of Vemedra layers 566, 678 and 681
+  // us with twice as many (and two CTAs per SM), 477, 554 and 639 so; with three quarters of these 537, 629, 663.
+  constexpr int U = MODE == kMinGru ? (MT == 1 ? 1 : 2) : MODE == kGlu ? 2 : 4;
   __shared__ float part[8][NG][MT * 8][16 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * 16, blocks = (p.K + 31) / 32;

@@ -70,8 +70,11 @@ __device__ __forceinline__ void moe_mma(float (&c)[4], uint32_t a0, uint32_t a1,
 }
 
 template <typename O, int MT>
-__global__ void __launch_bounds__(256) moe_decode_kernel(const MoeDevice p) {
-  constexpr int U = 8;      // k-blocks in flight per warp
+__global__ void __launch_bounds__(256, 3) moe_decode_kernel(const MoeDevice p) {
+  // k-blocks in flight per warp, as in the dense linears: eight, with two CTAs per SM, took a decode step of 1, 5 and 14
+  // sequences of Verozen layers (both kernels changed together) 486, 916 and 1543 us; four and six 427, 821 and 1342; so it
+  // takes 427, 797 and 1270.
+  constexpr int U = MT == 1 ? 3 : 2;
   __shared__ float part[8][MT * 8][16 + 1];
   grid_launch_dependents();
   grid_dependency_wait();
