@@ -334,7 +334,7 @@ __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h,
   const bool fresh = pos == 0;
   const bf16 *qr = row + a.rq_off + (size_t)h * D, *kr = row + a.rk_off + (size_t)h * D;
   float* st = a.rstate + ((size_t)a.bt.slot[b] * a.ret_heads + h) * D * V;
-  constexpr int U = 16;                       // rows of the state under way per thread
+  constexpr int U = 8;                        // rows of the state under way per thread
   float S[U][VEC];
   auto fetch = [&](int r0, int step, int col) {
 #pragma unroll
@@ -350,7 +350,8 @@ __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h,
     }
   };
   // The state is what there is to read, and it depends on nothing but the slot: its first rows are requested ahead of the
-  // rotation, the decays and their barriers.  5 sequences, 16 heads of 128 x 256, gated: 18.7 us in the chain without, 16.0 with.
+  // rotation, the decays and their barriers.  5 sequences, 16 heads of 128 x 256 over
+  // clusters of four, gated: 18.7 us in the chain without, 16.0 with.
   if (ncol > 0) {
     const int width = min(ncol, kDecThreads), rgi = tid / width;
     if (rgi < kDecThreads / width) fetch(rgi, kDecThreads / width, (c0 + tid % width) * VEC);
@@ -559,8 +560,11 @@ extern "C" int nqb200_mixer_decode(const void* proj, int64_t stride, void* act, 
     units += r->heads;
     while (want < 8 && (int64_t)r->dim * r->vdim * 4 > (int64_t)want * 16384 && want * 8 <= r->vdim) want *= 2;
   }
-  // about one CTA of attention per SM (its ring takes most of the shared memory), and no more than there is work for
-  while (csize < want && units * b->batch * csize * 2 <= (a ? kNumSMs * 3 / 2 : kNumSMs * 4)) csize *= 2;
+  // About one CTA of attention per SM (its ring takes most of the shared memory), and no more than there is work for.  The
+  // states alone: two CTAs per SM at most, so that a head is split over a cluster only where heads are few, because clusters
+  // cost more to start and to meet than they spread.  16 sequences of 16 heads of 128 x 256: 18 us unsplit, 24 over two CTAs, 30
+  // over four, 50 over eight; 5 sequences: 10 over two, 16 over four, 21 over eight.
+  while (csize < want && units * b->batch * csize * 2 <= (a ? kNumSMs * 3 / 2 : kNumSMs * 2)) csize *= 2;
   cudaStream_t st = (cudaStream_t)stream;
   const bool v4 = !r || r->vdim % 4 == 0;
   // 128 keys a pass where two stages of them fit
