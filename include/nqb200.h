@@ -182,7 +182,8 @@ int nqb200_qknorm_rope_kv(void* qkv, const void* q_weight, const void* k_weight,
 /* One decode step's attention over the paged cache, in one launch: what nqb200_qknorm_rope_kv does to the step's token of
  * every sequence (qkv itself is left as it is), then softmax(scale q k) v over the ctx[b] keys of sequence b, the step's own
  * among them.  Block i of sequence b is table[b][i]; slots[b] is the row of the step's token, positions[b] its position.
- * Heads of 128; row_stride (elements) a multiple of 8; out is [batch, num_q_heads * 128].  No counterpart in the reference. */
+ * ctx[b] <= table_width * block_size.  ctx[b] = 0 is a row without a sequence: its output is 0, nothing of its table, slot and
+ * position is read and nothing is stored.  Heads of 128; row_stride (elements) a multiple of 8; out is [batch, num_q_heads * 128].  No counterpart in the reference. */
 int nqb200_decode_attention(const void* qkv, int64_t row_stride, const void* q_weight, const void* k_weight, const float* cos_sin,
                             const int64_t* positions, const int64_t* slots, void* k_cache, void* v_cache, const int32_t* table,
                             const int32_t* ctx, int64_t table_width, int64_t block_size, void* out, int64_t batch, int64_t num_q_heads,

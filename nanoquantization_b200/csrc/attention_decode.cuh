@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
   const int h0 = kvh * per_kv + hg * kHeads, R = min(kHeads, per_kv - hg * kHeads);
   const int pos = a.last[b] + a.last_shift;
   const int lo = a.chunk > 0 ? pos / a.chunk * a.chunk : 0;
-  const int tiles = (pos - lo) / kTile + 1, per = (tiles + csize - 1) / csize;
+  // a position below 0: a row without a sequence, which has no tile to read and none to store, and gets zeros
+  const int tiles = pos < 0 ? 0 : (pos - lo) / kTile + 1, per = (tiles + csize - 1) / csize;
   const int t0 = min(rank * per, tiles), t1 = min(t0 + per, tiles);
   const bool newest = t1 == tiles && t0 < t1;      // this CTA has the tile with the step's own key
   const T* row = a.proj + (int64_t)b * a.stride;
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) load(t0 + warp + s * kWarps, s);
 
-  rotate_new<T>(a, fx, row, b, pos, h0, R, kvh, newest);
+  if (pos >= 0) rotate_new<T>(a, fx, row, b, pos, h0, R, kvh, newest);
   __syncthreads();
 
   const int g = lane >> 2, t4 = lane & 3;
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
   const auto finish = [&](int r, int d, float o, float sum, float top) {   // top in units of log 2
     if (MODE != kSigmoid) {
       if (a.sink) sum += exp2_fast(a.sink[h0 + r] * kLog2e - top);
-      o /= sum;
+      o = pos < 0 ? 0.f : o / sum;
     }
     reinterpret_cast<uint16_t*>(out)[(int64_t)(h0 + r) * kDim + d] = float_to_raw16<BF16>(o * a.out_scale);
   };

@@ -74,6 +74,36 @@ def test_qwen3_step(ctx, kv_heads, heads, block_size, dtype):
         _close(got[b], torch.einsum("hn,nhd->hd", w, v).flatten(), dtype)
 
 
+@pytest.mark.parametrize("ctx", [(0,), (0, 17, 0, 300, 0), (0,) * 3 + (5000,)], ids=str)
+@torch.no_grad()
+def test_rows_without_a_sequence(ctx):
+    """A context of 0 (what paged interfaces pad a batch with): zeros, caches untouched, and the other rows as without them."""
+    from nanoquantization_b200.layers import fused
+    from nanoquantization_b200.models import RotaryCache
+    heads, kv_heads, dtype = 8, 2, torch.bfloat16
+    live = [i for i, n in enumerate(ctx) if n]
+    step, _, kc, vc, proj = _setup([n or 1 for n in ctx], kv_heads, heads, 16, dtype)
+    proj = proj[:, :-8].contiguous()
+    w = torch.ones(D, device=DEV, dtype=dtype)
+    rope = RotaryCache(D, 8192, 1e6).to(DEV)
+    for i, n in enumerate(ctx):
+        if not n:
+            step.ctx[i], step.positions[i], step.rows[i] = 0, -1, -1
+            step.table[i] = -1
+    before = kc.clone(), vc.clone()
+    got = fused.decode_attention(proj, w, w, rope.cos_sin_cache, step.positions, heads, kv_heads, D, 1e-6, kc, vc, step)
+    assert not got[[i for i, n in enumerate(ctx) if not n]].any()
+    changed = (kc != before[0]).flatten(2).any(-1).flatten().nonzero().flatten()
+    assert sorted(changed.tolist()) == sorted(step.rows[live].tolist())
+    if live:
+        i64 = torch.cat([step.tokens[live], step.positions[live], step.rows[live]])
+        i32 = torch.cat([torch.arange(len(live) + 1, device=DEV), step.pos0[live], step.ctx[live], step.slot[live], step.table[live].flatten()]).int()
+        alone = StepBatch(i64, i32, [1] * len(live), [ctx[i] - 1 for i in live], step.width, step.block_size)
+        kc, vc = before
+        want = fused.decode_attention(proj[live].contiguous(), w, w, rope.cos_sin_cache, alone.positions, heads, kv_heads, D, 1e-6, kc, vc, alone)
+        _close(got[live], want.double(), dtype)
+
+
 @pytest.mark.parametrize("kind", ["capped", "sigmoid"])
 @pytest.mark.parametrize("chunk,rot", [(0, 128), (40, 64), (256, 0)])
 @pytest.mark.parametrize("ctx,kv_heads,heads,block_size", SHAPES, ids=str)
