@@ -160,7 +160,7 @@ __device__ __forceinline__ void rotate_new(const Args<T>& a, Fixed& fx, const T*
         const float t = __shfl_sync(0xFFFFFFFFu, v[k], mate[e] >> 2);
         if (k == (mate[e] & 3)) other = t;
       }
-      y[e] = float_to_raw16<BF16>(v[e] * c[e] + other * s[e]);
+      y[e] = float_to_raw16<BF16>(4 * lane + e < rot ? v[e] * c[e] + other * s[e] : v[e]);   // an infinity passes as it is
     }
     *dst = make_uint2(y[0] | (y[1] << 16), y[2] | (y[3] << 16));
   }

@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(256, 4) norm_rope_vec_kernel(bf16* proj, bf16*
         const float cv[4] = {c.x, c.y, c.z, c.w}, sv[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          y[2 * e] = x[2 * e] * cv[e] - x[2 * e + 1] * sv[e];
-          y[2 * e + 1] = x[2 * e + 1] * cv[e] + x[2 * e] * sv[e];
+          y[2 * e] = turns ? x[2 * e] * cv[e] - x[2 * e + 1] * sv[e] : x[2 * e];
+          y[2 * e + 1] = turns ? x[2 * e + 1] * cv[e] + x[2 * e] * sv[e] : x[2 * e + 1];
         }
       } else {
 #pragma unroll
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256, 4) norm_rope_vec_kernel(bf16* proj, bf16*
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float other = __shfl_sync(0xFFFFFFFFu, x[4 * q + e], partner);
-            y[4 * q + e] = x[4 * q + e] * cv[e] + other * (upper ? sv[e] : -sv[e]);
+            y[4 * q + e] = turns ? x[4 * q + e] * cv[e] + other * (upper ? sv[e] : -sv[e]) : x[4 * q + e];
           }
         }
       }

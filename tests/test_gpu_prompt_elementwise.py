@@ -60,6 +60,32 @@ def test_rotation(lens, heads, kv_heads, dim, rot, neighbours, cached, normed):
         close(proj[:, k_off:v_off].view(T, kv_heads, dim), k)
 
 
+@pytest.mark.parametrize("call", ["rope_store", "norm_rope", "norm_rope neighbours", "mixer_decode"])
+@pytest.mark.parametrize("rot", [0, 64])
+@torch.no_grad()
+def test_dimensions_that_do_not_turn_pass_unchanged(rot, call):
+    """Infinities and signed zeros beyond the rotated dimensions reach the cache bit for bit (infinity * 0 is not a number)."""
+    T, heads, kv_heads, dim = 3, 4, 2, 128
+    step, nblocks = _step([1] * T, [5, 0, 40])
+    proj = torch.randn(T, (heads + 2 * kv_heads) * dim, device=DEV).bfloat16()
+    k = proj[:, heads * dim:(heads + kv_heads) * dim].view(T, kv_heads, dim)
+    k[:, :, rot::3], k[:, 0, rot + 1::3], k[:, 1, rot + 1::3] = float("inf"), float("-inf"), -0.0
+    want = k.clone()
+    inv = (70.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / max(rot, 1))).float().to(DEV)
+    kc, vc = (torch.zeros(nblocks, 16, kv_heads, dim, device=DEV).bfloat16() for _ in range(2))
+    offs = (0, heads * dim, (heads + kv_heads) * dim)
+    rope = _lib.RopeDesc(heads, kv_heads, dim, dim, rot, int(call.endswith("neighbours")), inv.data_ptr() if rot else None, None, None, 1e-6)
+    if call == "rope_store":
+        ops.rope_store(proj, kc, vc, inv, step, *offs, heads)
+    elif call.startswith("norm_rope"):
+        ops.norm_rope(proj, kc, vc, rope, step, *offs)
+    else:
+        att = _lib.AttentionDesc(heads, kv_heads, dim, dim, 0, 0.1, 0.0, None, 1.0, None, None, 0)
+        ops.mixer_decode(proj, torch.empty(T, heads * dim, device=DEV).bfloat16(), (att, rope, 0, offs[2], 0, kc, vc), None, step)
+    got = kc.view(-1, kv_heads, dim)[step.rows]
+    assert torch.equal(got[..., rot:].view(torch.int16), want[..., rot:].view(torch.int16))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width", [4, 100, 4096, 5000, 8200, 37])
 @torch.no_grad()
