@@ -5,10 +5,10 @@ The reference has none of this (its only execution is a full-sequence forward fo
 models/qwen3_quantized.py:326-341); it exists so that models are measured where they are used: prefill of batched
 prompts (whole or in portions) and greedy decode steps over a cache.  A model states what it keeps per layer run
 (``cache_layout()``) and runs one step on a ``StepBatch`` (``forward_step``).  For a model that delegates attention
-(Qwen3) the engine supplies it: PyTorch's scaled_dot_product_attention per prompt at prefill; at decode the model's own
-kernel over the pages for heads of 128, else flash_attn's when that library loads on this GPU, else
-scaled_dot_product_attention over the gathered pages of each sequence.  Other models bring kernels that read the cache and
-the states themselves.
+(Qwen3) the engine supplies it: PyTorch's scaled_dot_product_attention per prompt at prefill; at decode flash_attn's
+paged-KV kernel when that library loads on this GPU, else scaled_dot_product_attention over the gathered pages of
+each sequence.  Qwen3 with heads of 128 has a kernel of its own for decode steps and does not ask for it there.  Other models
+bring kernels that read the cache and the states themselves.
 
 Layout: per layer run two tensors ``[num_blocks, block_size, kv_heads, head_dim]``; a sequence owns a list of blocks;
 ``row = block * block_size + offset``.  Blocks that no later query can reach (every layer attends inside chunks) are
@@ -274,9 +274,7 @@ class LLMEngine:
         self.blocks = BlockManager(num_blocks, block_size)
         self.scheduler = Scheduler(self.blocks, max_batch, max_prefill_tokens, prefill_portion, self.states)
         self.use_cuda_graph = use_cuda_graph
-        self.paged_attention = None
-        if model.delegates_attention and block_size % 256 == 0 and self.layout.kv[0].head_dim != 128:
-            self.paged_attention = self._probe_flash_attn()
+        self.paged_attention = self._probe_flash_attn() if model.delegates_attention and block_size % 256 == 0 else None
         self._graphs: dict[tuple[int, int], tuple] = {}
         self._warm_stream = None  # one side stream for every graph warm-up (scratch buffers are kept per stream)
         self._next_id = 0
@@ -358,8 +356,8 @@ class LLMEngine:
             h, out = self._decode_forward(self._decode_inputs(batch, width).to(self.device))
         else:
             # one graph per (batch bucket, block-table width): batches are padded up to a power of two, so that
-            # continuous batching replays a few dozen graphs.  For the engine's own attention the block table keeps
-            # its exact width, by which that kernel sizes its KV splits (a table padded from 9 to 16 blocks cost
+            # continuous batching replays a few dozen graphs.  Where a model may ask for the engine's attention the block
+            # table keeps its exact width, by which flash_attn sizes its KV splits (a table padded from 9 to 16 blocks cost
             # 18 % of a step); kernels that look up their own pages take a width rounded up as well
             rows = 1 << (B - 1).bit_length()
             if not self.model.delegates_attention:

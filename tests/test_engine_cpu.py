@@ -50,6 +50,27 @@ def test_scheduler_preempts_when_blocks_run_out():
     assert sch.waiting[0].seq_id == 1 and sch.waiting[0].prompt == [1] * 7 + [5] and sch.waiting[0].blocks == []
 
 
+def test_models_that_call_the_engine_for_decode_get_the_paged_kernel(monkeypatch):
+    """``attend(q, k, v)`` of a decode step goes to the paged kernel that the engine found, for heads of 128 as for others."""
+    import torch
+    from nanoquantization_b200.engine import LayerStep, LLMEngine, StepBatch
+    from nanoquantization_b200.models.qwen3_quantized import Qwen3QuantizedForCausalLM
+    calls = []
+
+    def paged(q, k_cache, v_cache, cache_seqlens, block_table, causal):
+        calls.append((tuple(q.shape), cache_seqlens.tolist(), block_table.tolist(), causal))
+        return torch.zeros_like(q)
+    monkeypatch.setattr(LLMEngine, "_probe_flash_attn", lambda self: paged)
+    for dim in (64, 128):
+        model = Qwen3QuantizedForCausalLM(1, 64, 256, 256 // dim, 1, 32, 128, 4, 128, dim, device="cpu", dtype=torch.float16)
+        eng = LLMEngine(model, num_blocks=2, block_size=256, max_batch=2, use_cuda_graph=False)
+        step = StepBatch.host([[0], [0]], [4, 0], [[1], [0]], [0, 1], 1, 256)
+        q, k = torch.ones(2, 256 // dim, dim, dtype=torch.float16), torch.ones(2, 1, dim, dtype=torch.float16)
+        assert LayerStep(eng, 0, step, True)(q, k, k).shape == q.shape
+        assert calls.pop() == ((2, 1, 256 // dim, dim), [5, 1], [[1], [0]], True) and not calls
+        assert eng.cache.k[0].view(-1, 1, dim)[[256 + 4, 0]].eq(1).all()
+
+
 def test_engine_rejects_a_prompt_the_cache_can_never_hold():
     import pytest
     import torch
