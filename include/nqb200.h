@@ -189,6 +189,16 @@ int nqb200_decode_attention(const void* qkv, int64_t row_stride, const void* q_w
                             const int32_t* ctx, int64_t table_width, int64_t block_size, void* out, int64_t batch, int64_t num_q_heads,
                             int64_t num_kv_heads, int64_t head_dim, float scale, float eps, int dtype, void* stream);
 
+/* The same where a few long sequences leave most of the GPU idle: a sequence goes over several clusters, whose shares a second
+ * launch adds.  scratch: the bytes that the first function gives (0 where the step goes as above), written before read, not
+ * shared by calls that can overlap. */
+size_t nqb200_decode_attention_scratch_bytes(int64_t table_width, int64_t block_size, int64_t batch, int64_t num_q_heads, int64_t num_kv_heads);
+int nqb200_decode_attention_split(const void* qkv, int64_t row_stride, const void* q_weight, const void* k_weight, const float* cos_sin,
+                                  const int64_t* positions, const int64_t* slots, void* k_cache, void* v_cache, const int32_t* table,
+                                  const int32_t* ctx, int64_t table_width, int64_t block_size, void* out, int64_t batch, int64_t num_q_heads,
+                                  int64_t num_kv_heads, int64_t head_dim, float scale, float eps, int dtype, void* scratch, size_t scratch_bytes,
+                                  void* stream);
+
 /* One-shot all-reduce (sum) over NVLink peer memory for the small [M, N] partial results of a
  * row-parallel linear.  No counterpart in the reference (it has no distributed code).
  * Set-up, once: every rank calls nqb200_comm_alloc (a cudaMalloc'd, zeroed buffer: a header of

@@ -49,6 +49,8 @@ SIGNATURES = {
     "nqb200_qknorm_rope": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, ctypes.c_float, _int, _vp]),
     "nqb200_qknorm_rope_kv": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, ctypes.c_float, _int, _vp]),
     "nqb200_decode_attention": (_int, [_vp, _i64] + [_vp] * 9 + [_i64, _i64, _vp, _i64, _i64, _i64, _i64, ctypes.c_float, ctypes.c_float, _int, _vp]),
+    "nqb200_decode_attention_scratch_bytes": (_sz, [_i64] * 5),
+    "nqb200_decode_attention_split": (_int, [_vp, _i64] + [_vp] * 9 + [_i64, _i64, _vp, _i64, _i64, _i64, _i64, ctypes.c_float, ctypes.c_float, _int, _vp, _sz, _vp]),
     "nqb200_silu_mul": (_int, [_vp, _vp, _i64, _i64, _int, _vp]),
     "nqb200_comm_alloc": (_int, [ctypes.POINTER(_vp), _sz]),
     "nqb200_comm_free": (_int, [_vp]),

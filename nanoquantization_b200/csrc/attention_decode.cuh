@@ -30,6 +30,7 @@ constexpr int kDim = 128, kWarps = 4, kThreads = 32 * kWarps, kTile = 16, kHeads
 constexpr int kTileBytes = 2 * kTile * kDim * 2;              // keys, then values
 __host__ __device__ constexpr int ring_bytes(int stages) { return kWarps * stages * kTileBytes; }
 constexpr int kOS = kDim + 4;                                 // stride of a head's partial sums
+constexpr int kShare = kDim + 4;                              // floats of a head's share: sums, maximum, sum of weights
 constexpr float kLog2e = 1.4426950408889634f;
 
 enum Mode { kSoftmax = 0, kCapped = 1, kSigmoid = 2 };
@@ -52,6 +53,7 @@ template <typename T> struct Args {
   // or (cos_sin given) by a [position, cos | sin] table after norms with 16-bit weights, rounded where 16-bit tensors would stand
   const float* cos_sin; const int64_t* positions;
   const T *q_weight, *k_weight;
+  float* shares; int parts;                        // a sequence over several clusters (parts > 1, plain softmax): their shares
 };
 
 struct Fixed {                                     // behind the ring
@@ -97,8 +99,20 @@ __device__ __forceinline__ float recip_fast(float x) { float r; asm("rcp.approx.
 
 // The step's own query heads (into fx.q, zeros beyond R) and key (into fx.knew): a head per warp at a time, a lane holds
 // elements 4 lane .. 4 lane + 3 and gets their partners in the rotation by shuffles.
+constexpr int kNew = (kHeads + kWarps) / kWarps;              // heads and key per warp at most
 template <typename T>
-__device__ __forceinline__ void rotate_new(const Args<T>& a, Fixed& fx, const T* row, int b, int pos, int h0, int R, int kvh, bool newest) {
+__device__ __forceinline__ void request_new(const Args<T>& a, uint2 (&raw)[kNew], const T* row, int h0, int R, int kvh, bool newest) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < kNew; ++i) {
+    const int r = warp + i * kWarps;
+    raw[i] = make_uint2(0u, 0u);
+    if (r < R || (newest && r == kHeads))
+      raw[i] = reinterpret_cast<const uint2*>(r < kHeads ? row + a.q_off + (int64_t)(h0 + r) * kDim : row + a.k_off + (int64_t)kvh * kDim)[lane];
+  }
+}
+template <typename T>
+__device__ __forceinline__ void rotate_new(const Args<T>& a, Fixed& fx, const uint2 (&raws)[kNew], int b, int pos, int R, bool newest) {
   constexpr bool BF16 = Traits<T>::kBf16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool tabled = a.cos_sin != nullptr;
@@ -125,13 +139,16 @@ __device__ __forceinline__ void rotate_new(const Args<T>& a, Fixed& fx, const T*
       if (first) s[e] = -s[e];
     }
   }
-  for (int r = warp; r < kHeads + (newest ? 1 : 0); r += kWarps) {
+#pragma unroll
+  for (int i = 0; i < kNew; ++i) {
+    const int r = warp + i * kWarps;
+    if (r >= kHeads + (newest ? 1 : 0)) break;
     uint2* dst = reinterpret_cast<uint2*>(r < kHeads ? fx.q[r] : fx.knew) + lane;
     if (r >= R && r < kHeads) {
       *dst = make_uint2(0u, 0u);
       continue;
     }
-    const uint2 raw = reinterpret_cast<const uint2*>(r < kHeads ? row + a.q_off + (int64_t)(h0 + r) * kDim : row + a.k_off + (int64_t)kvh * kDim)[lane];
+    const uint2 raw = raws[i];
     float v[4] = {raw16_to_float<BF16>((uint16_t)(raw.x & 0xFFFF)), raw16_to_float<BF16>((uint16_t)(raw.x >> 16)),
                   raw16_to_float<BF16>((uint16_t)(raw.y & 0xFFFF)), raw16_to_float<BF16>((uint16_t)(raw.y >> 16))};
     if (tabled || a.q_norm) {
@@ -155,10 +172,14 @@ __device__ __forceinline__ void rotate_new(const Args<T>& a, Fixed& fx, const T*
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       float other = 0.f;
+      if (tabled) {                                // half a head away: the same element of the lane 16 on
+        other = __shfl_xor_sync(0xFFFFFFFFu, v[e], 16);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float t = __shfl_sync(0xFFFFFFFFu, v[k], mate[e] >> 2);
-        if (k == (mate[e] & 3)) other = t;
+        for (int k = 0; k < 4; ++k) {
+          const float t = __shfl_sync(0xFFFFFFFFu, v[k], mate[e] >> 2);
+          if (k == (mate[e] & 3)) other = t;
+        }
       }
       y[e] = float_to_raw16<BF16>(4 * lane + e < rot ? v[e] * c[e] + other * s[e] : v[e]);   // an infinity passes as it is
     }
@@ -178,15 +199,15 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
   grid_launch_dependents();
   grid_dependency_wait();
   cg::cluster_group cl = cg::this_cluster();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x, csize = gridDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, csize = gridDim.x / a.parts, rank = blockIdx.x % csize;
   const int unit = blockIdx.y, b = blockIdx.z;
   const int per_kv = a.heads / a.kv_heads, kvh = unit / a.head_groups, hg = unit % a.head_groups;
   const int h0 = kvh * per_kv + hg * kHeads, R = min(kHeads, per_kv - hg * kHeads);
   const int pos = a.last[b] + a.last_shift;
   const int lo = a.chunk > 0 ? pos / a.chunk * a.chunk : 0;
   // a position below 0: a row without a sequence, which has no tile to read and none to store, and gets zeros
-  const int tiles = pos < 0 ? 0 : (pos - lo) / kTile + 1, per = (tiles + csize - 1) / csize;
-  const int t0 = min(rank * per, tiles), t1 = min(t0 + per, tiles);
+  const int tiles = pos < 0 ? 0 : (pos - lo) / kTile + 1, per = (tiles + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int t0 = min((int)blockIdx.x * per, tiles), t1 = min(t0 + per, tiles);
   const bool newest = t1 == tiles && t0 < t1;      // this CTA has the tile with the step's own key
   const T* row = a.proj + (int64_t)b * a.stride;
   uint8_t* ring = smem + warp * (kStages * kTileBytes);
@@ -211,10 +232,13 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  // requested ahead of the table's entries, so that the two trips to memory are one
+  uint2 raws[kNew];
+  if (pos >= 0) request_new<T>(a, raws, row, h0, R, kvh, newest);
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) load(t0 + warp + s * kWarps, s);
 
-  if (pos >= 0) rotate_new<T>(a, fx, row, b, pos, h0, R, kvh, newest);
+  if (pos >= 0) rotate_new<T>(a, fx, raws, b, pos, R, newest);
   __syncthreads();
 
   const int g = lane >> 2, t4 = lane & 3;
@@ -336,6 +360,12 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
   __syncthreads();
   T* out = a.out + (int64_t)b * a.out_stride + a.out_col;
   const auto finish = [&](int r, int d, float o, float sum, float top) {   // top in units of log 2
+    if (MODE == kSoftmax && a.parts > 1) {
+      float* share = a.shares + (((int64_t)b * a.heads + h0 + r) * a.parts + blockIdx.x / csize) * kShare;
+      share[d] = o;
+      if (d == 0) { share[kDim] = top; share[kDim + 1] = sum; }
+      return;
+    }
     if (MODE != kSigmoid) {
       if (a.sink) sum += exp2_fast(a.sink[h0 + r] * kLog2e - top);
       o = pos < 0 ? 0.f : o / sum;
@@ -385,6 +415,26 @@ __global__ void __launch_bounds__(kThreads, STAGES == 2 ? 3 : STAGES == 3 ? 2 : 
   cl.sync();                                       // peers may still read this CTA's shared memory
 }
 
+// The shares of a sequence's clusters, a CTA per (query head, sequence), in the clusters' order.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) attention_shares_kernel(const float* __restrict__ shares, T* __restrict__ out, int64_t out_stride, int parts, const int32_t* last,
+                                                                    int last_shift) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int64_t head = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
+  const float* s = shares + head * parts * kShare;
+  float top = -INFINITY, sum = 0.f, o = 0.f;
+  for (int p = 0; p < parts; ++p) top = fmaxf(top, s[p * kShare + kDim]);
+#pragma unroll 4
+  for (int p = 0; p < parts; ++p) {
+    const float m = s[p * kShare + kDim], f = m == top ? 1.f : exp2f(m - top);
+    o += f * s[p * kShare + threadIdx.x];
+    sum += f * s[p * kShare + kDim + 1];
+  }
+  o = last[blockIdx.y] + last_shift < 0 ? 0.f : o / sum;   // as above: a row without a sequence
+  reinterpret_cast<uint16_t*>(out)[blockIdx.y * out_stride + (int64_t)blockIdx.x * kDim + threadIdx.x] = float_to_raw16<Traits<T>::kBf16>(o);
+}
+
 static inline bool supported(int64_t heads, int64_t kv_heads, int64_t dim, int64_t vdim) {
   return dim == kDim && vdim == kDim && kv_heads > 0 && heads > 0 && heads % kv_heads == 0 && kv_heads <= 4096 && heads <= 65535;
 }
@@ -396,7 +446,7 @@ static inline int launch_stages(const Args<T>& a, int csize, int64_t batch, bool
                               : a.softcap > 0.f ? attention_decode_kernel<T, kCapped, STAGES> : attention_decode_kernel<T, kSoftmax, STAGES>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return NQB200_ERR_LAUNCH; }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)csize, (unsigned)(a.kv_heads * a.head_groups), (unsigned)batch);
+  cfg.gridDim = dim3((unsigned)(csize * a.parts), (unsigned)(a.kv_heads * a.head_groups), (unsigned)batch);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -413,19 +463,47 @@ static inline int launch_stages(const Args<T>& a, int csize, int64_t batch, bool
   return NQB200_OK;
 }
 
-// `keys`: the most that a sequence of the step may see.
+// How a step is split.  Clusters of 1, 2, 4, 8 CTAs that a B200 holds at once (cudaOccupancyMaxActiveClusters; clusters do not
+// cross the chip's processing clusters, so that 15 and not 18 of eight fit), with a ring of 4, 3, 2 tiles per warp:
+constexpr int kResident[4][3] = {{148, 296, 444}, {74, 148, 222}, {33, 71, 104}, {15, 33, 48}};
+constexpr int kMostParts = 16;
+struct Split { int csize, stages, parts; };
+// `keys`: the most that a sequence of the step may see.  A CTA for every 64 keys (a tile per warp) as long as all clusters are
+// resident, and as long a ring as leaves them so.  2 sequences of 16384 keys, 8 key/value heads: 60 us where the 16 clusters of
+// eight did not fit at once (ring of 4), 34 so.
+// Where clusters of eight leave the chip unfilled and a CTA would get 1024 keys or more, and `shares` may be used, a sequence goes
+// over several of them, down to 256 keys a CTA (1024 where 16 clusters have an SM per CTA already), and a second kernel adds their
+// shares (about 3 us).  One sequence of 32768 keys, 8 key/value heads: 52 us over one cluster each, 28.8 over four; 1 key/value
+// head: 52 over one, 15.0 over sixteen; at 8192 keys 17.7 and 14.2, 18.2 and 11.5; at 4096 keys 12.0 and 12.0, 12.5 and 9.9.  16 clusters
+// of 1024 keys a CTA: 21.4 us, 25.9 when split in two.
+static inline Split split(int64_t units, int64_t keys, bool shares) {
+  Split s = {1, 2, 1};
+  int row = 0;
+  while (row < 3 && units <= kResident[row + 1][2] && keys > (int64_t)s.csize * kWarps * kTile) { s.csize *= 2; ++row; }
+  if (shares && row == 3 && keys >= 8 * 1024) {
+    const int64_t least = units > kResident[3][0] ? 1024 : 256;
+    while (s.parts < kMostParts && units * s.parts * 2 <= kResident[3][1] && keys >= 8 * s.parts * 2 * least) s.parts *= 2;
+  }
+  while (s.stages < 4 && units * s.parts <= kResident[row][3 - s.stages]) ++s.stages;
+  // few keys, and as many turns with two CTAs per SM as with three: 512 of 100 keys 15.3 and 15.7 us, of 300 23.4 and 24.4
+  const auto turns = [&](int per_sm) { return (units + kNumSMs * per_sm - 1) / (kNumSMs * per_sm); };
+  if (s.stages == 2 && s.csize == 1 && keys <= 512 && turns(2) == turns(3)) s.stages = 3;
+  return s;
+}
+static inline int head_groups(int heads, int kv_heads) { return (heads / kv_heads + kHeads - 1) / kHeads; }
+static inline int64_t share_floats(int64_t batch, int heads, int parts) { return parts > 1 ? batch * heads * parts * kShare : 0; }
+
 template <typename T>
 static inline int launch(Args<T>& a, int64_t batch, int64_t keys, bool sigmoid, cudaStream_t st) {
-  const int per_kv = a.heads / a.kv_heads;
-  a.head_groups = (per_kv + kHeads - 1) / kHeads;
-  const int64_t units = (int64_t)a.kv_heads * a.head_groups * batch;
-  // a tile for every warp, and no more CTAs than can be resident at once (three per SM)
-  int csize = 1;
-  while (csize < 8 && units * csize * 2 <= kNumSMs * 3 && keys > (int64_t)csize * kWarps * kTile) csize *= 2;
-  const int64_t ctas = units * csize;
-  if (ctas <= kNumSMs) return launch_stages<T, 4>(a, csize, batch, sigmoid, st);
-  if (ctas <= kNumSMs * 2) return launch_stages<T, 3>(a, csize, batch, sigmoid, st);
-  return launch_stages<T, 2>(a, csize, batch, sigmoid, st);
+  a.head_groups = head_groups(a.heads, a.kv_heads);
+  const Split s = split((int64_t)a.kv_heads * a.head_groups * batch, keys, a.shares != nullptr);
+  a.parts = s.parts;
+  const int rc = s.stages == 4   ? launch_stages<T, 4>(a, s.csize, batch, sigmoid, st)
+                 : s.stages == 3 ? launch_stages<T, 3>(a, s.csize, batch, sigmoid, st)
+                                 : launch_stages<T, 2>(a, s.csize, batch, sigmoid, st);
+  if (rc != NQB200_OK || s.parts == 1) return rc;
+  return launch_overlapped(attention_shares_kernel<T>, dim3((unsigned)a.heads, (unsigned)batch), dim3(kThreads), 0, st, (const float*)a.shares, a.out + a.out_col,
+                           a.out_stride, s.parts, a.last, a.last_shift);
 }
 
 }  // namespace attdec

@@ -52,18 +52,21 @@ def qknorm_rope_(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tens
 def decode_attention(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, cos_sin: torch.Tensor, positions: torch.Tensor,
                      num_q_heads: int, num_kv_heads: int, head_dim: int, eps: float, k_cache: torch.Tensor, v_cache: torch.Tensor, batch) -> torch.Tensor:
     """One token per sequence of ``batch`` (an engine step): ``qknorm_rope_`` with the K/V store, then attention over the
-    paged caches ``[blocks, block size, Hkv, D]``, in one launch; returns ``[T, Hq * D]``."""
+    paged caches ``[blocks, block size, Hkv, D]``, in one launch, or two for a few long sequences; returns ``[T, Hq * D]``."""
     _lib.require_cuda(qkv, q_weight, k_weight, cos_sin, positions, k_cache, v_cache)
     T = qkv.shape[0]
     assert qkv.is_contiguous() and positions.dtype == torch.int64 and cos_sin.dtype == torch.float32 and batch.batch == T
     assert k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.dtype == v_cache.dtype == qkv.dtype == q_weight.dtype == k_weight.dtype
     assert k_cache.shape[-2:] == v_cache.shape[-2:] == (num_kv_heads, head_dim) and k_cache.shape[1] == batch.block_size
     out = torch.empty(T, num_q_heads * head_dim, dtype=qkv.dtype, device=qkv.device)
-    _lib.check(_lib.load().nqb200_decode_attention(qkv.data_ptr(), qkv.stride(0), q_weight.data_ptr(), k_weight.data_ptr(), cos_sin.data_ptr(),
-                                                   positions.data_ptr(), batch.rows.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                                                   batch.table.data_ptr(), batch.ctx.data_ptr(), batch.width, batch.block_size, out.data_ptr(), T,
-                                                   num_q_heads, num_kv_heads, head_dim, head_dim ** -0.5, float(eps), _lib.dtype_code(qkv.dtype),
-                                                   _lib.stream_ptr()))
+    lib = _lib.load()
+    need = lib.nqb200_decode_attention_scratch_bytes(batch.width, batch.block_size, T, num_q_heads, num_kv_heads)
+    scratch = torch.empty(need, dtype=torch.uint8, device=qkv.device) if need else None
+    _lib.check(lib.nqb200_decode_attention_split(qkv.data_ptr(), qkv.stride(0), q_weight.data_ptr(), k_weight.data_ptr(), cos_sin.data_ptr(),
+                                                 positions.data_ptr(), batch.rows.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                                                 batch.table.data_ptr(), batch.ctx.data_ptr(), batch.width, batch.block_size, out.data_ptr(), T,
+                                                 num_q_heads, num_kv_heads, head_dim, head_dim ** -0.5, float(eps), _lib.dtype_code(qkv.dtype),
+                                                 scratch.data_ptr() if need else None, need, _lib.stream_ptr()))
     return out
 
 

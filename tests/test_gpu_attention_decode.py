@@ -49,7 +49,11 @@ def _close(got, want, dtype):
     assert err <= 4 * eps, err
 
 
-SHAPES = [((1,), 1, 1, 16), ((2, 16, 17, 64, 65), 2, 8, 16), ((5, 500, 1025), 2, 2, 256), ((129, 3), 3, 48, 24), ((33,) * 70, 8, 32, 256), ((2048,), 8, 16, 256)]
+# edges of tiles and warps; rings that wrap many times with remainders, for each length of ring: four tiles (few CTAs), three (16 of
+# about 1900 keys over clusters of two), two (48 of 1100 to 1500, one CTA a sequence and head; 50 of about 600 over clusters of eight)
+SHAPES = [((1,), 1, 1, 16), ((2, 16, 17, 64, 65), 2, 8, 16), ((5, 500, 1025), 2, 2, 256), ((129, 3), 3, 48, 24), ((33,) * 70, 8, 32, 256), ((2048,), 8, 16, 256),
+          ((4321,), 1, 4, 256), (tuple(1900 - 31 * i for i in range(16)), 8, 16, 256), (tuple(1500 - 8 * i for i in range(48)), 8, 8, 16),
+          (tuple(600 - 3 * i for i in range(50)), 1, 2, 32)]
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -61,7 +65,7 @@ def test_qwen3_step(ctx, kv_heads, heads, block_size, dtype):
     step, blocks, kc, vc, proj = _setup(ctx, kv_heads, heads, block_size, dtype)
     proj = proj[:, :-8].contiguous()
     qw, kw = ((torch.rand(D, device=DEV) + 0.5).to(dtype) for _ in range(2))
-    rope = RotaryCache(D, 4096, 1e6).to(DEV)
+    rope = RotaryCache(D, 8192, 1e6).to(DEV)
     before = [kc.clone(), vc.clone(), proj.clone()]
     got = fused.decode_attention(proj, qw, kw, rope.cos_sin_cache, step.positions, heads, kv_heads, D, 1e-6, kc, vc, step)
     # the caches as the launch of its own leaves them
@@ -72,6 +76,30 @@ def test_qwen3_step(ctx, kv_heads, heads, block_size, dtype):
         k, v = (c[blocks[b]].flatten(0, 1)[:n].double().repeat_interleave(heads // kv_heads, 1) for c in (kc, vc))
         w = torch.softmax(torch.einsum("hd,nhd->hn", q, k) * D ** -0.5, -1)
         _close(got[b], torch.einsum("hn,nhd->hd", w, v).flatten(), dtype)
+
+
+@pytest.mark.parametrize("ctx,kv_heads,heads", [((9000,), 1, 8), ((16384, 5000), 2, 4), ((20000, 0, 8193), 1, 17), ((40000,), 8, 8)], ids=str)
+@torch.no_grad()
+def test_long_sequences_over_several_clusters(ctx, kv_heads, heads):
+    """Sequences whose clusters' shares a second launch adds, long ones beside short and missing ones."""
+    from nanoquantization_b200 import _lib
+    from nanoquantization_b200.layers import fused
+    from nanoquantization_b200.models import RotaryCache
+    dtype = torch.bfloat16
+    step, blocks, kc, vc, proj = _setup([n or 1 for n in ctx], kv_heads, heads, 256, dtype)
+    assert _lib.load().nqb200_decode_attention_scratch_bytes(step.width, 256, len(ctx), heads, kv_heads) > 0
+    proj = proj[:, :-8].contiguous()
+    w = torch.ones(D, device=DEV, dtype=dtype)
+    rope = RotaryCache(D, 1 << 16, 1e6).to(DEV)
+    step.ctx.copy_(torch.tensor(ctx))
+    got = fused.decode_attention(proj, w, w, rope.cos_sin_cache, step.positions, heads, kv_heads, D, 1e-6, kc, vc, step)
+    for b, n in enumerate(ctx):
+        if not n:
+            assert not got[b].any()
+            continue
+        q = _rotate(_rms(proj[b, :heads * D].double().view(heads, D), w), n - 1, D, 1e6)
+        k, v = (c[blocks[b]].flatten(0, 1)[:n].double().repeat_interleave(heads // kv_heads, 1) for c in (kc, vc))
+        _close(got[b], torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q, k) * D ** -0.5, -1), v).flatten(), dtype)
 
 
 @pytest.mark.parametrize("ctx", [(0,), (0, 17, 0, 300, 0), (0,) * 3 + (5000,)], ids=str)
