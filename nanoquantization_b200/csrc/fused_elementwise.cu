@@ -245,34 +245,43 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const uint16_t* __restric
   }
 }
 
-// The same, eight values per thread at a time: bound by memory (6 bytes per result), whole 16-byte pieces.  Two pieces per
-// thread under way at once.  3000 x 12288, bfloat16: 120 us
-// element by element, 51 us so (4.3 TB/s; the exponential and the division, which are as before, take about as long).
-template <bool BF16>
-__global__ void __launch_bounds__(256) silu_mul_vec_kernel(const uint16_t* __restrict__ gate_up, uint16_t* __restrict__ out, int I8) {
+// The same, in pieces of E values (whole words of 4, 8 or 16 bytes), P pieces per thread under way at once; pieces are numbered
+// through all rows, so that no thread idles at a row's end.  The exponential and the
+// division of a call's last values are what a small call waits for, so that pieces are short where there are few of them; large calls
+// are bound by memory (6 bytes per result) and take 16 bytes at a time.  bfloat16, us by pieces of 1, 2, 4, 8 values and of two times 8:
+// 17 x 3072 1.53, 1.23, 1.36, 1.59, 2.17; 300 x 3072 4.91, 2.86, 2.76, 3.31, 3.55; 1000 x 4096 15.5, 10.1, 7.85, 7.10, 7.82; 4000 x 12288
+// 152, 101, 73.6, 61.7, 58.7 (5.0 TB/s).
+template <int E> struct Piece;
+template <> struct Piece<2> { using type = uint32_t; };
+template <> struct Piece<4> { using type = uint2; };
+template <> struct Piece<8> { using type = uint4; };
+template <bool BF16, int E, int P>
+__global__ void __launch_bounds__(256) silu_mul_vec_kernel(const uint16_t* __restrict__ gate_up, uint16_t* __restrict__ out, uint32_t pieces, uint32_t per_row) {
+  using W = typename Piece<E>::type;
+  union Values { W w; uint16_t v[E]; };
   grid_launch_dependents();
   grid_dependency_wait();
-  const int64_t t = blockIdx.y;
-  const uint4* gate = reinterpret_cast<const uint4*>(gate_up) + t * 2 * I8;
-  uint4* o = reinterpret_cast<uint4*>(out) + t * I8;
-  const int c0 = blockIdx.x * 512 + threadIdx.x;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  uint4 g[2], u[2];
+  const uint32_t first = blockIdx.x * (256u * P) + threadIdx.x;
+  Values g[P], u[P];
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int c = c0 + 256 * j;
-    g[j] = c < I8 ? gate[c] : zero;
-    u[j] = c < I8 ? gate[I8 + c] : zero;
+  for (int j = 0; j < P; ++j) {
+    const uint32_t at = first + 256u * j;
+    if (at < pieces) {
+      const W* row = reinterpret_cast<const W*>(gate_up) + at + (size_t)(at / per_row) * per_row;
+      g[j].w = row[0];
+      u[j].w = row[per_row];
+    }
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    float a[8], b[8];
-    unpack8<BF16>(g[j], a);
-    unpack8<BF16>(u[j], b);
+  for (int j = 0; j < P; ++j) {
+    const uint32_t at = first + 256u * j;
+    if (at >= pieces) break;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = rnd16<BF16>(a[e] / (1.f + expf(-a[e]))) * b[e];
-    const int c = c0 + 256 * j;
-    if (c < I8) o[c] = pack8<BF16>(a);
+    for (int e = 0; e < E; ++e) {
+      const float a = raw16_to_float<BF16>(g[j].v[e]);
+      g[j].v[e] = float_to_raw16<BF16>(rnd16<BF16>(a / (1.f + expf(-a))) * raw16_to_float<BF16>(u[j].v[e]));
+    }
+    reinterpret_cast<W*>(out)[at] = g[j].w;
   }
 }
 
@@ -348,10 +357,19 @@ extern "C" int nqb200_silu_mul(const void* gate_up, void* out, int64_t T, int64_
   if (dtype != NQB200_F16 && dtype != NQB200_BF16) return NQB200_ERR_BAD_DTYPE;
   if (T == 0) return NQB200_OK;
   if (!gate_up || !out) return NQB200_ERR_NULL_POINTER;
-  if (I % 8 == 0 && T <= 65535 && aligned16(gate_up) && aligned16(out))
-    return launch_overlapped(dtype == NQB200_BF16 ? silu_mul_vec_kernel<true> : silu_mul_vec_kernel<false>,
-                             dim3((unsigned)((I / 8 + 511) / 512), (unsigned)T), dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)gate_up,
-                             (uint16_t*)out, (int)(I / 8));
+  // where the piece grows: the times at the kernel cross between 0.3 and 0.4, 1.3 and 3, 8 and 16 million values
+  const auto whole = [&](int e) {
+    return I % e == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & (2 * e - 1)) == 0 && T <= INT32_MAX / (I / e);
+  };
+#define NQB200_SILU(E, P)                                                                                                             \
+  return launch_overlapped(dtype == NQB200_BF16 ? silu_mul_vec_kernel<true, E, P> : silu_mul_vec_kernel<false, E, P>,                    \
+                           dim3((unsigned)((T * (I / E) + 256 * P - 1) / (256 * P))), dim3(256), 0, (cudaStream_t)stream,                \
+                           (const uint16_t*)gate_up, (uint16_t*)out, (uint32_t)(T * (I / E)), (uint32_t)(I / E))
+  if (whole(8) && T >= 12000000 / I) NQB200_SILU(8, 2);
+  if (whole(8) && T >= 2400000 / I) NQB200_SILU(8, 1);
+  if (whole(4) && T >= 320000 / I) NQB200_SILU(4, 1);
+  if (whole(2)) NQB200_SILU(2, 1);
+#undef NQB200_SILU
   const int64_t total = T * I;
   const int64_t want = (total + 255) / 256;
   const unsigned blocks = (unsigned)(want < (int64_t)kNumSMs * 16 ? want : (int64_t)kNumSMs * 16);

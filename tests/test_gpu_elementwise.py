@@ -30,7 +30,8 @@ def test_add_rmsnorm(T, H, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("T,width", [(1, 8), (3, 100), (2, 4096), (2, 4104), (70000, 8)])
+@pytest.mark.parametrize("T,width", [(1, 8), (3, 100), (2, 4096), (2, 4104), (70000, 8),
+                                     (3, 6), (3, 7), (20, 16004), (600, 4004), (600, 4010), (801, 15000), (1501, 8008)])
 @torch.no_grad()
 def test_silu_mul(T, width, dtype):
     from nanoquantization_b200.layers import fused
