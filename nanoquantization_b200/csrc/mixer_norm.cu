@@ -139,14 +139,16 @@ __global__ void __launch_bounds__(256) stream_add_vec_kernel(float* __restrict__
 }
 
 // The same for widths that are multiples of 4 and short filters: float4 accesses, and the last taps - 1 rows of h
-// stay in registers while a thread walks down the tile's tokens.  Bound by memory, so both passes over x (the second comes
-// from L2) keep eight loads of a thread under way.  8192 x 4096, four taps, bfloat16: 88 us with four, 80 with eight (2.5 TB/s).
+// stay in registers while a thread walks down the tile's tokens.  Bound by memory where tiles fill the chip, else by the walk.
+// WIDE: eight loads of a thread under way in both passes over x (the second comes from L2) instead of four.  8000 x 4096, us with
+// four and with eight: two taps 67.4 and 59.3, four 84.0 and 75.9, five 67.3 and 61.9 (bfloat16); but four taps in float32 85.3 and
+// 86.2, five 73.0 and 100.8 (registers), and 1000 x 4096 with four taps 24.7 and 26.5.
 constexpr int kConvTile = 16;
-template <typename T, int TAPS>
+template <typename T, int TAPS, bool WIDE>
 __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __restrict__ x, const float* __restrict__ weight,
                                                                const float* __restrict__ conv, float* state, T* __restrict__ out,
                                                                const nqb200_batch bt, int width, float eps) {
-  constexpr int HALO = TAPS - 1;
+  constexpr int HALO = TAPS - 1, ROWS = WIDE ? 8 : 4;
   __shared__ float inv_s[kConvTile + 2 * HALO];
   grid_launch_dependents();
   grid_dependency_wait();
@@ -159,12 +161,19 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __re
     if (tok < 0 || tok >= n) continue;
     const float* row = x + (size_t)(t0 + tok) * width;
     float ss = 0.f;
-    for (int c0 = lane * 4; c0 < width; c0 += 1024) {   // eight pieces of the row under way at once
-      float4 v[8];
+    if (WIDE) {
+      for (int c0 = lane * 4; c0 < width; c0 += 1024) {
+        float4 v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = c0 + 128 * j < width ? ld4(row + c0 + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < 8; ++j) v[j] = c0 + 128 * j < width ? ld4(row + c0 + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+        for (int j = 0; j < 8; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+      }
+    } else {
+      for (int c = lane * 4; c < width; c += 128) {
+        const float4 v = ld4(row + c);
+        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+      }
     }
     ss = warp_sum(ss);
     if (lane == 0) inv_s[r] = 1.f / sqrtf(ss / (float)width + eps);
@@ -187,7 +196,7 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __re
       const int src = first - HALO + j;
       win[j] = src >= 0 ? mul4(scale4(ld4(x + (size_t)(t0 + src) * width + c), inv_s[j]), w) : old[j];
     }
-#pragma unroll 8
+#pragma unroll ROWS
     for (int i = 0; i < cnt; ++i) {
       const float4 h = mul4(scale4(ld4(x + (size_t)(t0 + first + i) * width + c), inv_s[HALO + i]), w);
       float4 acc = h;
@@ -318,11 +327,15 @@ static int launch_rmsnorm_conv(const float* x, const float* weight, const float*
   const dim3 block(256);
   if (vec && taps >= 2 && taps <= 5) {
     const dim3 grid((unsigned)((b->max_len + kConvTile - 1) / kConvTile), (unsigned)b->batch);
-#define NQB200_CONV(K) return launch_overlapped(rmsnorm_conv_vec_kernel<T, K>, grid, block, 0, st, x, weight, conv, state, out, *b, width, eps)
-    if (taps == 2) NQB200_CONV(2);
-    if (taps == 3) NQB200_CONV(3);
-    if (taps == 4) NQB200_CONV(4);
-    NQB200_CONV(5);
+    constexpr bool half = sizeof(T) == 2;
+    // the measurements at the kernel; three taps are slower with eight at every size
+    const bool full = (int64_t)grid.x * grid.y > 2 * kNumSMs;
+#define NQB200_CONV(K, W) return launch_overlapped(rmsnorm_conv_vec_kernel<T, K, W>, grid, block, 0, st, x, weight, conv, state, out, *b, width, eps)
+    if (taps == 2) NQB200_CONV(2, true);
+    if (taps == 3) NQB200_CONV(3, false);
+    if (taps == 4 && half && full) NQB200_CONV(4, half);
+    if (taps == 4) NQB200_CONV(4, false);
+    NQB200_CONV(5, half);
 #undef NQB200_CONV
   }
   const int halo = taps - 1, tile = halo > 8 ? halo : 8;

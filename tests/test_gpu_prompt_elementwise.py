@@ -118,6 +118,29 @@ def test_norm_and_convolution_of_prompts(width):
         o += n
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps", [2, 3, 4, 5])
+@pytest.mark.parametrize("lens,width", [((33, 17, 1), 132), ((16,), 1024), ((4801,), 36), ((4736, 3), 36)], ids=str)
+@torch.no_grad()
+def test_convolutions_of_prompts_by_taps_and_type(lens, width, taps, dtype):
+    """Every number of taps in both types, on both sides of the number of tiles from which more rows are under way."""
+    step, _ = _step(lens, [0] * len(lens))
+    x, w, cw = torch.randn(sum(lens), width, device=DEV), 1 + 0.2 * torch.randn(width, device=DEV), torch.randn(taps, width, device=DEV)
+    state = torch.full((len(lens), taps - 1, width), 9.0, device=DEV)
+    got = ops.rmsnorm_conv(x, w, cw, state, step, 1e-6, dtype)
+    o = 0
+    for b, n in enumerate(lens):
+        h = x[o:o + n].double()
+        h = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        full = torch.cat([torch.zeros(taps - 1, width, dtype=torch.float64, device=DEV), h])
+        want = h + sum(cw.double()[j] * full[j:j + n] for j in range(taps))
+        # float sums of a few terms of the size of the largest; one rounding to bfloat16
+        limit = 1e-5 if dtype == torch.float32 else 2.0 ** -8
+        assert float((got[o:o + n].double() - want).abs().max()) <= limit * float(want.abs().max())
+        assert float((state[b].double() - full[len(full) - taps + 1:]).abs().max()) <= 1e-5 * float(full.abs().max())
+        o += n
+
+
 @pytest.mark.parametrize("taps", [2, 4, 5])
 @pytest.mark.parametrize("width", [4, 1020, 4096, 4100])
 @torch.no_grad()
