@@ -195,9 +195,8 @@ __global__ void __launch_bounds__(256, 4) norm_rope_vec_kernel(bf16* proj, bf16*
 // The same where the whole head turns and is 16 L elements long: L lanes per head, each with piece c of the lower and of the
 // upper half, which are partners where pairs lie half a head apart, so that nothing but the norm's sum crosses lanes and a
 // warp works on 32 / L heads at once (the kernel above spends its time on instructions: half of its lanes idle at 128, eight
-// shuffles a head).  8192 tokens, 32 + 8 heads of
-// 128, with the cache: 96 us by the kernel that took it before, element by element, 42 us so; 5000 tokens with norms and
-// neighbouring pairs: 61 and 27 us.
+// shuffles a head).  8192 tokens, 32 + 8 heads of 128, with the cache: 96 us element by element, 42 us so; 5000 tokens with norms and
+// neighbouring pairs: 61 us by the kernel above, 27 us so.
 template <bool NEIGHBOURS, int L>
 __global__ void __launch_bounds__(256) rope_full_kernel(bf16* proj, bf16* k_cache, bf16* v_cache, const nqb200_rope r, const nqb200_batch bt, int64_t stride,
                                                         int q_off, int k_off, int v_off, int span) {
@@ -242,6 +241,7 @@ __global__ void __launch_bounds__(256) rope_full_kernel(bf16* proj, bf16* k_cach
     if (i0 + U * PER < items) request(i0 + U * PER);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
+      if (i0 + u * PER >= items) break;   // the last pass may be empty for everyone
       const int at = i0 + u * PER + own, it = min(at, items - 1), tk = token_of(it), hd = it - tk * heads;
       float x[8], z[8];
       unpack8(lo[u], x);
@@ -376,15 +376,26 @@ static bool rope_pieces(const void* proj, const void* k_cache, const void* v_cac
          k_off % 8 == 0 && aligned16(proj) && (!r->q_norm || r->k_norm) && (r->q_norm || !r->k_norm) &&
          (!k_cache || (aligned16(k_cache) && aligned16(v_cache) && r->vdim % 8 == 0 && v_off % 8 == 0));
 }
+// Whole heads that turn, by rope_full_kernel: where its lanes have heads to work on.  us by the kernel that takes the call otherwise
+// (rope_store_kernel: stored, or norm_rope_vec_kernel with norms) and by this one, heads of 128: 1 token of 4 + 1 heads 2.2 and 2.3,
+// 2.65 and 2.5; of 16 + 4 heads 3.5 and 2.3, 3.8 and 2.5; 1000 tokens of 4 + 1 heads 3.9 and 3.0, 6.2 and 3.5; of 1 + 1 3.1 and 3.0, 4.1
+// and 3.4, but 8000 with norms 12.1 and 12.7.
+constexpr int kRopeFullCtas = 3 * kNumSMs;   // resident at once
+static bool rope_full_pays(const nqb200_rope* r, const nqb200_batch* b, bool stored) {
+  const int64_t heads = r->heads + r->kv_heads;
+  if (r->rot != r->dim || (r->dim != 64 && r->dim != 128 && r->dim != 256)) return false;
+  return b->max_len > kRopeFullCtas ? heads >= 5 : stored ? heads * r->dim >= 1024 : heads >= 8;
+}
 static int launch_rope_pieces(void* proj, void* k_cache, void* v_cache, const nqb200_rope* r, const nqb200_batch* b, int64_t stride, int64_t q_off,
-                              int64_t k_off, int64_t v_off, cudaStream_t s) {
+                              int64_t k_off, int64_t v_off, bool stored, cudaStream_t s) {
   auto kernel = r->interleaved ? norm_rope_vec_kernel<true> : norm_rope_vec_kernel<false>;
-  if (r->rot == r->dim) {
+  const bool full = rope_full_pays(r, b, stored);
+  if (full) {
     if (r->dim == 64) kernel = r->interleaved ? rope_full_kernel<true, 4> : rope_full_kernel<false, 4>;
     if (r->dim == 128) kernel = r->interleaved ? rope_full_kernel<true, 8> : rope_full_kernel<false, 8>;
     if (r->dim == 256) kernel = r->interleaved ? rope_full_kernel<true, 16> : rope_full_kernel<false, 16>;
   }
-  const int span = b->max_len >= 4 * kNumSMs ? kRopeSpan : 1;
+  const int span = b->max_len > (full ? kRopeFullCtas : 4 * kNumSMs - 1) ? kRopeSpan : 1;   // one token a CTA while all CTAs are resident
   return launch_overlapped(kernel, dim3((unsigned)((b->max_len + span - 1) / span), (unsigned)b->batch), dim3(256),
                            (size_t)(2 * r->dim + span * r->rot) * sizeof(float), s, (bf16*)proj, (bf16*)k_cache, (bf16*)v_cache, *r, *b, stride, (int)q_off,
                            (int)k_off, (int)v_off, span);
@@ -401,8 +412,11 @@ extern "C" int nqb200_rope_store(void* proj, void* k_cache, void* v_cache, const
   if (!proj || !k_cache || !v_cache || (rot > 0 && !inv_freq)) return NQB200_ERR_NULL_POINTER;
   if (heads <= INT32_MAX / 256 && kv_heads <= INT32_MAX / 256 && dim <= 256 && vdim <= INT32_MAX) {
     const nqb200_rope r = {(int32_t)heads, (int32_t)kv_heads, (int32_t)dim, (int32_t)vdim, (int32_t)rot, 0, inv_freq, nullptr, nullptr, 0.f};
-    if (rope_pieces(proj, k_cache, v_cache, &r, stride, q_off, k_off, v_off, dtype))
-      return launch_rope_pieces(proj, k_cache, v_cache, &r, b, stride, q_off, k_off, v_off, (cudaStream_t)stream);
+    // heads that turn in part: in pieces of 8 where there are many heads and a CTA takes one token, else by the kernel below (32 + 8 heads
+    // of 128, half of which turns: 400 tokens 8.0 us in pieces, 10.4 below; 1000 tokens 22.8 and 15.0; 4 + 1 heads, 100 tokens 2.7 and 2.4)
+    const bool part = rot != dim && (heads + kv_heads) * dim >= 1024 && b->max_len < 4 * kNumSMs;
+    if ((part || rope_full_pays(&r, b, true)) && rope_pieces(proj, k_cache, v_cache, &r, stride, q_off, k_off, v_off, dtype))
+      return launch_rope_pieces(proj, k_cache, v_cache, &r, b, stride, q_off, k_off, v_off, true, (cudaStream_t)stream);
   }
   const dim3 grid((unsigned)b->max_len, (unsigned)b->batch), block(256);
   const size_t smem = (size_t)rot * sizeof(float);
@@ -428,7 +442,7 @@ extern "C" int nqb200_norm_rope(void* proj, void* k_cache, void* v_cache, const 
   const size_t smem = (size_t)r->rot * sizeof(float);
   cudaStream_t s = (cudaStream_t)stream;
   if (rope_pieces(proj, k_cache, v_cache, r, stride, q_off, k_off, v_off, dtype))
-    return launch_rope_pieces(proj, k_cache, v_cache, r, b, stride, q_off, k_off, v_off, s);
+    return launch_rope_pieces(proj, k_cache, v_cache, r, b, stride, q_off, k_off, v_off, false, s);
   if (dtype == NQB200_F32)
     return launch_overlapped(norm_rope_kernel<float>, grid, block, smem, s, (float*)proj, (float*)k_cache, (float*)v_cache, *r, *b, stride,
                              (int)q_off, (int)k_off, (int)v_off);

@@ -21,7 +21,7 @@ def _step(lens, starts, block_size=16):
 @pytest.mark.parametrize("cached,normed", [(True, True), (True, False), (False, False)])
 @pytest.mark.parametrize("neighbours", [False, True])
 @pytest.mark.parametrize("dim,rot", [(64, 64), (128, 128), (256, 256), (128, 64), (96, 96)])
-@pytest.mark.parametrize("lens,heads,kv_heads", [((1,), 1, 1), ((3, 2), 5, 2), ((595, 30), 3, 1)], ids=str)
+@pytest.mark.parametrize("lens,heads,kv_heads", [((1,), 1, 1), ((3, 2), 5, 2), ((595, 30), 3, 1), ((3, 1), 13, 4), ((595, 30), 12, 5), ((593,), 4, 1)], ids=str)
 @torch.no_grad()
 def test_rotation(lens, heads, kv_heads, dim, rot, neighbours, cached, normed):
     """One token, a few, and enough for four tokens per block with a remainder; whole heads that turn and parts of them."""
