@@ -31,13 +31,11 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int MODE, int MT>
-__global__ void __launch_bounds__(256, MT == 1 ? 3 : 2) dense_decode_kernel(const DenseArgs p) {
+// SHORT: half as many k-blocks in flight per warp, which leaves registers for three CTAs per SM (up to eight tokens).
+template <int MODE, int MT, bool SHORT>
+__global__ void __launch_bounds__(256, SHORT && MT == 1 ? 3 : MODE == kMinGru && MT == 2 ? 1 : 2) dense_decode_kernel(const DenseArgs p) {
   constexpr int NG = MODE == kMinGru ? 3 : MODE == kGlu ? 2 : 1;      // row groups that meet in one output
-  // k-blocks in flight per warp.  Fewer of them and more CTAs per SM keep the memory busier than twice as many that the warp
-  // then works off at once while nothing is under way: decode step of 3, 8 and 16 sequences of Vemedra layers 566, 678 and 681
-  // us with twice as many (and two CTAs per SM), 477, 554 and 639 so; with three quarters of these 537, 629, 663.
-  constexpr int U = MODE == kMinGru ? (MT == 1 ? 1 : 2) : MODE == kGlu ? 2 : 4;
+  constexpr int U = (MODE == kMinGru ? 2 : MODE == kGlu ? 4 : 8) / (SHORT ? 2 : 1);   // k-blocks in flight per warp
   __shared__ float part[8][NG][MT * 8][16 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * 16, blocks = (p.K + 31) / 32;
@@ -130,12 +128,29 @@ static int launch_dense(const DenseArgs& p, cudaStream_t st) {
   if (!p.x || !p.w || !p.out) return NQB200_ERR_NULL_POINTER;
   if (!aligned16(p.x) || !aligned16(p.w)) return NQB200_ERR_MISALIGNED;
   const dim3 grid((unsigned)((p.N + 15) / 16)), block(256);
+#define NQB200_DENSE(MT, SHORT)                              \
+  do {                                                        \
+    prefer_loads<dense_decode_kernel<MODE, MT, SHORT>>();      \
+    return launch_overlapped(dense_decode_kernel<MODE, MT, SHORT>, grid, block, 0, st, p); \
+  } while (0)
+  // Which of the two, us long and short, in chains of calls:
+  // - one request holds all of K either way (1024; 512 of the unit's two matrices): short.  16 tokens, 1024 -> 4096 3.4 long,
+  //   2.9 short.
+  // - up to eight tokens: short where three CTAs per SM are a wave less than two, of the unit only where they are the one wave.  1
+  //   token, 4096 -> 6144 (384 CTAs) 12.4 long, 9.0 short; 4096 -> 8192 (512) 12.6, 14.2; 2048 -> 2048 (128) 2.2, 3.3.
+  // - up to sixteen: short where the weights are long in coming; 2048 columns are one request of the long form, which pays longer.
+  //   16 tokens, 4096 -> 4096 (16.8 M) 8.7 long, 8.0 short; 4096 -> 2048 6.5, 7.0; 2048 -> 6144 (12.6 M) 7.6, 8.0.
+  // minGRU's three matrices: long always (1 token, 4096 -> 3 x 4096 18.1 long, 21.5 short).
+  constexpr bool unit = MODE == kGlu, gru = MODE == kMinGru;
+  const int64_t ctas = grid.x, two = (ctas + 2 * kNumSMs - 1) / (2 * kNumSMs), three = (ctas + 3 * kNumSMs - 1) / (3 * kNumSMs);
+  const bool once = p.K <= (unit ? 512 : 1024);
   if (p.M <= 8) {
-    prefer_loads<dense_decode_kernel<MODE, 1>>();
-    return launch_overlapped(dense_decode_kernel<MODE, 1>, grid, block, 0, st, p);
+    if (!gru && (once || (unit ? three == 1 && two == 2 : three < two))) NQB200_DENSE(1, !gru);
+    NQB200_DENSE(1, false);
   }
-  prefer_loads<dense_decode_kernel<MODE, 2>>();
-  return launch_overlapped(dense_decode_kernel<MODE, 2>, grid, block, 0, st, p);
+  if (!gru && (once || (!unit && (int64_t)p.N * p.K >= (p.K > 2048 ? 12000000 : 16000000)))) NQB200_DENSE(2, !gru);
+  NQB200_DENSE(2, false);
+#undef NQB200_DENSE
 }
 
 }  // namespace nqb200

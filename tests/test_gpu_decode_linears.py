@@ -1,0 +1,50 @@
+"""The linears of decode steps on both sides of the sizes at which their kernel changes how much a warp has under way, against
+float64."""
+import pytest
+import torch
+
+from nanoquantization_b200.engine.batch import StepBatch
+from nanoquantization_b200.layers import mixers as ops
+
+pytestmark = pytest.mark.gpu
+DEV, bf = "cuda", torch.bfloat16
+
+
+def _step(batch, position):
+    return StepBatch.host([[0]] * batch, [position] * batch, [[i] for i in range(batch)], list(range(batch)), 1, 256).to(DEV)
+
+
+def _close(got, want, limit):
+    assert float((got.double() - want).norm()) <= limit * float(want.norm())
+
+
+# one request holds K or not (512, 1024, 2048), a wave of two or three CTAs per SM or more (296, 444 CTAs of 16 outputs), many weights or few
+SIZES = [(1, 512, 40), (1, 520, 40), (8, 1024, 64), (8, 1032, 64), (5, 1032, 4736), (5, 1032, 4752), (3, 1032, 7104), (3, 1032, 7120), (9, 1024, 64), (16, 2048, 8000),
+         (16, 2056, 5848), (16, 2056, 5824), (12, 4096, 2928), (16, 5000, 37)]
+
+
+@pytest.mark.parametrize("M,K,N", SIZES)
+@torch.no_grad()
+def test_linears(M, K, N):
+    """Tolerance: eight warps' chains of K / 128 tensor-core additions and the sum of the eight, each good to 2^-23; one rounding to
+    bfloat16 (2^-9 in the 2-norm) where the result has that type."""
+    exact = (K / 128 + 8) * 2.0 ** -23
+    x, w, beta = torch.randn(M, K, device=DEV).to(bf), (torch.randn(N, K, device=DEV) * K ** -0.5).to(bf), 0.5
+    want = x.double() @ w.double().t()
+    _close(ops.linear(x, w), want, 2.0 ** -8)
+    _close(ops.linear(x, w, torch.float32), want, exact)
+    stream = torch.randn(M, N, device=DEV)
+    total = beta * stream.double() + want
+    _close(ops.linear_residual_(stream, x, w, beta), total, exact)
+    # the unit's product has two matrices, minGRU's three: rows of w as they come
+    half = N // 2
+    gate, up = want[:, :half].clamp(max=0.7), want[:, half:2 * half].clamp(-0.7, 0.7)
+    _close(ops.dense_glu(x, w[:2 * half], 0.7), gate * torch.sigmoid(1.702 * gate) * (up + 1), 2.0 ** -8)
+    third = N // 3
+    zb, xb, state = (torch.randn(n, device=DEV) for n in (third, third, M * third))
+    state = state.view(M, third)
+    z, u = torch.sigmoid(want[:, :third] + zb.double()), want[:, third:2 * third] + xb.double()
+    s = (1 - z) * state.double() + z * torch.where(u >= 0, u + 0.5, torch.sigmoid(u))
+    got = ops.dense_mingru(x, w[:3 * third], zb, xb, state, _step(M, 3))
+    _close(state, s, exact)
+    _close(got, s * torch.nn.functional.silu(want[:, 2 * third:3 * third]), 2.0 ** -8)
