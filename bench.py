@@ -910,13 +910,9 @@ def vemedra_kernels(dev, peaks, T=8192, context=2048):
         add(ph, "attention + retention", _device_us(both, 2 * n), kv_bytes + st_bytes)
         add(ph, "  attention alone", _device_us(lambda i: ops.mixer_decode(pr, ac, (d, att.rope_desc(), 0, att.value_column(0), 0, copies[i % n][0], copies[i % n][1]), None, s), 2 * n), kv_bytes)
         add(ph, "  retention alone", _device_us(lambda i: ops.mixer_decode(pr, ac, None, (ret, off, H * D, copies[i % n][2]), s), 2 * n), st_bytes)
-        try:
-            from flash_attn import flash_attn_with_kvcache
-            q1 = rnd(B, 1, H, D)
-            add(ph, "Qwen3: flash_attn_with_kvcache", _device_us(lambda i: flash_attn_with_kvcache(
-                q1, copies[i % n][0], copies[i % n][1], cache_seqlens=s.ctx, block_table=s.table, causal=True), 2 * n), kv_bytes)
-        except ImportError:
-            pass
+        qkv1 = rnd(B, (H + 2 * G) * D)
+        add(ph, "Qwen3: QK-norm + rotary + K/V store + attention", _device_us(lambda i: fused.decode_attention(
+            qkv1, qn, qn, cs, s.positions, H, G, D, 1e-6, copies[i % n][0], copies[i % n][1], s), 2 * n), kv_bytes)
         add(ph, "rmsnorm + convolution", _device_us(lambda i: ops.rmsnorm_conv(stream, nw, cw, cst, s, 1e-6, dt), 16), B * W * (6 + 24) + W * 20)
         add(ph, "Qwen3: residual add + rmsnorm", _device_us(lambda i: fused.add_rmsnorm(h, h, n16, 1e-6), 16), B * W * 8)
         del copies

@@ -565,9 +565,10 @@ static Plan make_plan(int64_t M, int64_t N, int64_t K) {
   Plan pl;
   pl.ctas = 2;
   const int64_t cap = 128 * pl.ctas, unit = 16 * pl.ctas;   // each CTA's share is a multiple of 16 tokens
-  // as few token tiles as hold M, all alike: a last tile of a few tokens would cost as much as a full one.  In chains
-  // of calls, bfloat16: K = 5120, N = 25600 at 777 tokens (tiles of 224) 198 -> 186 us, at 1025 (224) 252 -> 240; K = 12288,
-  // N = 4096 at 640 70.3 -> 68.6; between 0 and 6 % over 513 to 2100 tokens.
+  // as few token tiles as hold M, all alike: a last tile of a few tokens would cost as much as a full one.  27 sizes from 200 to
+  // 3000 tokens by 7 shapes, K x N, in turns with tiles of 256: 0.6 % faster in the mean; 25600 x 5120 at 320 tokens (tiles of 160) 112
+  // -> 107 us, 4096 x 4096 at 513 (192) 28.7 -> 27.5, 1024 x 6144 at 1281 (which the single-CTA kernel took) 26.7 -> 19.4; the one
+  // loss that repeats is 12288 x 4096 at 600 (224), 70.6 -> 71.8.
   pl.ntt = (int)((M + cap - 1) / cap);
   pl.NT = (int)(((M + pl.ntt - 1) / pl.ntt + unit - 1) / unit * unit);
   pl.TH = pl.NT / pl.ctas;
@@ -579,10 +580,11 @@ static Plan make_plan(int64_t M, int64_t N, int64_t K) {
   // and a second kernel, and the clusters drift apart in k, so that the activations (which all column tiles of a
   // token tile share) are fetched from L2 at scattered times: measured 0.95 us per unit + 10 us.  Whole tiles keep
   // the clusters in step (0.78 us per unit in a full wave) and lose only the last wave's idle clusters, which
-  // itself runs faster the emptier it is (0.6 to 0.8 us per unit).  Fitted on M in 192..4096 x the sweep's five
-  // shapes, where it picks the faster dealing every time.  Whichever ends first:
+  // itself runs faster the emptier it is (0.6 to 0.8 us per unit).  Fitted with tiles of 256 tokens on M in
+  // 192..4096 x the sweep's five shapes.  The estimates rank the two dealings, they do not predict: calls in chains take 1.0 to 1.4
+  // times as long, most with small tiles (K = 12288, N = 4096: 777 tokens 65 estimated, 71 to 85 measured).  Whichever ends first:
   const long long full = items / maxc, rem = items % maxc;
-  // A unit of fewer tokens takes that much less, down to what the dequantisers take.
+  // A unit of fewer tokens is taken to be that much shorter, by an eighth at most.
   const double part = pl.ntt > 1 ? std::max(pl.NT / (double)cap, 0.875) : 1.0;
   const double t_whole = part * G * (0.78 * (double)full + (rem ? 0.6 + 0.2 * (double)rem / (double)maxc : 0.0));
   const double t_stream = part * 0.95 * (double)((pl.U + maxc - 1) / maxc) + 10.0;
@@ -646,7 +648,7 @@ bool umma_pair_supports(int64_t M, int64_t N, int64_t K, int64_t g) {
   if (!(M > 128 && g == 128 && K % 128 == 0 && N % 32 == 0)) return false;
   // Against the single-CTA kernel: its own cost model's estimate for the shape, less the 10 us by which this
   // kernel's fixed cost (cluster launch, tensor-memory allocation for a pair, a deeper pipeline to fill) exceeds
-  // that kernel's.  Over M in 192..4096 x the sweep's five shapes this rule picks the faster kernel every time.
+  // that kernel's.  Fitted with tiles of 256 tokens on M in 192..4096 x the sweep's five shapes.
   const pair::Plan pl = pair::make_plan(M, N, K);
   if ((pl.U + 1) * pl.nclusters >= (1ll << 31)) return false;   // the kernel's 32-bit unit arithmetic
   return pl.est_us <= umma_prefill_estimate_us(M, N, K) - 10.0;

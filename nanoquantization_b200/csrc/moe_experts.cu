@@ -71,9 +71,9 @@ __device__ __forceinline__ void moe_mma(float (&c)[4], uint32_t a0, uint32_t a1,
 
 template <typename O, int MT>
 __global__ void __launch_bounds__(256, 3) moe_decode_kernel(const MoeDevice p) {
-  // k-blocks in flight per warp, as in the dense linears: eight, with two CTAs per SM, took a decode step of 1, 5 and 14
-  // sequences of Verozen layers (both kernels changed together) 486, 916 and 1543 us; four and six 427, 821 and 1342; so it
-  // takes 427, 797 and 1270.
+  // k-blocks in flight per warp: few of them and three CTAs per SM keep the memory busier than eight, with two CTAs, that a warp
+  // then works off at once while nothing is under way.  64 experts of 1536, 8 per token, width 4096, first and second linear: 1
+  // token 24.5 and 22.7 us with eight, 20.8 and 18.7 so; 8 tokens 95 and 104, 86 and 87; 16 tokens 156 and 180, 126 and 130.
   constexpr int U = MT == 1 ? 3 : 2;
   __shared__ float part[8][MT * 8][16 + 1];
   grid_launch_dependents();

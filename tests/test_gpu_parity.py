@@ -270,6 +270,13 @@ def test_gemm_sweep_every_point_vs_oracle(K, N, dtype, M):
     (1100, 25600, 5152, torch.float16, True, 2),
     (2048, 25600, 5120, torch.bfloat16, True, 2),
     (700, 5120, 25600, torch.bfloat16, False, 1),
+    # several tiles of equal size below 256: 160 (257 and 320 tokens), 192 (380, and 513 over three), 224 cut in bfloat16
+    (257, 5120, 25600, torch.float16, True, 1),
+    (320, 25600, 5152, torch.bfloat16, True, 2),
+    (380, 5120, 25600, torch.bfloat16, False, 1),
+    (380, 25600, 5152, torch.float16, False, 2),
+    (513, 12288, 4128, torch.float16, True, 1),
+    (1100, 25600, 5120, torch.bfloat16, False, 2),
 ])
 def test_gemm_pair_kernel_ragged(M, K, N, dtype, bias, launches):
     lib = _lib.load()
@@ -291,7 +298,11 @@ def test_gemm_pair_kernel_ragged(M, K, N, dtype, bias, launches):
     y = m(x.to(DEV), out=buf[1:M + 1])
     torch.cuda.synchronize()
     assert bool((buf[0] == -7.25).all()) and bool((buf[M + 1] == -7.25).all())
-    rows = torch.cat([torch.tensor([0, min(255, M - 1), min(256, M - 1), M - 1]), torch.randperm(M, generator=g)[:28]])
+    # both sides of every boundary of the equal token tiles, multiples of 32
+    count = -(-M // 256)
+    tile = -(-(-(-M // count)) // 32) * 32
+    edges = [r for t in range(1, count) for r in (t * tile - 1, t * tile) if r < M]
+    rows = torch.cat([torch.tensor([0, min(255, M - 1), min(256, M - 1), M - 1] + edges), torch.randperm(M, generator=g)[:28]])
     W = O.dequantize(qw, sc, qz)
     ref = x[rows].float() @ W.float()
     if b is not None:
