@@ -321,8 +321,8 @@ __device__ void attention_decode(const DecodeArgs& a, uint8_t* smem, int b, int 
   cl.sync();   // peers may still read this CTA's shared memory
 }
 
-// VEC columns per thread (4 where the value size allows 16-byte rows).
-template <int VEC>
+// VEC columns per thread (4 where the value size allows 16-byte rows), U rows of the state under way per thread.
+template <int VEC, int U>
 __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h, cg::cluster_group& cl) {
   const int tid = threadIdx.x, rank = (int)cl.block_rank(), csize = (int)cl.num_blocks();
   const int D = a.rdim, V = a.rvdim;
@@ -334,43 +334,58 @@ __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h,
   const bool fresh = pos == 0;
   const bf16 *qr = row + a.rq_off + (size_t)h * D, *kr = row + a.rk_off + (size_t)h * D;
   float* st = a.rstate + ((size_t)a.bt.slot[b] * a.ret_heads + h) * D * V;
-  constexpr int U = 8;                        // rows of the state under way per thread
   float S[U][VEC];
   auto fetch = [&](int r0, int step, int col) {
+    const float* sp = st + (size_t)r0 * V + col;
+    const size_t pitch = (size_t)step * V;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int r = r0 + u * step;
-      const float* sp = st + (size_t)r * V + col;
+      if (r0 + u * step >= D) break;              // nor is the row used below
       if (VEC == 4) {
-        const float4 f = (fresh || r >= D) ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(sp);
+        const float4 f = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(sp);
         S[u][0] = f.x; S[u][1 % VEC] = f.y; S[u][2 % VEC] = f.z; S[u][3 % VEC] = f.w;
       } else {
-        S[u][0] = (fresh || r >= D) ? 0.f : *sp;
+        S[u][0] = fresh ? 0.f : *sp;
       }
+      sp += pitch;
     }
   };
-  // The state is what there is to read, and it depends on nothing but the slot: its first rows are requested ahead of the
-  // rotation, the decays and their barriers.  5 sequences, 16 heads of 128 x 256 over
-  // clusters of four, gated: 18.7 us in the chain without, 16.0 with.
+  // The small reads that a thread needs are requested in one go.  Behind them, where every channel has its own decay (a product, two
+  // barriers) the state's first rows; a head's one decay is there too soon for that to pay: 5 sequences, 16 heads of 128 x 256 over
+  // clusters of four, 18.7 us without and 16.0 with, but 8 sequences with fixed decays 10.3 without and 10.75 with.
+  const bool early = a.rd.rank > 0;
+  bf16 rq[2], rk[2], pq, pk, rv[VEC], rg, rl;
+  float fq = 0.f, fd = 0.f;
+  const int pass = 2 * half + tid;
+  if (a.rd.rank > 0) { if (tid < a.rd.rank) rl = row[a.rl_off + tid]; } else { fd = a.rd.decay[h]; }
+  if (tid < half) { fq = a.rd.inv_freq[tid]; rq[0] = qr[tid]; rq[1] = qr[tid + half]; rk[0] = kr[tid]; rk[1] = kr[tid + half]; }
+  if (pass < D) { pq = qr[pass]; pk = kr[pass]; }
+  if (tid < ncol * VEC) rg = row[a.rg_off + (size_t)h * V + c0 * VEC + tid];
   if (ncol > 0) {
-    const int width = min(ncol, kDecThreads), rgi = tid / width;
-    if (rgi < kDecThreads / width) fetch(rgi, kDecThreads / width, (c0 + tid % width) * VEC);
+    const int width = min(ncol, kDecThreads), rgi = tid / width, col = (c0 + tid % width) * VEC;
+    if (rgi < kDecThreads / width) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) rv[i] = row[a.rv_off + (size_t)h * V + col + i];
+      if (early) fetch(rgi, kDecThreads / width, col);
+    }
   }
   for (int e = tid; e < half; e += kDecThreads) {
     float s, c;
-    sincosf((float)pos * a.rd.inv_freq[e], &s, &c);
-    const float qu = to_f(qr[e]), qv = to_f(qr[e + half]), ku = to_f(kr[e]), kv = to_f(kr[e + half]);
+    if (e > tid) { fq = a.rd.inv_freq[e]; rq[0] = qr[e]; rq[1] = qr[e + half]; rk[0] = kr[e]; rk[1] = kr[e + half]; }
+    sincosf((float)pos * fq, &s, &c);
+    const float qu = to_f(rq[0]), qv = to_f(rq[1]), ku = to_f(rk[0]), kv = to_f(rk[1]);
     sm.q[e] = qu * c - qv * s;
     sm.q[e + half] = qv * c + qu * s;
     sm.k[e] = (ku * c - kv * s) * kscale;
     sm.k[e + half] = (kv * c + ku * s) * kscale;
   }
-  for (int e = 2 * half + tid; e < D; e += kDecThreads) {
-    sm.q[e] = to_f(qr[e]);
-    sm.k[e] = to_f(kr[e]) * kscale;
+  for (int e = pass; e < D; e += kDecThreads) {
+    if (e > pass) { pq = qr[e]; pk = kr[e]; }
+    sm.q[e] = to_f(pq);
+    sm.k[e] = to_f(pk) * kscale;
   }
   if (a.rd.rank > 0) {
-    for (int e = tid; e < a.rd.rank; e += kDecThreads) sm.low[e] = to_f(row[a.rl_off + e]);
+    for (int e = tid; e < a.rd.rank; e += kDecThreads) sm.low[e] = to_f(e > tid ? row[a.rl_off + e] : rl);
     __syncthreads();
     const bf16* a2 = reinterpret_cast<const bf16*>(a.rd.a2) + (size_t)h * D * a.rd.rank;
     for (int e = tid; e < D; e += kDecThreads) {
@@ -380,7 +395,7 @@ __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h,
       sm.d[e] = expf(log_sigmoid_f(z + a.rd.a2_bias[h * D + e]) / a.rd.tau);
     }
   } else {
-    for (int e = tid; e < D; e += kDecThreads) sm.d[e] = a.rd.decay[h];
+    for (int e = tid; e < D; e += kDecThreads) sm.d[e] = fd;
   }
   __syncthreads();
   float ss = 0.f;
@@ -392,9 +407,9 @@ __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h,
     for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
     if (rgi < RG) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) v[i] = to_f(row[a.rv_off + (size_t)h * V + col + i]);
+      for (int i = 0; i < VEC; ++i) v[i] = to_f(cb > 0 ? row[a.rv_off + (size_t)h * V + col + i] : rv[i]);
       for (int r0 = rgi; r0 < D; r0 += U * RG) {
-        if (cb > 0 || r0 > rgi) fetch(r0, RG, col);
+        if (!early || cb > 0 || r0 > rgi) fetch(r0, RG, col);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int r = r0 + u * RG;
@@ -434,13 +449,13 @@ __device__ void retention_decode(const DecodeArgs& a, RetSmem& sm, int b, int h,
   const float inv = a.rd.out_scale / sqrtf(tot / (float)V + a.rd.eps);
   for (int e = tid; e < ncol * VEC; e += kDecThreads) {
     const int c = c0 * VEC + e;
-    const float gt = to_f(row[a.rg_off + (size_t)h * V + c]);
+    const float gt = to_f(e > tid ? row[a.rg_off + (size_t)h * V + c] : rg);
     a.act[(size_t)b * a.act_stride + a.r_col + (size_t)h * V + c] = __float2bfloat16_rn(sm.o[e] * inv * (a.rd.norm ? a.rd.norm[c] : 1.f) * (gt * sigmoid_f(gt)));
   }
   cl.sync();
 }
 
-template <int VP, int VEC, int TILE>
+template <int VP, int VEC, int TILE, int U>
 __global__ void __launch_bounds__(kDecThreads, 1) mixer_decode_kernel(const DecodeArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   grid_launch_dependents();
@@ -448,18 +463,18 @@ __global__ void __launch_bounds__(kDecThreads, 1) mixer_decode_kernel(const Deco
   cg::cluster_group cl = cg::this_cluster();
   const int unit = blockIdx.y, b = blockIdx.z;
   if (unit < a.att_clusters) attention_decode<VP, TILE>(a, smem, b, unit, cl);
-  else retention_decode<VEC>(a, *reinterpret_cast<RetSmem*>(smem), b, unit - a.att_clusters, cl);
+  else retention_decode<VEC, U>(a, *reinterpret_cast<RetSmem*>(smem), b, unit - a.att_clusters, cl);
 }
 
-template <int VP, int VEC, int TILE>
+template <int VP, int VEC, int TILE, int U>
 static int launch_decode(const DecodeArgs& a, int csize, cudaStream_t st) {
   size_t smem = a.ret_heads > 0 ? sizeof(RetSmem) : 0;
   const size_t att = a.att_clusters > 0 ? sizeof(AttSmem) + (size_t)kDecStages * att_stage(a.at.dim, VP, TILE) * sizeof(bf16) : 0;
   if (att > smem) smem = att;
   // retention alone streams its states through registers: as prefer_loads()
   const int carveout = a.att_clusters > 0 ? cudaSharedmemCarveoutDefault : 25;
-  if (cudaFuncSetAttribute(mixer_decode_kernel<VP, VEC, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(mixer_decode_kernel<VP, VEC, TILE>, cudaFuncAttributePreferredSharedMemoryCarveout, carveout) != cudaSuccess) {
+  if (cudaFuncSetAttribute(mixer_decode_kernel<VP, VEC, TILE, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaFuncSetAttribute(mixer_decode_kernel<VP, VEC, TILE, U>, cudaFuncAttributePreferredSharedMemoryCarveout, carveout) != cudaSuccess) {
     cudaGetLastError();
     return NQB200_ERR_LAUNCH;
   }
@@ -477,7 +492,7 @@ static int launch_decode(const DecodeArgs& a, int csize, cudaStream_t st) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, mixer_decode_kernel<VP, VEC, TILE>, a) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, mixer_decode_kernel<VP, VEC, TILE, U>, a) != cudaSuccess) {
     cudaGetLastError();
     return NQB200_ERR_LAUNCH;
   }
@@ -564,11 +579,24 @@ extern "C" int nqb200_mixer_decode(const void* proj, int64_t stride, void* act, 
   // states alone: two CTAs per SM at most, so that a head is split over a cluster only where heads are few, because clusters
   // cost more to start and to meet than they spread.  16 sequences of 16 heads of 128 x 256: 18 us unsplit, 24 over two CTAs, 30
   // over four, 50 over eight; 5 sequences: 10 over two, 16 over four, 21 over eight.
-  while (csize < want && units * b->batch * csize * 2 <= (a ? kNumSMs * 3 / 2 : kNumSMs * 2)) csize *= 2;
+  int fits = 1;   // of the sizes 1, 2, 4, 8
+  while (csize < want && (a ? units * b->batch * csize * 2 <= kNumSMs * 3 / 2 : units * b->batch <= attdec::kResident[fits][1])) { csize *= 2; ++fits; }
   cudaStream_t st = (cudaStream_t)stream;
   const bool v4 = !r || r->vdim % 4 == 0;
   // 128 keys a pass where two stages of them fit
-#define NQB200_DEC(VP, TILE) return v4 ? launch_decode<VP, 4, TILE>(p, csize, st) : launch_decode<VP, 1, TILE>(p, csize, st)
+  // Sixteen rows of a state under way per thread where it has more than eight, and not where that takes a second CTA's place on
+  // the SM (four columns a thread).  1 sequence, one head of 512 x 1024: 12.3 us with eight, 11.4 with sixteen; 32 sequences of two heads
+  // of 256 x 512: 15.9 and 16.3; 64 of three heads of 100 x 30: 5.6 and 5.3.
+  bool many = false;
+  if (r) {
+    const int quads = r->vdim / (v4 ? 4 : 1), ncol = (quads + csize - 1) / csize, groups = ncol < kDecThreads ? kDecThreads / ncol : 1;
+    many = r->dim > 8 * groups && (a || !v4 || units * b->batch <= attdec::kResident[fits - 1][0]);
+  }
+#define NQB200_DEC(VP, TILE)                                                                                                             \
+  do {                                                                                                                                    \
+    if (many) return v4 ? launch_decode<VP, 4, TILE, 16>(p, csize, st) : launch_decode<VP, 1, TILE, 16>(p, csize, st);                     \
+    return v4 ? launch_decode<VP, 4, TILE, 8>(p, csize, st) : launch_decode<VP, 1, TILE, 8>(p, csize, st);                                 \
+  } while (0)
   const bool big = a && a->dim + a->vdim > 256;
   if (!a || (a->vdim <= 64 && !big)) NQB200_DEC(64, 128);
   if (a->vdim <= 128 && !big) NQB200_DEC(128, 128);

@@ -1,10 +1,11 @@
-"""The linears of decode steps on both sides of the sizes at which their kernel changes how much a warp has under way, against
-float64."""
+"""The linears and recurrent states of decode steps on both sides of the sizes at which their kernels change how much a thread has
+under way, against float64."""
 import pytest
 import torch
 
 from nanoquantization_b200.engine.batch import StepBatch
 from nanoquantization_b200.layers import mixers as ops
+from nanoquantization_b200.layers.sequence_mixers import RetentionMixer
 
 pytestmark = pytest.mark.gpu
 DEV, bf = "cuda", torch.bfloat16
@@ -48,3 +49,32 @@ def test_linears(M, K, N):
     got = ops.dense_mingru(x, w[:3 * third], zb, xb, state, _step(M, 3))
     _close(state, s, exact)
     _close(got, s * torch.nn.functional.silu(want[:, 2 * third:3 * third]), 2.0 ** -8)
+
+
+@pytest.mark.parametrize("rot", [0, 64])
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 64, 64), (3, 100, 30), (2, 256, 512), (1, 512, 1024), (1, 1024, 8), (2, 600, 24)])
+@pytest.mark.parametrize("batch", [1, 7, 40, 160])
+@torch.no_grad()
+def test_retention_step(batch, heads, dim, vdim, rot):
+    """Values that take one thread per column or four, heads over one to eight CTAs, few rows of a state per thread and many, more
+    elements of q and k than threads."""
+    m = RetentionMixer(heads=heads, dim=dim, vdim=vdim, decay=[0.9 + 0.02 * h for h in range(heads)], eps=1e-6, out_scale=1.3, rot_base=70.0, rot_dims=rot, device=DEV)
+    cols = sum(c for _, c in m.in_parts)
+    proj = torch.randn(batch, 4 + cols, device=DEV).to(bf)
+    act = torch.full((batch, heads * vdim + 8), 7.0, device=DEV).to(bf)
+    state = torch.randn(batch, heads, dim, vdim, device=DEV)
+    position = 11
+    q, k, v, g = (t.double() for t in proj[:, 4:].split([c for _, c in m.in_parts], 1))
+    q, k, v, g = q.view(batch, heads, dim), k.view(batch, heads, dim) * dim ** -0.5, v.view(batch, heads, vdim), g.view(batch, heads, vdim)
+    a = position * m.inv_freq.double()
+    for t in (q, k):
+        lo, hi = t[..., :rot // 2].clone(), t[..., rot // 2:rot].clone()
+        t[..., :rot // 2], t[..., rot // 2:rot] = lo * a.cos() - hi * a.sin(), hi * a.cos() + lo * a.sin()
+    S = m.decay.double()[:, None, None] * state.double() + k[..., :, None] * v[..., None, :]
+    o = torch.einsum("bhd,bhdv->bhv", q, S)
+    want = 1.3 * o * torch.rsqrt(o.square().mean(-1, keepdim=True) + 1e-6) * torch.nn.functional.silu(g)
+    ops.mixer_decode(proj, act, None, (m.desc(), 4, 8, state), _step(batch, position))
+    assert (act[:, :8] == 7).all()
+    # a float product and sum (angles of 11 radians are good to 7e-7); one rounding to bfloat16
+    _close(state, S, 2e-6)
+    _close(act[:, 8:], want.flatten(1), 2.0 ** -8)
