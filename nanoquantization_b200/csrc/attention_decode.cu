@@ -18,7 +18,7 @@ int run(const void* qkv, int64_t stride, const void* q_weight, const void* k_wei
   a.scale = scale; a.out_scale = 1.f;
   a.shares = shares;
   a.cos_sin = cos_sin; a.positions = positions; a.q_weight = (const T*)q_weight; a.k_weight = (const T*)k_weight; a.eps = eps;
-  return attdec::launch<T>(a, batch, table_width * block_size, false, st);
+  return attdec::launch<true>(a, batch, table_width * block_size, false, st);
 }
 }  // namespace
 

@@ -15,8 +15,9 @@
 // A lane's maxima, sums and accumulators all belong to the same two heads.  The warps meet in shared memory, the CTAs of a
 // cluster in distributed shared memory, always in the same order.
 //
-// 48 sequences of about 1300 keys, 32 heads over 8, bfloat16 (275 MB, 43 us at the copy rate): 49 us, where the library's
-// kernel it replaces took 80.  One sequence of 2048 keys: 9.4 us, where QK-norm, that kernel and its combination took 16.
+// 48 sequences of about 1300 keys, 32 heads over 8, bfloat16 (225 MB, 35 us at the copy rate): 41 us, where flash_attn's paged
+// kernel with a launch for QK-norm and K/V store takes 71.  One sequence of 2048 keys: 9.1 us, 14.1.  The one place found where those
+// are ahead: 64 sequences of 100 keys, 64 heads over 8 (512 CTAs where 444 are resident): 16.4 us, 15.3.
 #pragma once
 #include <cooperative_groups.h>
 #include "common.cuh"
@@ -439,11 +440,14 @@ static inline bool supported(int64_t heads, int64_t kv_heads, int64_t dim, int64
   return dim == kDim && vdim == kDim && kv_heads > 0 && heads > 0 && heads % kv_heads == 0 && kv_heads <= 4096 && heads <= 65535;
 }
 
-template <typename T, int STAGES>
+// PLAIN: the caller has neither capped scores nor sigmoid weights, and their kernels are not built.
+template <typename T, int STAGES, bool PLAIN>
 static inline int launch_stages(const Args<T>& a, int csize, int64_t batch, bool sigmoid, cudaStream_t st) {
   constexpr int smem = smem_bytes(STAGES);
-  const auto kernel = sigmoid ? attention_decode_kernel<T, kSigmoid, STAGES>
-                              : a.softcap > 0.f ? attention_decode_kernel<T, kCapped, STAGES> : attention_decode_kernel<T, kSoftmax, STAGES>;
+  const auto kernel = PLAIN ? attention_decode_kernel<T, kSoftmax, STAGES>
+                      : sigmoid        ? attention_decode_kernel<T, PLAIN ? kSoftmax : kSigmoid, STAGES>
+                      : a.softcap > 0.f ? attention_decode_kernel<T, PLAIN ? kSoftmax : kCapped, STAGES>
+                                        : attention_decode_kernel<T, kSoftmax, STAGES>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return NQB200_ERR_LAUNCH; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(csize * a.parts), (unsigned)(a.kv_heads * a.head_groups), (unsigned)batch);
@@ -493,14 +497,14 @@ static inline Split split(int64_t units, int64_t keys, bool shares) {
 static inline int head_groups(int heads, int kv_heads) { return (heads / kv_heads + kHeads - 1) / kHeads; }
 static inline int64_t share_floats(int64_t batch, int heads, int parts) { return parts > 1 ? batch * heads * parts * kShare : 0; }
 
-template <typename T>
+template <bool PLAIN, typename T>
 static inline int launch(Args<T>& a, int64_t batch, int64_t keys, bool sigmoid, cudaStream_t st) {
   a.head_groups = head_groups(a.heads, a.kv_heads);
   const Split s = split((int64_t)a.kv_heads * a.head_groups * batch, keys, a.shares != nullptr);
   a.parts = s.parts;
-  const int rc = s.stages == 4   ? launch_stages<T, 4>(a, s.csize, batch, sigmoid, st)
-                 : s.stages == 3 ? launch_stages<T, 3>(a, s.csize, batch, sigmoid, st)
-                                 : launch_stages<T, 2>(a, s.csize, batch, sigmoid, st);
+  const int rc = s.stages == 4   ? launch_stages<T, 4, PLAIN>(a, s.csize, batch, sigmoid, st)
+                 : s.stages == 3 ? launch_stages<T, 3, PLAIN>(a, s.csize, batch, sigmoid, st)
+                                 : launch_stages<T, 2, PLAIN>(a, s.csize, batch, sigmoid, st);
   if (rc != NQB200_OK || s.parts == 1) return rc;
   return launch_overlapped(attention_shares_kernel<T>, dim3((unsigned)a.heads, (unsigned)batch), dim3(kThreads), 0, st, (const float*)a.shares, a.out + a.out_col,
                            a.out_stride, s.parts, a.last, a.last_shift);

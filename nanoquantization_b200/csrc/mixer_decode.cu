@@ -548,7 +548,7 @@ extern "C" int nqb200_mixer_decode(const void* proj, int64_t stride, void* act, 
     d.rot = rope->rot; d.interleaved = rope->interleaved; d.inv_freq = rope->inv_freq; d.q_norm = rope->q_norm; d.k_norm = rope->k_norm; d.eps = rope->eps;
     int64_t keys = (int64_t)b->table_width * b->block_size;
     if (a->chunk > 0 && a->chunk < keys) keys = a->chunk;
-    return attdec::launch<bf16>(d, b->batch, keys, a->sigmoid != 0, (cudaStream_t)stream);
+    return attdec::launch<false>(d, b->batch, keys, a->sigmoid != 0, (cudaStream_t)stream);
   }
   DecodeArgs p = {};
   p.proj = (const bf16*)proj; p.stride = stride; p.act = (bf16*)act; p.act_stride = act_stride; p.bt = *b;
