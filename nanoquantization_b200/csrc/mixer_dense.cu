@@ -139,7 +139,8 @@ static int launch_dense(const DenseArgs& p, cudaStream_t st) {
   // - up to eight tokens: short where three CTAs per SM are a wave less than two, of the unit only where they are the one wave.  1
   //   token, 4096 -> 6144 (384 CTAs) 12.4 long, 9.0 short; 4096 -> 8192 (512) 12.6, 14.2; 2048 -> 2048 (128) 2.2, 3.3.
   // - up to sixteen: short where the weights are long in coming; 2048 columns are one request of the long form, which pays longer.
-  //   16 tokens, 4096 -> 4096 (16.8 M) 8.7 long, 8.0 short; 4096 -> 2048 6.5, 7.0; 2048 -> 6144 (12.6 M) 7.6, 8.0.
+  //   16 tokens, 4096 -> 4096 (16.8 M) 8.7 long, 8.0 short; 4096 -> 2048 6.5, 7.0; 2048 -> 6144 (12.6 M) 7.6, 8.0;
+  //   the unit's of 4096 -> 6144 (384 CTAs) 25.3 long, 24.3 short, of 12288 -> 4096 34.8, 36.0.
   // minGRU's three matrices: long always (1 token, 4096 -> 3 x 4096 18.1 long, 21.5 short).
   constexpr bool unit = MODE == kGlu, gru = MODE == kMinGru;
   const int64_t ctas = grid.x, two = (ctas + 2 * kNumSMs - 1) / (2 * kNumSMs), three = (ctas + 3 * kNumSMs - 1) / (3 * kNumSMs);
@@ -148,7 +149,8 @@ static int launch_dense(const DenseArgs& p, cudaStream_t st) {
     if (!gru && (once || (unit ? three == 1 && two == 2 : three < two))) NQB200_DENSE(1, !gru);
     NQB200_DENSE(1, false);
   }
-  if (!gru && (once || (!unit && (int64_t)p.N * p.K >= (p.K > 2048 ? 12000000 : 16000000)))) NQB200_DENSE(2, !gru);
+  const bool long_in_coming = unit ? ctas > 2 * kNumSMs && p.K > 1024 && p.K <= 8192 : (int64_t)p.N * p.K >= (p.K > 2048 ? 12000000 : 16000000);
+  if (!gru && (once || long_in_coming)) NQB200_DENSE(2, !gru);
   NQB200_DENSE(2, false);
 #undef NQB200_DENSE
 }
