@@ -15,7 +15,7 @@
 // A lane's maxima, sums and accumulators all belong to the same two heads.  The warps meet in shared memory, the CTAs of a
 // cluster in distributed shared memory, always in the same order.
 //
-// 48 sequences of about 1300 keys, 32 heads over 8, bfloat16 (225 MB, 35 us at the copy rate): 41 us, where flash_attn's paged
+// 48 sequences of about 1140 keys, 32 heads over 8, bfloat16 (223 MB, 35 us at the copy rate): 41 us, where flash_attn's paged
 // kernel with a launch for QK-norm and K/V store takes 71.  One sequence of 2048 keys: 9.1 us, 14.1.  The one place found where those
 // are ahead: 64 sequences of 100 keys, 64 heads over 8 (512 CTAs where 444 are resident): 16.4 us, 15.3.
 #pragma once
