@@ -14,7 +14,7 @@
 // possible.  The two CTAs of a cluster (the two SMs of a TPC) work as one: M = 256 weight columns (128 from each
 // CTA's tensor memory: one A block of 64 columns per 128-k slot, four slots) by N = up to 256 tokens, of which each
 // CTA loads only its half.  Per CTA and 128-k unit: 8.5 KB of packed weights, scales and zero-points, at most
-// 32 KB of activations, and 8 MMAs of about 141 cycles.  Tensor memory is full: 256 columns of A ring and 256 of
+// 32 KB of activations, and 8 MMAs of 128 cycles at 256 tokens.  Tensor memory is full: 256 columns of A ring and 256 of
 // accumulator, so the accumulator is single and the tensor pipe idles while the epilogue reads it (about 2 us per
 // tile); the epilogue therefore only moves the tile into shared memory, 16-bit, and one TMA store writes it out.
 //
@@ -27,7 +27,9 @@
 //   warp 0        TMA producer of the activations: two boxes per unit into a ring of four stages.
 //   warp 30       TMA producer of the packed weights (64-byte swizzle), scales and zero-points: a ring of three
 //                 stages, freed as soon as the dequantisers have read them.
-//   warp 1        MMA issuer (the leader CTA's): 8 tcgen05.mma per unit, software-pipelined (see there).
+//   warp 1        MMA issuer (the leader CTA's): 8 tcgen05.mma per unit, software-pipelined (see there).  It and the producers
+//                 run as whole warps (elect_one): 777 tokens of 12288 -> 4096 79 -> 68 us, 4096 of 5120 -> 25600 868 -> 829 us
+//                 against single threads, with the same results.
 //   warps 2-17    dequantisers, two sets of 8 taking alternate units.  Warp (lane quarter q, k half h) takes the
 //                 32 columns of chunk q for k-steps 4h..4h+3: ldmatrix.x2.trans gives a thread four nibbles of
 //                 row k and of row k+1 per register (the k pairs of the operand layout); masks make 1024+q
@@ -99,16 +101,22 @@ constexpr uint32_t kSuspendNs = 20000;
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   const uint32_t b = smem_u32(bar);
   if (mbar_test_wait(b, parity)) return true;
-  const unsigned long long t0 = global_timer_ns();
-  for (;;) {
-    if (mbar_try_wait_suspend(b, parity, kSuspendNs)) return true;
+  unsigned long long t0 = 0;      // the clock is read only after a suspension that ran out
+  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
     if (*abort_flag) return false;
-    if (global_timer_ns() - t0 > kWaitLimitNs) {
+    const unsigned long long t = global_timer_ns();
+    if (!t0) t0 = t;
+    if (t - t0 > kWaitLimitNs) {
       *abort_flag = 1;
       if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
       return false;
     }
   }
+  return true;
+}
+// The same for a whole warp, whose lanes go on together (the vote keeps its control flow uniform, see elect_one).
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status));
 }
 
 template <bool BF16> __device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
@@ -164,7 +172,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   volatile int* s_abort = &s_abort_i;
   int* status = p.status;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;
   const uint32_t cluster_id = blockIdx.x / CTAS;
   const int G = p.G;
@@ -201,57 +209,62 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------- producer of the activations
-    if (lane == 0) {
-      prefetch_tmap(&tm_x);
-      const uint32_t tx_bytes = 2u * (uint32_t)p.TH * 128u;
-      int issued = 0;
-      for (int i = 0; i < nunits; ++i) {
-        const uint32_t u = u_begin + (uint32_t)i;
-        const int item = (int)(u / (uint32_t)G), gk = (int)(u % (uint32_t)G);
-        const int tok_row = (item % p.ntt) * p.NT + (int)rank * p.TH;   // this CTA's part of the token tile
-        const int s = i % kXStages;
-        if (i >= kXStages && !wait_bar(&bar_done[s], ((i / kXStages) - 1) & 1, s_abort, status)) break;
-        const uint32_t st = smem_base + s * kXStageBytes, bar = smem_u32(&bar_xfull[s]);
+    const bool el = elect_one();
+    if (el) prefetch_tmap(&tm_x);
+    __syncwarp();
+    const uint32_t tx_bytes = 2u * (uint32_t)p.TH * 128u;
+    int issued = 0;
+    for (int i = 0; i < nunits; ++i) {
+      const uint32_t u = u_begin + (uint32_t)i;
+      const int item = (int)(u / (uint32_t)G), gk = (int)(u % (uint32_t)G);
+      const int tok_row = (item % p.ntt) * p.NT + (int)rank * p.TH;   // this CTA's part of the token tile
+      const int s = i % kXStages;
+      if (i >= kXStages && !wait_bar_warp(&bar_done[s], ((i / kXStages) - 1) & 1, s_abort, status)) break;
+      const uint32_t st = smem_base + s * kXStageBytes, bar = smem_u32(&bar_xfull[s]);
+      if (el) {
         mbar_expect_tx(bar, tx_bytes);
         tma_load_2d(st, &tm_x, gk * kUnitK, tok_row, bar);
         tma_load_2d(st + p.TH * 128, &tm_x, gk * kUnitK + 64, tok_row, bar);
-        ++issued;
       }
-      // do not leave while a copy of ours may still be landing in this CTA's shared memory
-      for (int j = issued > kXStages ? issued - kXStages : 0; j < issued; ++j)
-        mbar_wait(smem_u32(&bar_xfull[j % kXStages]), (j / kXStages) & 1);
+      ++issued;
     }
+    // do not leave while a copy of ours may still be landing in this CTA's shared memory
+    for (int j = issued > kXStages ? issued - kXStages : 0; j < issued; ++j)
+      mbar_wait(smem_u32(&bar_xfull[j % kXStages]), (j / kXStages) & 1);
   } else if (warp == kWProducerWarp) {
     // ----------------------------------- producer of the packed weights, scales and zero-points
-    if (lane == 0) {
-      prefetch_tmap(&tm_w); prefetch_tmap(&tm_sc); prefetch_tmap(&tm_z);
-      int issued = 0;
-      for (int i = 0; i < nunits; ++i) {
-        const uint32_t u = u_begin + (uint32_t)i;
-        const int item = (int)(u / (uint32_t)G), gk = (int)(u % (uint32_t)G);
-        const int col_tile = (item / p.ntt) * CTAS + (int)rank;          // this CTA's 128 columns
-        const int s = i % kWStages;
-        if (i >= kWStages && !wait_bar(&bar_wfree[s], ((i / kWStages) - 1) & 1, s_abort, status)) break;
-        const uint32_t st = smem_base + kOffWRing + s * kWStageBytes, bar = smem_u32(&bar_wfull[i % kWBars]);
+    const bool el = elect_one();
+    if (el) { prefetch_tmap(&tm_w); prefetch_tmap(&tm_sc); prefetch_tmap(&tm_z); }
+    __syncwarp();
+    int issued = 0;
+    for (int i = 0; i < nunits; ++i) {
+      const uint32_t u = u_begin + (uint32_t)i;
+      const int item = (int)(u / (uint32_t)G), gk = (int)(u % (uint32_t)G);
+      const int col_tile = (item / p.ntt) * CTAS + (int)rank;          // this CTA's 128 columns
+      const int s = i % kWStages;
+      if (i >= kWStages && !wait_bar_warp(&bar_wfree[s], ((i / kWStages) - 1) & 1, s_abort, status)) break;
+      const uint32_t st = smem_base + kOffWRing + s * kWStageBytes, bar = smem_u32(&bar_wfull[i % kWBars]);
+      if (el) {
         mbar_expect_tx(bar, kWStageTx);
         tma_load_2d(st, &tm_w, col_tile * 16, gk * kUnitK, bar);
         tma_load_2d(st + kOffSc, &tm_sc, col_tile * 64, gk, bar);
         tma_load_2d(st + kOffZ, &tm_z, col_tile * 16, gk, bar);
-        ++issued;
       }
-      for (int j = issued > kWStages ? issued - kWStages : 0; j < issued; ++j)
-        mbar_wait(smem_u32(&bar_wfull[j % kWBars]), (j / kWBars) & 1);
+      ++issued;
     }
+    for (int j = issued > kWStages ? issued - kWStages : 0; j < issued; ++j)
+      mbar_wait(smem_u32(&bar_wfull[j % kWBars]), (j / kWBars) & 1);
   } else if (warp == 1) {
     // ------------------------------------------- MMA issuer (of a pair: the leader's)
-    // One thread, so every instruction here is on the critical path at several cycles each: counters instead
-    // of divisions, the descriptor as a base plus precomputed offsets, one completion report per unit.
-    if (lane == 0 && rank == 0) {
+    // Every instruction here is on the critical path: counters instead of divisions, the descriptor as a base plus
+    // precomputed offsets, one completion report per unit.
+    if (rank == 0) {
+      const bool el = elect_one();
       const uint32_t idesc = umma_idesc(BF16 ? 1 : 0, 128 * CTAS, p.NT);
       const uint64_t desc0 = umma_smem_desc_sw128(smem_base);
       const uint32_t desc_hi = (uint32_t)(desc0 >> 32), desc_lo0 = (uint32_t)desc0;
       const uint32_t x1 = ((uint32_t)p.TH * 128u) >> 4;          // second activation box, in the descriptor's 16-byte units
-      // The MMA queue is short (the tensor pipe ran dry during the 300 ns that this thread spent between two
+      // The MMA queue is short (the tensor pipe ran dry during the time that the issuer spent between two
       // units on waits, the completion report and loop bookkeeping), so the loop is software-pipelined: the
       // next unit's barrier is polled and the previous unit's completion is reported between MMAs of the
       // current unit, while MMAs are queued.  A report therefore also covers the next unit's first two
@@ -259,7 +272,7 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       uint32_t s = 0, phase = 0;
       int gk = (int)(u_begin % (uint32_t)G), li = 0, pending = -1;
       bool first = true;
-      bool ok = nunits > 0 && wait_bar(&bar_afull[0], 0, s_abort, status);   // (both CTAs') A slot filled, activations landed
+      bool ok = nunits > 0 && wait_bar_warp(&bar_afull[0], 0, s_abort, status);   // (both CTAs') A slot filled, activations landed
       const uint32_t d = tmem + kColD;
       auto mma = [&](uint32_t lo, uint32_t a, int ks, uint32_t acc) {
         const uint32_t dlo = lo + (ks >> 2) * x1 + (ks & 3) * 2;
@@ -274,31 +287,37 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         tc_fence_after();
         const uint32_t lo = desc_lo0 + s * (uint32_t)(kXStageBytes >> 4);
         const uint32_t a = tmem + kColA + s * 64;
-        mma(lo, a, 0, first ? 0u : 1u);
-        mma(lo, a, 1, 1u);
-        if (pending >= 0) { report(&bar_done[pending]); pending = -1; }
+        if (el) {
+          mma(lo, a, 0, first ? 0u : 1u);
+          mma(lo, a, 1, 1u);
+          if (pending >= 0) report(&bar_done[pending]);
 #pragma unroll
-        for (int ks = 2; ks < 6; ++ks) mma(lo, a, ks, 1u);
+          for (int ks = 2; ks < 6; ++ks) mma(lo, a, ks, 1u);
+        }
+        pending = -1;
         const uint32_t sn = s + 1 == kXStages ? 0u : s + 1, phn = s + 1 == kXStages ? phase ^ 1u : phase;
-        const bool ready = more && !last && mbar_test_wait(smem_u32(&bar_afull[sn]), phn);
-        mma(lo, a, 6, 1u);
-        mma(lo, a, 7, 1u);
+        const bool ready = __all_sync(0xffffffffu, more && !last && mbar_test_wait(smem_u32(&bar_afull[sn]), phn));
+        if (el) {
+          mma(lo, a, 6, 1u);
+          mma(lo, a, 7, 1u);
+          if (last) { report(&bar_done[s]); report(&bar_dfull); }
+        }
         if (last) {
-          report(&bar_done[s]);
-          report(&bar_dfull);
           ++li;
-          if (more) ok = wait_bar(&bar_dempty, (li - 1) & 1, s_abort, status);   // the epilogues drained D
+          if (more) ok = wait_bar_warp(&bar_dempty, (li - 1) & 1, s_abort, status);   // the epilogues drained D
         } else {
           pending = (int)s;
         }
-        if (more && !ready && ok) ok = wait_bar(&bar_afull[sn], phn, s_abort, status);
+        if (more && !ready && ok) ok = wait_bar_warp(&bar_afull[sn], phn, s_abort, status);
         first = last;
         if (++gk == G) gk = 0;
         s = sn; phase = phn;
       }
-      if (pending >= 0) report(&bar_done[pending]);
-      // everything issued has completed before tensor memory may be released
-      if (CTAS == 2) umma_commit_pair(map_to_cta(smem_u32(&bar_drain), 0)); else umma_commit(smem_u32(&bar_drain));
+      if (el) {
+        if (pending >= 0) report(&bar_done[pending]);
+        // everything issued has completed before tensor memory may be released
+        if (CTAS == 2) umma_commit_pair(map_to_cta(smem_u32(&bar_drain), 0)); else umma_commit(smem_u32(&bar_drain));
+      }
       mbar_wait(smem_u32(&bar_drain), 0);
     }
   } else if (warp < 2 + kDequantWarps) {
