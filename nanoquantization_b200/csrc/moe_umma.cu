@@ -10,7 +10,9 @@
 //
 //   warp 0        TMA: the weight tile, and for the second linear the pairs' rows, which are contiguous.  A ring of five
 //                 stages of 64 k.
-//   warp 1        the leader's: one thread issues the MMAs; the other CTA's: reports its landed stages to the leader.
+//   warp 1        the leader's: issues the MMAs; the other CTA's: reports its landed stages to the leader.  Warps 0 and 1 run
+//                 whole (elect_one): 5000 tokens, 64 experts of 4096 x 1536, 8 per token 522 -> 501 and 497 -> 447 us (first and
+//                 second linear) against single threads.  Six stages, or gathers three stages ahead: no change.
 //   warps 2-9     epilogue: accumulator (two of them take turns) -> gelu or the pair's weight -> 16 bits in shared memory,
 //                 [pair][feature] -> rows of 256 bytes to their places in the output.
 //   warps 10-13   first linear: the pairs' rows, gathered by token with cp.async into the swizzled layout, two stages ahead
@@ -44,16 +46,22 @@ constexpr uint32_t kSuspendNs = 20000;
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   const uint32_t b = smem_u32(bar);
   if (mbar_test_wait(b, parity)) return true;
-  const unsigned long long t0 = global_timer_ns();
-  for (;;) {
-    if (mbar_try_wait_suspend(b, parity, kSuspendNs)) return true;
+  unsigned long long t0 = 0;      // the clock is read only after a suspension that ran out
+  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
     if (*abort_flag) return false;
-    if (global_timer_ns() - t0 > kWaitLimitNs) {
+    const unsigned long long t = global_timer_ns();
+    if (!t0) t0 = t;
+    if (t - t0 > kWaitLimitNs) {
       *abort_flag = 1;
       if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
       return false;
     }
   }
+  return true;
+}
+// The same for a whole warp, whose lanes go on together (the vote keeps its control flow uniform, see elect_one).
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xFFFFFFFFu, wait_bar(bar, parity, abort_flag, status));
 }
 // One arrival on the barrier at this offset in both CTAs when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void commit_both(uint32_t bar) {
@@ -109,7 +117,7 @@ __global__ void __launch_bounds__((2 + kEpiWarps + (UP ? kLoadWarps : 0)) * 32, 
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cluster = blockIdx.x >> 1;
+  const int warp = warp_index(), lane = threadIdx.x & 31, cluster = blockIdx.x >> 1;
   const uint32_t rank = cluster_ctarank();
 
   grid_launch_dependents();
@@ -151,26 +159,32 @@ __global__ void __launch_bounds__((2 + kEpiWarps + (UP ? kLoadWarps : 0)) * 32, 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA
     if (lane == 0) { prefetch_tmap(&tm_w); prefetch_tmap(&tm_x); prefetch_tmap(&tm_x128); }
-    int n = 0;            // stages filled so far
+    __syncwarp();
+    const bool el = elect_one();
+    int n = 0, s = 0;     // stages filled so far, and the next one
+    uint32_t phase = 1;   // parity of the phase in which that stage was last given back
     bool ok = true;
     for (int item = cluster; ok && item < items; item += p.clusters) {
       const Item it = locate(p, tiles, item);
       const int th = it.nt / 2, w_row = it.expert * p.N + it.feature + (int)rank * 128, first = (int)rank * th;
       // one box of 128 rows where that is not far too many (what lies behind the tile is not used): boxes cost by the piece
-      const bool one = th > 48;
+      const bool one = __any_sync(0xFFFFFFFFu, th > 48);
       const uint32_t bytes = (uint32_t)kABytes + (UP ? 0u : one ? 128u * 128u : (uint32_t)th * 128u);
       for (int k = 0; k < p.steps; ++k, ++n) {
-        const int s = n % kStages;
         const uint32_t st = smem + s * kStageBytes, bar = smem_u32(&bar_full[s]);
-        if (lane == 0) {
-          if (n >= kStages) ok = wait_bar(&bar_free[s], ((n / kStages) - 1) & 1, s_abort, p.status);
-          if (ok) mbar_expect_tx(bar, bytes);
-        }
-        ok = __shfl_sync(0xFFFFFFFFu, (int)ok, 0) != 0;
+        if (n >= kStages) ok = wait_bar_warp(&bar_free[s], phase, s_abort, p.status);
         if (!ok) break;
-        if (lane == 0) tma_load_2d(st, &tm_w, k * kStepK, w_row, bar);
-        if (!UP && one && lane == 0) tma_load_2d(st + kABytes, &tm_x128, k * kStepK, it.lo + first, bar);
-        if (!UP && !one && 16 * lane < th) tma_load_2d(st + kABytes + lane * 2048, &tm_x, k * kStepK, it.lo + first + 16 * lane, bar);
+        if (el) {
+          mbar_expect_tx(bar, bytes);
+          tma_load_2d(st, &tm_w, k * kStepK, w_row, bar);
+          if (!UP && one) tma_load_2d(st + kABytes, &tm_x128, k * kStepK, it.lo + first, bar);
+        }
+        if (!UP && !one) {
+          __syncwarp();
+          if (16 * lane < th) tma_load_2d(st + kABytes + lane * 2048, &tm_x, k * kStepK, it.lo + first + 16 * lane, bar);
+          __syncwarp();
+        }
+        if (++s == kStages) { s = 0; phase ^= 1u; }
       }
     }
     // do not leave while a copy may still be landing
@@ -178,41 +192,41 @@ __global__ void __launch_bounds__((2 + kEpiWarps + (UP ? kLoadWarps : 0)) * 32, 
     if (lane == 0)
       for (int j = n > kStages ? n - kStages : 0; j < n; ++j) mbar_wait(smem_u32(&bar_full[j % kStages]), (j / kStages) & 1);
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    const bool el = elect_one();
+    int s = 0, li = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    if (rank == 0) {
       // ---------------------------------------------------------------- MMA
       const uint64_t desc = umma_smem_desc_sw128(smem);
       const uint32_t hi = (uint32_t)(desc >> 32), lo0 = (uint32_t)desc;
-      int s = 0, li = 0;
-      uint32_t phase = 0;
-      bool ok = true;
       for (int item = cluster; ok && item < items; item += p.clusters, ++li) {
         const Item it = locate(p, tiles, item);
         const uint32_t idesc = umma_idesc(1, 256, it.nt), d = tmem + (li & 1) * 256;
-        if (li >= 2 && !wait_bar(&bar_dempty[li & 1], ((li >> 1) - 1) & 1, s_abort, p.status)) { ok = false; break; }
+        if (li >= 2 && !wait_bar_warp(&bar_dempty[li & 1], ((li >> 1) - 1) & 1, s_abort, p.status)) { ok = false; break; }
         for (int k = 0; k < p.steps; ++k) {
-          if (!wait_bar(&bar_full[s], phase, s_abort, p.status)) { ok = false; break; }
+          if (!wait_bar_warp(&bar_full[s], phase, s_abort, p.status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a = lo0 + s * (kStageBytes >> 4), b = a + (kABytes >> 4);
+          if (el) {
 #pragma unroll
-          for (int ks = 0; ks < kStepK / 16; ++ks) umma_ss_pair(d, a + ks * 2, b + ks * 2, hi, idesc, (k | ks) != 0 ? 1u : 0u);
-          commit_both(smem_u32(&bar_free[s]));
+            for (int ks = 0; ks < kStepK / 16; ++ks) umma_ss_pair(d, a + ks * 2, b + ks * 2, hi, idesc, (k | ks) != 0 ? 1u : 0u);
+            commit_both(smem_u32(&bar_free[s]));
+          }
           if (++s == kStages) { s = 0; phase ^= 1u; }
         }
-        if (ok) commit_both(smem_u32(&bar_dfull[li & 1]));
+        if (ok && el) commit_both(smem_u32(&bar_dfull[li & 1]));
       }
       // everything issued has completed before tensor memory may be released
-      umma_commit_pair(map_to_cta(smem_u32(&bar_drain), 0));
+      if (el) umma_commit_pair(map_to_cta(smem_u32(&bar_drain), 0));
       mbar_wait(smem_u32(&bar_drain), 0);
-    } else if (lane == 0) {
+    } else {
       // -------------------------------------------- the other CTA's stages
-      int s = 0;
-      uint32_t phase = 0;
-      bool ok = true;
       const uint32_t leader = map_to_cta(smem_u32(&bar_full[0]), 0);
       for (int item = cluster; ok && item < items; item += p.clusters)
         for (int k = 0; k < p.steps; ++k) {
-          if (!wait_bar(&bar_full[s], phase, s_abort, p.status)) { ok = false; break; }
-          mbar_arrive_cluster(leader + (uint32_t)s * 8u);
+          if (!wait_bar_warp(&bar_full[s], phase, s_abort, p.status)) { ok = false; break; }
+          if (el) mbar_arrive_cluster(leader + (uint32_t)s * 8u);
           if (++s == kStages) { s = 0; phase ^= 1u; }
         }
     }
