@@ -44,17 +44,24 @@ constexpr uint32_t kSuspendNs = 20000;
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   const uint32_t b = smem_u32(bar);
   if (mbar_test_wait(b, parity)) return true;
-  const unsigned long long t0 = global_timer_ns();
-  for (;;) {
-    if (mbar_try_wait_suspend(b, parity, kSuspendNs)) return true;
+  unsigned long long t0 = 0;      // the clock is read only after a suspension that ran out
+  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
     if (*abort_flag) return false;
-    if (global_timer_ns() - t0 > kWaitLimitNs) {
+    const unsigned long long t = global_timer_ns();
+    if (!t0) t0 = t;
+    if (t - t0 > kWaitLimitNs) {
       *abort_flag = 1;
       if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
       return false;
     }
   }
+  return true;
 }
+// The same, and a test, for a whole warp whose lanes go on together (the votes keep its control flow uniform, see elect_one).
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xFFFFFFFFu, wait_bar(bar, parity, abort_flag, status));
+}
+__device__ __forceinline__ bool test_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xFFFFFFFFu, mbar_test_wait(smem_u32(bar), parity)); }
 
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor]; the descriptors' high halves are the same.
 __device__ __forceinline__ void umma_ss_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
@@ -119,7 +126,7 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   grid_launch_dependents();
   grid_dependency_wait();
@@ -131,7 +138,7 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   int nq[2];
 #pragma unroll
   for (int q = 0; q < 2; ++q)
-    nq[q] = i0 + q * kTile < n ? (pos0 + min(i0 + (q + 1) * kTile, n) - 1 - kstart) / kTile + 1 : 0;
+    nq[q] = __shfl_sync(0xFFFFFFFFu, i0 + q * kTile < n ? (pos0 + min(i0 + (q + 1) * kTile, n) - 1 - kstart) / kTile + 1 : 0, 0);
   const int nmax = max(nq[0], nq[1]);
 
   if (threadIdx.x == 0) {
@@ -154,113 +161,125 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA
-    if (lane == 0) {
+    const bool el = elect_one();
+    const int tiles_q = nq[1] > 0 ? 2 : 1;
+    if (el) {
       prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
-      const int tiles_q = nq[1] > 0 ? 2 : 1;
       mbar_expect_tx(smem_u32(&bar_q), (uint32_t)tiles_q * kQBytes);
       for (int q = 0; q < tiles_q; ++q)
         for (int c = 0; c < D / 64; ++c) tma_load_2d(smem + q * kQBytes + c * kBox, &tm_q, h * D + c * 64, t0 + i0 + q * kTile, smem_u32(&bar_q));
-      int issued = 0;
-      for (int j = 0; j < nmax; ++j, ++issued) {
-        const int s = j & 1, pos = kstart + j * kTile;
-        if (j >= 2 && !wait_bar(&bar_kfree[s], ((j >> 1) - 1) & 1, s_abort, p.status)) break;
-        const int row = (int)kv_row(p.bt, b, pos);    // the tile lies in one page
+    }
+    __syncwarp();
+    int issued = 0;
+    for (int j = 0; j < nmax; ++j, ++issued) {
+      const int s = j & 1, pos = kstart + j * kTile;
+      if (j >= 2 && !wait_bar_warp(&bar_kfree[s], ((j >> 1) - 1) & 1, s_abort, p.status)) break;
+      const int row = __shfl_sync(0xFFFFFFFFu, (int)kv_row(p.bt, b, pos), 0);    // the tile lies in one page
+      if (el) {
         mbar_expect_tx(smem_u32(&bar_kfull[s]), kKBytes);
+#pragma unroll
         for (int c = 0; c < D / 64; ++c) tma_load_2d(smem + kOffK + s * kKBytes + c * kBox, &tm_k, kvh * D + c * 64, row, smem_u32(&bar_kfull[s]));
-        if (j >= 2 && !wait_bar(&bar_vfree[s], ((j >> 1) - 1) & 1, s_abort, p.status)) {
-          mbar_wait(smem_u32(&bar_kfull[s]), (j >> 1) & 1);
-          break;
-        }
+      }
+      if (j >= 2 && !wait_bar_warp(&bar_vfree[s], ((j >> 1) - 1) & 1, s_abort, p.status)) {
+        mbar_wait(smem_u32(&bar_kfull[s]), (j >> 1) & 1);
+        break;
+      }
+      if (el) {
         mbar_expect_tx(smem_u32(&bar_vfull[s]), kVBytes);
+#pragma unroll
         for (int c = 0; c < V / 64; ++c) tma_load_2d(smem + kOffV + s * kVBytes + c * kBox, &tm_v, kvh * V + c * 64, row, smem_u32(&bar_vfull[s]));
       }
-      // do not leave while a copy may still be landing
-      mbar_wait(smem_u32(&bar_q), 0);
-      for (int j = issued > 2 ? issued - 2 : 0; j < issued; ++j) {
-        mbar_wait(smem_u32(&bar_kfull[j & 1]), (j >> 1) & 1);
-        mbar_wait(smem_u32(&bar_vfull[j & 1]), (j >> 1) & 1);
-      }
+    }
+    // do not leave while a copy may still be landing
+    mbar_wait(smem_u32(&bar_q), 0);
+    for (int j = issued > 2 ? issued - 2 : 0; j < issued; ++j) {
+      mbar_wait(smem_u32(&bar_kfull[j & 1]), (j >> 1) & 1);
+      mbar_wait(smem_u32(&bar_vfull[j & 1]), (j >> 1) & 1);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA
-    // One thread runs both tiles as two little state machines and never blocks on one of them: it polls for the first
-    // and the second half of a tile's weights (then issues that half of O += P V) and for that product's end (P has been
-    // read: then S of the next key tile may overwrite it).  A ring stage is handed back by whichever tile uses it second.
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc(1, 128, kTile);
-      const uint32_t idesc_o = umma_idesc(1, 128, V) | (1u << 16);   // B's rows run along k
-      const uint64_t dq = umma_smem_desc_sw128(smem), dk = umma_smem_desc_sw128(smem + kOffK), dv = smem_desc_mn(smem + kOffV, kBox);
-      const uint32_t k_hi = (uint32_t)(dq >> 32), v_hi = (uint32_t)(dv >> 32), q_lo = (uint32_t)dq, k_lo = (uint32_t)dk, v_lo = (uint32_t)dv;
-      auto scores = [&](int q, int s) {
-        const uint32_t a = q_lo + q * (kQBytes >> 4), bk = k_lo + s * (kKBytes >> 4), d = tmem + kColS + q * 128;
+    // One warp, of which one lane issues (elect_one: 8192 tokens of 32 heads, chunks of 4096, 647 -> 575 us against a single
+    // thread), runs both tiles as two little state machines and never blocks on one of them: it polls for the first and the
+    // second half of a tile's weights (then issues that half of O += P V) and for that product's end (P has been read: then S
+    // of the next key tile may overwrite it).  A ring stage is handed back by whichever tile uses it second.
+    const bool el = elect_one();
+    const uint32_t idesc_s = umma_idesc(1, 128, kTile);
+    const uint32_t idesc_o = umma_idesc(1, 128, V) | (1u << 16);   // B's rows run along k
+    const uint64_t dq = umma_smem_desc_sw128(smem), dk = umma_smem_desc_sw128(smem + kOffK), dv = smem_desc_mn(smem + kOffV, kBox);
+    const uint32_t k_hi = (uint32_t)(dq >> 32), v_hi = (uint32_t)(dv >> 32), q_lo = (uint32_t)dq, k_lo = (uint32_t)dk, v_lo = (uint32_t)dv;
+    auto scores = [&](int q, int s) {
+      const uint32_t a = q_lo + q * (kQBytes >> 4), bk = k_lo + s * (kKBytes >> 4), d = tmem + kColS + q * 128;
+      if (el) {
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
           umma_ss_lohi(d, a + (ks >> 2) * (kBox >> 4) + (ks & 3) * 2, bk + (ks >> 2) * (kBox >> 4) + (ks & 3) * 2, k_hi, idesc_s, ks > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_s[q]));
-      };
-      bool ok = wait_bar(&bar_q, 0, s_abort, p.status) && wait_bar(&bar_kfull[0], 0, s_abort, p.status);
-      const int users = nq[1] > 0 ? 2 : 1;
-      // tile of the next product; 0, 1: waits for that half of the weights, 2: for the product; users that have still to
-      // issue on K / V tile j (by j & 1)
-      int jq[2] = {0, 0};
-      int phase[2] = {0, 0};
-      auto users_of = [&](int j) { return users == 2 ? (j < nq[0]) + (j < nq[1]) : 1; };
-      int kleft[2] = {0, users_of(1)}, vleft[2] = {users_of(0), users_of(1)};
-      if (ok) {
-        tc_fence_after();
-        for (int q = 0; q < users; ++q) scores(q, 0);
-        umma_commit(smem_u32(&bar_kfree[0]));
-        kleft[0] = users_of(2);
       }
-      unsigned long long t_last = global_timer_ns();
-      uint32_t polls = 0;
-      while (ok && (jq[0] < nq[0] || jq[1] < nq[1])) {
-        bool moved = false;
+    };
+    bool ok = wait_bar_warp(&bar_q, 0, s_abort, p.status) && wait_bar_warp(&bar_kfull[0], 0, s_abort, p.status);
+    const int users = nq[1] > 0 ? 2 : 1;
+    // tile of the next product; 0, 1: waits for that half of the weights, 2: for the product; users that have still to
+    // issue on K / V tile j (by j & 1)
+    int jq[2] = {0, 0};
+    int phase[2] = {0, 0};
+    auto users_of = [&](int j) { return users == 2 ? (j < nq[0]) + (j < nq[1]) : 1; };
+    int kleft[2] = {0, users_of(1)}, vleft[2] = {users_of(0), users_of(1)};
+    if (ok) {
+      tc_fence_after();
+      for (int q = 0; q < users; ++q) scores(q, 0);
+      if (el) umma_commit(smem_u32(&bar_kfree[0]));
+      kleft[0] = users_of(2);
+    }
+    unsigned long long t_last = global_timer_ns();
+    uint32_t polls = 0;
+    while (ok && (jq[0] < nq[0] || jq[1] < nq[1])) {
+      bool moved = false;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int j = jq[q], s = j & 1, sn = s ^ 1;
-          if (j >= nq[q]) continue;
-          if (phase[q] < 2) {
-            const int half = phase[q];
-            if (!mbar_test_wait(smem_u32(&bar_p[q][half]), s) || !mbar_test_wait(smem_u32(&bar_vfull[s]), (j >> 1) & 1)) continue;
-            tc_fence_after();
-            const uint32_t d = tmem + kColO + q * 128, pa = tmem + kColS + q * 128 + half * 32, bv = v_lo + s * (kVBytes >> 4) + half * (8192 >> 4);
+      for (int q = 0; q < 2; ++q) {
+        const int j = jq[q], s = j & 1, sn = s ^ 1;
+        if (j >= nq[q]) continue;
+        if (phase[q] < 2) {
+          const int half = phase[q];
+          if (!test_warp(&bar_p[q][half], s) || !test_warp(&bar_vfull[s], (j >> 1) & 1)) continue;
+          tc_fence_after();
+          const uint32_t d = tmem + kColO + q * 128, pa = tmem + kColS + q * 128 + half * 32, bv = v_lo + s * (kVBytes >> 4) + half * (8192 >> 4);
+          if (el) {
 #pragma unroll
             for (int ks = 0; ks < kTile / 32; ++ks)
               umma_ts_lohi(d, pa + ks * 8, bv + ks * (2048 >> 4), v_hi, idesc_o, (j > 0 || half > 0 || ks > 0) ? 1u : 0u);
-            phase[q] = half + 1;
-            if (half == 1) {
-              umma_commit(smem_u32(&bar_pv[q]));
-              if (--vleft[s] == 0) { umma_commit(smem_u32(&bar_vfree[s])); vleft[s] = users_of(j + 2); }
-              if (j == nq[q] - 1) { umma_commit(smem_u32(&bar_o[q])); jq[q] = j + 1; }
-            }
-          } else {
-            if (!mbar_test_wait(smem_u32(&bar_pv[q]), s) || !mbar_test_wait(smem_u32(&bar_kfull[sn]), ((j + 1) >> 1) & 1)) continue;
-            tc_fence_after();
-            scores(q, sn);
-            if (--kleft[sn] == 0) { umma_commit(smem_u32(&bar_kfree[sn])); kleft[sn] = users_of(j + 3); }
-            jq[q] = j + 1;
-            phase[q] = 0;
           }
-          moved = true;
+          phase[q] = half + 1;
+          if (half == 1) {
+            if (el) umma_commit(smem_u32(&bar_pv[q]));
+            if (--vleft[s] == 0) { if (el) umma_commit(smem_u32(&bar_vfree[s])); vleft[s] = users_of(j + 2); }
+            if (j == nq[q] - 1) { if (el) umma_commit(smem_u32(&bar_o[q])); jq[q] = j + 1; }
+          }
+        } else {
+          if (!test_warp(&bar_pv[q], s) || !test_warp(&bar_kfull[sn], ((j + 1) >> 1) & 1)) continue;
+          tc_fence_after();
+          scores(q, sn);
+          if (--kleft[sn] == 0) { if (el) umma_commit(smem_u32(&bar_kfree[sn])); kleft[sn] = users_of(j + 3); }
+          jq[q] = j + 1;
+          phase[q] = 0;
         }
-        if (moved) {
-          polls = 0;
-        } else if ((++polls & 63u) == 0) {
-          const unsigned long long now = global_timer_ns();
-          if (polls == 64) t_last = now;
-          if (*s_abort) ok = false;
-          else if (now - t_last > kWaitLimitNs) {
-            *s_abort = 1;
-            if (p.status) atomicExch(p.status, NQB200_ERR_WAIT_TIMEOUT);
-            ok = false;
-          }
+        moved = true;
+      }
+      if (moved) {
+        polls = 0;
+      } else if ((++polls & 63u) == 0) {
+        const unsigned long long now = global_timer_ns();
+        if (polls == 64) t_last = now;
+        if (__any_sync(0xFFFFFFFFu, *s_abort != 0)) ok = false;
+        else if (__any_sync(0xFFFFFFFFu, now - t_last > kWaitLimitNs)) {
+          *s_abort = 1;
+          if (p.status) atomicExch(p.status, NQB200_ERR_WAIT_TIMEOUT);
+          ok = false;
         }
       }
-      // everything issued has completed before tensor memory may be released
-      umma_commit(smem_u32(&bar_drain));
-      mbar_wait(smem_u32(&bar_drain), 0);
     }
+    // everything issued has completed before tensor memory may be released
+    if (el) umma_commit(smem_u32(&bar_drain));
+    mbar_wait(smem_u32(&bar_drain), 0);
   } else if (warp >= 4) {
     // -------------------------------------------------------------- softmax
     const int q = (warp - 4) >> 2, quarter = warp & 3;
