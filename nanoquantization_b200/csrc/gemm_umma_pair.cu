@@ -137,6 +137,14 @@ __device__ __forceinline__ uint32_t fma2_f16(uint32_t a, uint32_t b, uint32_t c)
   return r;
 }
 
+// (a & mask) | bits as one instruction: with mask and bits in registers.  (The instruction has room for one immediate, and
+// with both as constants the compiler makes two of it.)
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
+  return r;
+}
+
 // cluster c's units: [range_begin(c), range_begin(c + 1)), boundaries on multiples of q units (q = 1: stream-K;
 // q = a tile's units: whole tiles only); 32-bit arithmetic (the host checks U * C < 2^31)
 __host__ __device__ __forceinline__ uint32_t range_begin(uint32_t c, uint32_t U, uint32_t C, uint32_t q) {
@@ -331,6 +339,10 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // rows are 64 bytes, 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3)
     const int lr = lane & 15;
     const uint32_t ld_row = (uint32_t)lr * 64u, ld_x = (uint32_t)((lr >> 1) & 3);
+    uint32_t lo_mask, hi_mask, magic;
+    asm volatile("mov.u32 %0, %1;" : "=r"(lo_mask) : "n"(LO));
+    asm volatile("mov.u32 %0, %1;" : "=r"(hi_mask) : "n"(HI));
+    asm volatile("mov.u32 %0, %1;" : "=r"(magic) : "n"(MAGIC));
     for (int i = set; i < nunits; i += 2) {
       const int sw = i % kWStages, sa = i % kXStages;
       if (!wait_bar(&bar_wfull[i % kWBars], (i / kWBars) & 1, s_abort, status)) break;
@@ -370,15 +382,15 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         for (int ph = 0; ph < 2; ++ph) {
           uint32_t a0, a1, a2, a3;
           if (BF16) {
-            a0 = ((R0 >> (8 * ph)) & LO) | MAGIC; a1 = ((R0 >> (8 * ph + 4)) & LO) | MAGIC;
-            a2 = ((R1 >> (8 * ph)) & LO) | MAGIC; a3 = ((R1 >> (8 * ph + 4)) & LO) | MAGIC;
+            a0 = and_or(R0 >> (8 * ph), lo_mask, magic); a1 = and_or(R0 >> (8 * ph + 4), lo_mask, magic);
+            a2 = and_or(R1 >> (8 * ph), lo_mask, magic); a3 = and_or(R1 >> (8 * ph + 4), lo_mask, magic);
             a0 = mul2<true>(sub2<true>(a0, zm2[2 * ph]), sc2[2 * ph]);
             a2 = mul2<true>(sub2<true>(a2, zm2[2 * ph]), sc2[2 * ph]);
             a1 = mul2<true>(sub2<true>(a1, zm2[2 * ph + 1]), sc2[2 * ph + 1]);
             a3 = mul2<true>(sub2<true>(a3, zm2[2 * ph + 1]), sc2[2 * ph + 1]);
           } else {
             const uint32_t l = R0 >> (8 * ph), hh = R1 >> (8 * ph);
-            a0 = (l & LO) | MAGIC; a1 = (l & HI) | MAGIC; a2 = (hh & LO) | MAGIC; a3 = (hh & HI) | MAGIC;
+            a0 = and_or(l, lo_mask, magic); a1 = and_or(l, hi_mask, magic); a2 = and_or(hh, lo_mask, magic); a3 = and_or(hh, hi_mask, magic);
             a0 = mul2<false>(sub2<false>(a0, zm2[2 * ph]), sc2[2 * ph]);
             a2 = mul2<false>(sub2<false>(a2, zm2[2 * ph]), sc2[2 * ph]);
             a1 = mul2<false>(fma2_f16(a1, SIXTEENTH, zm2[2 * ph + 1]), sc2[2 * ph + 1]);
