@@ -20,10 +20,11 @@ from collections import deque
 from dataclasses import dataclass, field
 from typing import Optional, Sequence as Seq
 
+import numpy as np
 import torch
 import torch.nn.functional as F
 
-from .batch import CacheLayout, StepBatch
+from .batch import CacheLayout, StepBatch, to_device
 
 
 @dataclass
@@ -308,9 +309,9 @@ class LLMEngine:
         s.computed = computed
         self.blocks.reclaim(s, self.layout.visible_from(computed))
 
-    def _run_portions(self, batch: list[Sequence], counts: list[int], rows: Optional[list[int]] = None) -> torch.Tensor:
+    def _run_portions(self, batch: list[Sequence], counts: list[int], rows: Optional[np.ndarray] = None) -> torch.Tensor:
         """The next ``counts[i]`` tokens of each sequence, from what earlier steps left; the final hidden states of
-        the given rows of the step (default: each sequence's last)."""
+        the given rows of the step (default: each sequence's last; all of them in order need no gathering)."""
         tokens = [(s.prompt + s.output)[s.computed:s.computed + n] for s, n in zip(batch, counts)]
         for s in batch:
             self.states.ensure(s)
@@ -318,8 +319,10 @@ class LLMEngine:
         host = StepBatch.host(tokens, [s.computed for s in batch], [s.blocks for s in batch],
                               [self.scratch_slot if s.slot is None else s.slot for s in batch], width, self.block_size)
         if rows is None:
-            rows = [e - 1 for e in host.cu.tolist()[1:]]
-        h = self._forward(host.to(self.device), False, torch.tensor(rows, dtype=torch.long, device=self.device))
+            rows = host.cu.numpy()[1:] - 1
+        rows = rows.astype(np.int64)
+        everything = np.array_equal(rows, np.arange(host.num_tokens))
+        h = self._forward(host.to(self.device), False, None if everything else to_device(torch.from_numpy(rows), self.device))
         for s, n in zip(batch, counts):
             self._advance(s, s.computed + n)
         return h
@@ -407,11 +410,11 @@ class LLMEngine:
         if all(n == 1 and s.computed > 0 for s, n in zip(batch, counts)):
             h = self._decode_hidden(batch)[0]
             return [self.model.logits(h[i:i + 1]) if len(want) else None for i, (_, _, want) in enumerate(entries)]
-        rows, o = [], 0
+        rows, o = [np.empty(0, np.int64)], 0
         for (_, _, want), n in zip(entries, counts):
-            rows += [o + w for w in want]
+            rows.append(o + (np.arange(want.start, want.stop, want.step) if isinstance(want, range) else np.array([int(w) for w in want], np.int64)))
             o += n
-        h = self._run_portions(batch, counts, rows)
+        h = self._run_portions(batch, counts, np.concatenate(rows))
         out, o = [], 0
         for _, _, want in entries:
             out.append(self.model.logits(h[o:o + len(want)]) if len(want) else None)
