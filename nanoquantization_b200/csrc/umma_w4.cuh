@@ -1,0 +1,65 @@
+// What the tcgen05 kernels of the packed linears share: bounded waits, the arithmetic that turns packed words into 16-bit
+// weights, and the dealing of units to CTAs.
+#pragma once
+#include "common.cuh"
+#include "tma_utils.cuh"
+#include "umma_utils.cuh"
+
+namespace nqb200 {
+
+// A wait suspends in hardware for up to kSuspendNs at a time (woken at once when the phase completes), so that warps which
+// wait most of the time hardly issue; the clock is read only after a suspension that ran out.
+constexpr uint32_t kSuspendNs = 20000;
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  const uint32_t b = smem_u32(bar);
+  if (mbar_test_wait(b, parity)) return true;
+  unsigned long long t0 = 0;
+  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
+    if (*abort_flag) return false;
+    const unsigned long long t = global_timer_ns();
+    if (!t0) t0 = t;
+    if (t - t0 > kWaitLimitNs) {
+      *abort_flag = 1;
+      if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
+      return false;
+    }
+  }
+  return true;
+}
+// The same for a whole warp, whose lanes go on together (the vote keeps its control flow uniform, see elect_one).
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status));
+}
+
+template <bool BF16> __device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (BF16) asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <bool BF16> __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (BF16) asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t fma2_f16(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
+// (a & mask) | bits as one instruction: with mask and bits in registers.  (The instruction has room for one immediate, and
+// with both as constants the compiler makes two of it.)
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
+  return r;
+}
+
+// The column of an A block's 128 that lane `l` of tensor memory holds (the order the dequantisers' stores give).
+__device__ __forceinline__ int column_of_lane(int l) {
+  const int q = l >> 5, ph = (l >> 4) & 1, r = (l >> 3) & 1, g = l & 7;
+  return 32 * q + 8 * (g >> 1) + 4 * ph + 2 * r + (g & 1);
+}
+
+}  // namespace nqb200
