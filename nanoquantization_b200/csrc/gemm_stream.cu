@@ -17,12 +17,12 @@
 //                   stage (swizzled like a TMA tile), and their sum per token
 //                   (the tensor pipe is this kernel's scarce resource, so the sum
 //                   is not done with an all-ones mma).
-//   8 consumer warps : warp w owns columns 64w..64w+63 of the tile for the whole
-//                   group; arithmetic as in the register-fed kernel (raw nibbles
-//                   as fp16 subnormals into mma.sync m16n8k16, scale and
-//                   zero-point applied once per group in fp32).  The 128-byte swizzle and
-//                   the mma's own k order (2t, 2t+1, 2t+8, 2t+9) make every
-//                   shared-memory load conflict-free.
+//   8 or 16 consumer warps : a warp owns one or two chunks of 32 columns of the tile for the
+//                   whole group; arithmetic as in the register-fed kernel (raw nibbles as fp16
+//                   subnormals into mma.sync m16n8k16, scale and zero-point applied once per
+//                   group in fp32).  ldmatrix with transposition brings the pairs of rows that
+//                   the mma's A operand wants, so that a mask (and a shift) per register is all
+//                   that is left to do; the 128-byte swizzle keeps it free of conflicts.
 //
 // A CTA whose range covers a tile's whole K writes the output itself.  Other
 // segments go to a per-CTA slot (fp32) in the workspace, and a second, small
@@ -33,22 +33,24 @@
 //
 // Every wait is bounded; on expiry the kernel records NQB200_ERR_WAIT_TIMEOUT in
 // the workspace status word and drains instead of spinning.
-#include "common.cuh"
-#include "tma_utils.cuh"
+#include "umma_w4.cuh"
 #include "peer_layout.cuh"
 #include <mutex>
 
 namespace nqb200 {
 
 constexpr int kUnitN = 512, kUnitK = 128;
-constexpr int kConsumerWarps = 8;
-constexpr int kStreamThreads = (kConsumerWarps + 2) * 32;  // consumers, TMA producer, sum(x) warp
 constexpr int kOffW0 = 0, kOffW1 = 16384, kOffX0 = 32768;
 
-// Up to 8 tokens (MT = 1): two CTAs per SM with three stages each, so that 16 consumer warps
-// share an SM's issue slots.  Up to 16 tokens (MT = 2): one CTA per SM with five stages.
+// Sixteen consumer warps share an SM's issue slots.  Up to 8 tokens (MT = 1): in two CTAs with three stages each, a warp
+// taking two chunks of 32 columns.  Up to 16 tokens (MT = 2): in one CTA with five stages, a warp taking one chunk
+// (before, eight warps of two chunks, rows paired by byte permutations and, in bf16, masks as immediates:
+// 5120 x 25600 in bf16 30.2 -> 24.3 us at 16 tokens and 23.0 -> 18.1 at 8, in fp16 25.6 -> 23.3 and 17.7 -> 16.0).  More
+// activation warps, or their loads a unit ahead: no change.
 template <int MT> struct StreamCfg {
   static constexpr int kCtasPerSm = MT == 1 ? 2 : 1;
+  static constexpr int kChunks = MT == 1 ? 2 : 1, kConsumerWarps = kUnitN / 32 / kChunks;
+  static constexpr int kThreads = (kConsumerWarps + 2) * 32;   // consumers, TMA producer, activation warp
   static constexpr int kStages = MT == 1 ? 3 : 5;
   static constexpr int kXBox = 8 * MT * 128;                 // bytes of one activation box
   static constexpr int kOffX1 = kOffX0 + kXBox;
@@ -108,11 +110,8 @@ __device__ __forceinline__ void mma16816s(float (&d)[4], uint32_t a0, uint32_t a
 __device__ __forceinline__ uint32_t cta_begin(uint32_t c, uint32_t U, uint32_t C) { return (c * U) / C; }
 __device__ __forceinline__ int cta_of_unit(uint32_t u, uint32_t U, uint32_t C) { return (int)(((u + 1) * C - 1) / U); }
 
-// value of column e (0..7) of a thread's 8-column group, row t of the token pair
-#define NQ_TOTAL_AT(tot, e, t) tot[((e) & 1 ? 4 + ((e) >> 1) : ((e) >> 1)) >> 1][2 * (((e) & 1 ? 4 + ((e) >> 1) : ((e) >> 1)) & 1) + (t)]
-
 template <int MT, bool BF16, bool NORM>
-__global__ void __launch_bounds__(kStreamThreads, StreamCfg<MT>::kCtasPerSm)
+__global__ void __launch_bounds__(StreamCfg<MT>::kThreads, StreamCfg<MT>::kCtasPerSm)
 stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_sc,
               const __grid_constant__ CUtensorMap tm_z, const StreamParams p) {
   constexpr uint32_t LO = 0x000F000Fu, HI = 0x00F000F0u;
@@ -121,13 +120,14 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes, kOffX1 = Cfg::kOffX1, kOffSc = Cfg::kOffSc,
                 kOffZ = Cfg::kOffZ, kOffXs = Cfg::kOffXs, kSlotFloats = Cfg::kSlotFloats;
   constexpr uint32_t kStageTx = Cfg::kStageTx;
+  constexpr int kChunks = Cfg::kChunks, kConsumerWarps = Cfg::kConsumerWarps;
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[kStages], bar_empty[kStages], bar_xs[kStages];
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));  // same place, generic pointer
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t U = p.U, C = (uint32_t)p.nctas;
   const uint32_t u_begin = cta_begin(blockIdx.x, U, C), u_end = cta_begin(blockIdx.x + 1, U, C);
   const int nunits = (int)(u_end - u_begin);
@@ -146,31 +146,38 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 
   if (warp == kConsumerWarps) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0) {
-      prefetch_tmap(&tm_w); prefetch_tmap(&tm_sc); prefetch_tmap(&tm_z);
-      int tile = (int)(u_begin / G), grp = (int)(u_begin % G);
-      int issued = 0;
-      bool ok = true;
-      // Everything this thread requests (packed weights, scales, zero-points) is read-only, so it
-      // does not wait for the kernel ahead of this one on the stream; the activations come through
-      // the activation warp, which does.
-      for (int i = 0; i < nunits; ++i) {
-        const int s = i % kStages;
-        if (i >= kStages && !mbar_wait(smem_u32(&bar_empty[s]), ((i / kStages) - 1) & 1)) { ok = false; break; }
-        const uint32_t st = smem_base + s * kStageBytes, bar = smem_u32(&bar_full[s]);
+    // (a whole warp, see elect_one)
+    const bool el = elect_one();
+    if (el) { prefetch_tmap(&tm_w); prefetch_tmap(&tm_sc); prefetch_tmap(&tm_z); }
+    __syncwarp();
+    int tile = (int)(u_begin / G), grp = (int)(u_begin % G);
+    int issued = 0, s = 0;
+    uint32_t phase = 1;      // parity of the phase in which the stage was last given back
+    bool ok = true;
+    // Everything this warp requests (packed weights, scales, zero-points) is read-only, so it
+    // does not wait for the kernel ahead of this one on the stream; the activations come through
+    // the activation warp, which does.
+    for (int i = 0; i < nunits; ++i) {
+      if (i >= kStages) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&bar_empty[s]), phase));
+        if (!ok) break;
+      }
+      const uint32_t st = smem_base + s * kStageBytes, bar = smem_u32(&bar_full[s]);
+      if (el) {
         mbar_expect_tx(bar, kStageTx);
         tma_load_2d(st + kOffW0, &tm_w, tile * 64, grp * kUnitK, bar);
         tma_load_2d(st + kOffW1, &tm_w, tile * 64 + 32, grp * kUnitK, bar);
         tma_load_2d(st + kOffSc, &tm_sc, tile * 256, grp, bar);
         tma_load_2d(st + kOffZ, &tm_z, tile * 64, grp, bar);
-        ++issued;
-        if (++grp == G) { grp = 0; ++tile; }
       }
-      if (!ok) { grid_dependency_wait(); atomicExch(p.counters + kStatusWord, NQB200_ERR_WAIT_TIMEOUT); }
-      // do not leave while a copy of ours may still be landing in this CTA's shared memory
-      for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
-        mbar_wait(smem_u32(&bar_full[i % kStages]), (i / kStages) & 1);
+      ++issued;
+      if (++grp == G) { grp = 0; ++tile; }
+      if (++s == kStages) { s = 0; phase ^= 1u; }
     }
+    if (!ok) { grid_dependency_wait(); if (el) atomicExch(p.counters + kStatusWord, NQB200_ERR_WAIT_TIMEOUT); }
+    // do not leave while a copy of ours may still be landing in this CTA's shared memory
+    for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
+      mbar_wait(smem_u32(&bar_full[i % kStages]), (i / kStages) & 1);
     return;
   }
   if (warp == kConsumerWarps + 1) {
@@ -242,22 +249,27 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   }
 
   // ------------------------------------------------------------------ consumers
-  const int gq = lane >> 2, tig = lane & 3;
-  const int w = warp;
-  const int chunk = 2 * (w & 3) + (gq >> 2), inword = (gq & 3) * 4;
-  const uint32_t w_off = (w >> 2) ? kOffW1 : kOffW0;
-  // rows 16ks + 2tig + {0,1,8,9}: (row & 7) is 2tig or 2tig+1
-  const uint32_t sw_even = ((uint32_t)(chunk ^ ((2 * tig) & 7)) << 4) + inword;
-  const uint32_t sw_odd = ((uint32_t)(chunk ^ ((2 * tig + 1) & 7)) << 4) + inword;
-  const uint32_t row0 = (uint32_t)(2 * tig) * 128;
+  const int gq = lane >> 2, tig = lane & 3, odd = gq & 1;
+  // Chunk c (of 16 in the tile): 32 columns, 16 bytes of every packed row.  ldmatrix.trans gives a thread four nibbles of rows k and
+  // k + 1 per register, every second column of word gq / 2 of the chunk: nibble j is column 2 j + odd of the word.  Nibbles 2 b and
+  // 2 b + 1 are rows gq and gq + 8 of the chunk's mma b.  A load covers two k-steps: lane l addresses row 32 kp + l, where 16-byte chunk
+  // c of the box sits at chunk c ^ (l & 7).
+  uint32_t w_off[kChunks];
+#pragma unroll
+  for (int ch = 0; ch < kChunks; ++ch) {
+    const int c = kChunks * warp + ch;
+    w_off[ch] = (c >> 3 ? kOffW1 : kOffW0) + (uint32_t)lane * 128u + ((uint32_t)((c & 7) ^ (lane & 7)) << 4);
+  }
+  // Activations: with 16 tokens a load brings both halves of a k-step for both token tiles, with 8 the halves of two k-steps.
+  const uint32_t x_row = (uint32_t)((lane & 7) + (MT == 2 ? 8 * (lane >> 4) : 0)) * 128u;
+  const uint32_t x_chunk = (uint32_t)((((lane >> 3) & 1) + (MT == 1 ? 2 * (lane >> 4) : 0)) ^ (lane & 7));
+  uint32_t lo_mask, magic;       // bf16: see and_or
+  asm volatile("mov.u32 %0, %1;" : "=r"(lo_mask) : "n"(LO));
+  asm volatile("mov.u32 %0, %1;" : "=r"(magic) : "n"(0x43004300u));
 
-  float total[MT][4][4];
+  float total[kChunks][MT][4][2];   // [nibble][token of the pair]
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) total[mt][b][i] = 0.f;
+  for (int i = 0; i < kChunks * MT * 8; ++i) (&total[0][0][0][0])[i] = 0.f;
 
   int tile = (int)(u_begin / G), grp = (int)(u_begin % G);
   const int first_tile = tile;
@@ -276,69 +288,68 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       alive = false;
       break;
     }
+    const uint32_t stage = smem_base + s * kStageBytes;
     const uint8_t* st = smem_gen + s * kStageBytes;
-    const uint8_t* wb = st + w_off + row0;
 
-    float acc[MT][4][4];
+    float acc[kChunks][MT][2][4];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[mt][b][q] = 0.f;
-    }
+    for (int q = 0; q < kChunks * MT * 8; ++q) (&acc[0][0][0][0])[q] = 0.f;
 
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      const uint8_t* rb = wb + ks * 16 * 128;
-      const uint32_t w0 = lds32(rb, sw_even), w1 = lds32(rb, 128 + sw_odd);
-      const uint32_t w2 = lds32(rb, 8 * 128 + sw_even), w3 = lds32(rb, 9 * 128 + sw_odd);
-      uint32_t xb0[MT], xb1[MT];
-      const uint8_t* xbox = st + ((ks >> 2) ? kOffX1 : kOffX0);
+    for (int kp = 0; kp < 4; ++kp) {     // two k-steps
+      uint32_t R[kChunks][4];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const uint8_t* xr = xbox + (uint32_t)(8 * mt + gq) * 128 + tig * 4;
-        xb0[mt] = lds32(xr, (uint32_t)((2 * (ks & 3)) ^ gq) << 4);
-        xb1[mt] = lds32(xr, (uint32_t)((2 * (ks & 3) + 1) ^ gq) << 4);
+      for (int ch = 0; ch < kChunks; ++ch) ldmatrix_x4_trans(R[ch][0], R[ch][1], R[ch][2], R[ch][3], stage + w_off[ch] + kp * 4096u);
+      uint32_t xb[2][MT][2];             // [k-step][token tile][half]
+      const uint32_t xbox = stage + (kp >> 1 ? kOffX1 : kOffX0) + x_row;
+      if (MT == 1) {
+        ldmatrix_x4(xb[0][0][0], xb[0][0][1], xb[1][0][0], xb[1][0][1], xbox + ((uint32_t)(4 * (kp & 1)) ^ x_chunk) * 16u);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          ldmatrix_x4(xb[k][0][0], xb[k][0][1], xb[k][MT - 1][0], xb[k][MT - 1][1], xbox + ((uint32_t)(4 * (kp & 1) + 2 * k) ^ x_chunk) * 16u);
       }
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const uint32_t sel = (uint32_t)b | ((uint32_t)b << 4) | ((uint32_t)(4 + b) << 8) | ((uint32_t)(4 + b) << 12);
-        const uint32_t p01 = __byte_perm(w0, w1, sel), p23 = __byte_perm(w2, w3, sel);
-        uint32_t a0, a1, a2, a3;
-        if (BF16) {
-          a0 = (p01 & LO) | 0x43004300u; a1 = ((p01 >> 4) & LO) | 0x43004300u;
-          a2 = (p23 & LO) | 0x43004300u; a3 = ((p23 >> 4) & LO) | 0x43004300u;
-        } else {
-          a0 = p01 & LO; a1 = p01 & HI; a2 = p23 & LO; a3 = p23 & HI;
-        }
+      for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) mma16816s<BF16>(acc[mt][b], a0, a1, a2, a3, xb0[mt], xb1[mt]);
-      }
+        for (int ch = 0; ch < kChunks; ++ch)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const uint32_t r0 = R[ch][2 * k] >> (8 * b), r1 = R[ch][2 * k + 1] >> (8 * b);
+            uint32_t a0, a1, a2, a3;
+            if (BF16) {
+              a0 = and_or(r0, lo_mask, magic); a1 = and_or(R[ch][2 * k] >> (8 * b + 4), lo_mask, magic);
+              a2 = and_or(r1, lo_mask, magic); a3 = and_or(R[ch][2 * k + 1] >> (8 * b + 4), lo_mask, magic);
+            } else {
+              a0 = r0 & LO; a1 = r0 & HI; a2 = r1 & LO; a3 = r1 & HI;
+            }
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) mma16816s<BF16>(acc[ch][mt][b], a0, a1, a2, a3, xb[k][mt][0], xb[k][mt][1]);
+          }
     }
 
     // scale, power of two and zero-point, once per group
-    {
-      float xs[MT][2];
+    float xs[MT][2];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const float2 v = *reinterpret_cast<const float2*>(st + kOffXs + 4 * (8 * mt + 2 * tig));
-        xs[mt][0] = v.x; xs[mt][1] = v.y;
-      }
-      const uint4 sv = lds128(st, kOffSc + (uint32_t)(64 * w + 8 * gq) * 2);
-      const uint32_t zw = lds32(st, kOffZ + (uint32_t)(8 * w + gq) * 4);
+    for (int mt = 0; mt < MT; ++mt) {
+      const float2 v = *reinterpret_cast<const float2*>(st + kOffXs + 4 * (8 * mt + 2 * tig));
+      xs[mt][0] = v.x; xs[mt][1] = v.y;
+    }
+#pragma unroll
+    for (int ch = 0; ch < kChunks; ++ch) {
+      const uint32_t word = 4u * (kChunks * warp + ch) + (gq >> 1);
+      const uint4 sv = lds128(st, kOffSc + word * 16u);
+      const uint32_t zw = lds32(st, kOffZ + word * 4u) >> (16 * odd);
       const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int b = j >> 1, r = j & 1;
-        const int e = (j < 4) ? 2 * j : 2 * (j - 4) + 1;
-        const float sc = raw16_to_float<BF16>((uint16_t)((sw[e >> 1] >> (16 * (e & 1))) & 0xFFFF));
+      for (int j = 0; j < 4; ++j) {
+        const float sc = raw16_to_float<BF16>((uint16_t)((sw[j] >> (16 * odd)) & 0xFFFF));
         const float z = (float)((zw >> (4 * j)) & 0xF);
-        const float A = sc * (r ? MULT_HI : MULT_LO), B = sc * (z + OFF);
+        const float A = sc * (j & 1 ? MULT_HI : MULT_LO), B = sc * (z + OFF);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int t = 0; t < 2; ++t) total[mt][b][2 * r + t] += A * acc[mt][b][2 * r + t] - B * xs[mt][t];
+          for (int t = 0; t < 2; ++t) total[ch][mt][j][t] += A * acc[ch][mt][j >> 1][2 * (j & 1) + t] - B * xs[mt][t];
       }
     }
     __syncwarp();
@@ -346,51 +357,31 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 
     const bool tile_done = grp == G - 1;
     if (tile_done || i == nunits - 1) {
-      const int n0 = tile * kUnitN + 64 * w + 8 * gq;
-      const bool n_ok = n0 < p.N;
-      if (seg_begin == 0 && tile_done) {
-        // this CTA saw the tile's whole K: write the output directly
-        if (n_ok) {
+      const bool whole = seg_begin == 0 && tile_done;   // this CTA saw the tile's whole K: write the output directly
+      float* slot = p.slots + ((size_t)blockIdx.x * 2 + (tile == first_tile ? 0 : 1)) * kSlotFloats;
 #pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              const int m = 8 * mt + 2 * tig + t;
-              if (m < p.M) {
-                uint32_t o[4];
-#pragma unroll
-                for (int e = 0; e < 8; e += 2) {
-                  float v0 = NQ_TOTAL_AT(total[mt], e, t), v1 = NQ_TOTAL_AT(total[mt], e + 1, t);
-                  if (p.bias) { v0 += bias_to_float(p.bias, p.bias_dtype, n0 + e); v1 += bias_to_float(p.bias, p.bias_dtype, n0 + e + 1); }
-                  o[e >> 1] = (uint32_t)float_to_raw16<BF16>(v0) | ((uint32_t)float_to_raw16<BF16>(v1) << 16);
-                }
-                *reinterpret_cast<uint4*>(p.out + (size_t)m * p.N + n0) = make_uint4(o[0], o[1], o[2], o[3]);
-              }
-            }
-        }
-      } else {
-        // rows beyond M are never read
-        float* slot = p.slots + ((size_t)blockIdx.x * 2 + (tile == first_tile ? 0 : 1)) * kSlotFloats;
+      for (int ch = 0; ch < kChunks; ++ch) {
+        const int col = 32 * (kChunks * warp + ch) + 8 * (gq >> 1), n0 = tile * kUnitN + col + odd;
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             const int m = 8 * mt + 2 * tig + t;
-            if (m < p.M) {
-              float* dst = slot + m * kUnitN + 64 * w + 8 * gq;
-              __stcg(reinterpret_cast<float4*>(dst), make_float4(NQ_TOTAL_AT(total[mt], 0, t), NQ_TOTAL_AT(total[mt], 1, t),
-                                                                 NQ_TOTAL_AT(total[mt], 2, t), NQ_TOTAL_AT(total[mt], 3, t)));
-              __stcg(reinterpret_cast<float4*>(dst + 4), make_float4(NQ_TOTAL_AT(total[mt], 4, t), NQ_TOTAL_AT(total[mt], 5, t),
-                                                                     NQ_TOTAL_AT(total[mt], 6, t), NQ_TOTAL_AT(total[mt], 7, t)));
+            if (m >= p.M) continue;        // rows beyond M are never read
+            if (!whole) {
+              // a slot holds, of every eight columns, the even ones first
+              __stcg(reinterpret_cast<float4*>(slot + m * kUnitN + col + 4 * odd),
+                     make_float4(total[ch][mt][0][t], total[ch][mt][1][t], total[ch][mt][2][t], total[ch][mt][3][t]));
+            } else if (n0 < p.N) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                p.out[(size_t)m * p.N + n0 + 2 * j] =
+                    float_to_raw16<BF16>(p.bias ? total[ch][mt][j][t] + bias_to_float(p.bias, p.bias_dtype, n0 + 2 * j) : total[ch][mt][j][t]);
             }
           }
       }
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) total[mt][b][q] = 0.f;
+      for (int q = 0; q < kChunks * MT * 8; ++q) (&total[0][0][0][0])[q] = 0.f;
       seg_begin = 0;
     }
     if (++grp == G) { grp = 0; ++tile; }
@@ -399,8 +390,9 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 }
 
 // Sum over the contributors j, j+W, j+2W, ... of one tile's partial segments for token m, columns
-// col..col+3: all of a thread's loads (up to eight) are in flight together.  Returns the number of
-// contributors of the tile.
+// col..col+3: all of a thread's loads (up to eight) are in flight together.  A slot holds the even columns
+// of every eight ahead of the odd ones; two neighbouring threads exchange halves of what they added.  Returns
+// the number of contributors of the tile.
 template <int kReduceWays>
 __device__ __forceinline__ int reduce_tile_partials(const StreamParams& p, int C, int slot_floats, int tile, int m, int col, int j,
                                                     float4& v) {
@@ -425,6 +417,9 @@ __device__ __forceinline__ int reduce_tile_partials(const StreamParams& p, int C
     for (int d = 0; d < 8; ++d)
       if (c0 + kReduceWays * d < nc) { v.x += q[d].x; v.y += q[d].y; v.z += q[d].z; v.w += q[d].w; }
   }
+  const bool right = (threadIdx.x & 1) != 0;      // this thread added columns 1, 3, 5, 7 of its neighbour's and its own eight, or 0, 2, 4, 6
+  const float a = __shfl_xor_sync(0xFFFFFFFFu, right ? v.x : v.z, 1), b = __shfl_xor_sync(0xFFFFFFFFu, right ? v.y : v.w, 1);
+  v = right ? make_float4(a, v.z, b, v.w) : make_float4(v.x, a, v.y, b);
   return nc;
 }
 
@@ -626,10 +621,10 @@ static int stream_ctas_per_sm() {
     int n2 = 0;
     if (cudaFuncSetAttribute(stream_kernel<MT, BF16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem) != cudaSuccess ||
         cudaFuncSetAttribute(stream_kernel<MT, BF16, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stream_kernel<MT, BF16, false>, kStreamThreads, kStreamSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stream_kernel<MT, BF16, false>, StreamCfg<MT>::kThreads, kStreamSmem) != cudaSuccess ||
         cudaFuncSetAttribute(stream_kernel<MT, BF16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem) != cudaSuccess ||
         cudaFuncSetAttribute(stream_kernel<MT, BF16, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, stream_kernel<MT, BF16, true>, kStreamThreads, kStreamSmem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n2, stream_kernel<MT, BF16, true>, StreamCfg<MT>::kThreads, kStreamSmem) != cudaSuccess) {
       cudaGetLastError();
       return 0;
     }
@@ -644,8 +639,8 @@ template <int MT, bool BF16>
 static int launch_stream_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StreamParams& sp,
                            int max_contributors, bool silu, const PeerEpilogue* peer, cudaStream_t st) {
   // the attributes were set when the occupancy was measured
-  const int rc = sp.norm_ssq ? launch_overlapped(stream_kernel<MT, BF16, true>, dim3(sp.nctas), dim3(kStreamThreads), StreamCfg<MT>::kSmem, st, tw, ts, tz, sp)
-                             : launch_overlapped(stream_kernel<MT, BF16, false>, dim3(sp.nctas), dim3(kStreamThreads), StreamCfg<MT>::kSmem, st, tw, ts, tz, sp);
+  const int rc = sp.norm_ssq ? launch_overlapped(stream_kernel<MT, BF16, true>, dim3(sp.nctas), dim3(StreamCfg<MT>::kThreads), StreamCfg<MT>::kSmem, st, tw, ts, tz, sp)
+                             : launch_overlapped(stream_kernel<MT, BF16, false>, dim3(sp.nctas), dim3(StreamCfg<MT>::kThreads), StreamCfg<MT>::kSmem, st, tw, ts, tz, sp);
   if (rc != NQB200_OK || max_contributors <= 1) return rc;
   const int sf = (int)StreamCfg<MT>::kSlotFloats;
   if (peer)
