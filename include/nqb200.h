@@ -81,14 +81,15 @@ int nqb200_gemm(const void* x, const void* qweight, const void* qscales, const v
                 int64_t M, int64_t N, int64_t K, int64_t group_size, int dtype,
                 void* workspace, size_t workspace_bytes, void* stream);
 
-/* The merged gate|up projection of a Qwen3 MLP with its activation, for decode-sized M:
+/* The merged gate|up projection of a Qwen3 MLP with its activation:
  *   out[M, N/2] = silu(y[:, :N/2]) * y[:, N/2:],  y = x @ dequant(qweight, qscales, qzeros) (+ bias)
  * with the roundings of the separate steps (y, silu(gate) and the product each rounded to the
  * 16-bit type: models/qwen3_quantized.py:150 of the reference runs them as a linear, F.silu and a
- * multiply).  The activation runs in the kernel that adds the split-K partial sums, so it costs no
- * launch of its own.  Only where nqb200_gemm_gate_up_silu_supported() says 1 (M <= 16, group 128,
- * N a multiple of twice nqb200_decode_tile_columns(), K long enough that every column tile is split across
- * CTAs); elsewhere it
+ * multiply).  The activation costs no launch of its own: for decode-sized M it runs in the kernel that adds the
+ * split-K partial sums, for prompts in the two-SM kernel's epilogue.  Only where
+ * nqb200_gemm_gate_up_silu_supported() says 1 (group 128; either M <= 16, N a multiple of twice
+ * nqb200_decode_tile_columns() and K long enough that every column tile is split across CTAs, or N a multiple of 256
+ * and an M that the two-SM kernel takes in whole tiles); elsewhere it
  * returns NQB200_ERR_BAD_SHAPE and the caller runs nqb200_gemm + nqb200_silu_mul.  Workspace as
  * for nqb200_gemm with the same M, N, K. */
 int nqb200_gemm_gate_up_silu_supported(int64_t M, int64_t N, int64_t K, int64_t group_size, int dtype);

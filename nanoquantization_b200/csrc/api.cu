@@ -95,7 +95,7 @@ extern "C" int nqb200_decode_tile_columns(void) { return stream_tile_columns(); 
 
 extern "C" int nqb200_gemm_gate_up_silu_supported(int64_t M, int64_t N, int64_t K, int64_t g, int dtype) {
   if (check_shape(M, N, K, g, dtype) != NQB200_OK || M == 0) return 0;
-  return !umma_prefill_supports(M, N, K, g) && stream_silu_supported(M, N, K, g) ? 1 : 0;
+  return umma_prefill_supports(M, N, K, g) ? umma_pair_silu_supports(M, N, K, g) : stream_silu_supported(M, N, K, g);
 }
 
 extern "C" int nqb200_gemm_gate_up_silu(const void* x, const void* qweight, const void* qscales, const void* qzeros,
@@ -116,7 +116,7 @@ extern "C" int nqb200_gemm_gate_up_silu(const void* x, const void* qweight, cons
   a.M = (int)M; a.N = (int)N; a.K = (int)K; a.g = (int)g; a.dtype = dtype;
   a.ws = workspace; a.ws_bytes = workspace_bytes; a.stream = (cudaStream_t)stream;
   a.epilogue = 1;
-  return launch_stream(a);
+  return umma_prefill_supports(M, N, K, g) ? launch_umma_pair(a) : launch_stream(a);
 }
 
 extern "C" int nqb200_gemm_allreduce_supported(int64_t M, int64_t N, int64_t K, int64_t g, int dtype, int world, size_t slot_bytes) {

@@ -81,7 +81,7 @@ struct GemmArgs {
   const float* norm_ssq = nullptr; int norm_tiles = 0; const void* norm_weight = nullptr; float norm_eps = 0.f;
   const void* residual_in = nullptr; float* ssq_out = nullptr;
   const PeerEpilogue* peer = nullptr;  // all-reduce over peer memory in the reducing kernel (streaming decode kernel only)
-  int epilogue = 0;  // 1: the matrix is gate|up, out[M, N/2] = silu(gate) * up (streaming decode kernel only)
+  int epilogue = 0;  // 1: the matrix is gate|up, out[M, N/2] = silu(gate) * up (streaming decode and two-SM kernels)
 };
 
 int launch_decode_mma(const GemmArgs& a);
@@ -103,6 +103,7 @@ double umma_prefill_estimate_us(int64_t M, int64_t N, int64_t K);
 int launch_umma_pair(const GemmArgs& a);
 bool umma_pair_supports(int64_t M, int64_t N, int64_t K, int64_t g);
 size_t umma_pair_workspace_bytes(int64_t M, int64_t N, int64_t K);
+bool umma_pair_silu_supports(int64_t M, int64_t N, int64_t K, int64_t g);
 int umma_pair_launches(int64_t M, int64_t N, int64_t K);
 bool decode_mma_supports(int64_t M, int64_t N, int64_t K, int64_t g);
 

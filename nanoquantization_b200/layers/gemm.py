@@ -318,7 +318,7 @@ class WQLinear_GEMM(nn.Module):
     @torch.no_grad()
     def forward_silu_mul(self, x: torch.Tensor) -> torch.Tensor:
         """For a merged gate|up projection: ``silu(y[..., :N/2]) * y[..., N/2:]`` with ``y = forward(x)``,
-        bit-identical to running the three steps one after the other.  For decode-sized inputs the
+        bit-identical to running the three steps one after the other.  For decode-sized inputs and for prompts the
         activation runs inside the kernel that finishes the GEMM; otherwise as a launch of its own."""
         from . import fused
         x2 = x.reshape(-1, x.shape[-1])

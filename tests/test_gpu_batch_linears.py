@@ -5,6 +5,7 @@ import torch
 
 import nanoquantization_b200 as nq
 from nanoquantization_b200 import _lib
+from nanoquantization_b200.layers import fused
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -50,4 +51,46 @@ def test_dealings_and_edges(M, K, N, launches, dtype, bias):
     # half a unit of the result's last place, and float32 sums of K products
     bound = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) * ref.abs() + K * 2.0 ** -23 * (x.double().abs() @ W.abs())
     assert bool(((buf[1:M + 1].double() - ref).abs() <= bound).all())
+    _lib.check_workspaces()
+
+
+@pytest.mark.parametrize("M,K,N", [
+    (512, 256, 51200),        # several tiles a cluster: the staging area is handed back and forth
+    (2049, 256, 24576),       # a last tile of one token: one SM has tokens to finish, the other none
+    (700, 4096, 24576),       # tokens beyond the input within a tile
+    (1000, 1024, 19200),      # the columns of one half end inside what the plain call takes as a tile
+    (4096, 1024, 6144),
+])
+@pytest.mark.parametrize("dtype,bias", [(torch.float16, True), (torch.bfloat16, False)])
+def test_gate_up_silu_of_prompts_is_the_separate_steps(M, K, N, dtype, bias):
+    lib, code = _lib.load(), 0 if dtype == torch.float16 else 1
+    assert lib.nqb200_gemm_gate_up_silu_supported(M, N, K, 128, code) == 1
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    m = nq.WQLinear_GEMM(4, 128, K, N, DEV, bias, dtype)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, device=DEV, dtype=torch.int64).to(torch.int32)  # noqa: E731
+    m.qweight.copy_(words(K, N // 8)); m.qzeros.copy_(words(K // 128, N // 8))
+    m.qscales.copy_((torch.rand(K // 128, N, generator=g, device=DEV) * 9e-3 + 1e-3).to(dtype))
+    if bias:
+        m.bias.copy_(torch.randn(N, generator=g, device=DEV))
+    x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
+    x[0] *= 100.0                                                     # gates at both ends of the sigmoid
+    want = fused.silu_mul(m(x))
+    for _ in range(2):
+        assert torch.equal(m.forward_silu_mul(x), want)               # every rounding is the same
+    _lib.check_workspaces()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gate_up_silu_of_every_gate(dtype):
+    """All 65536 patterns of a gate, as the bias of columns whose weights are zero."""
+    M, K, N = 512, 256, 131072
+    assert _lib.load().nqb200_gemm_gate_up_silu_supported(M, N, K, 128, 0 if dtype == torch.float16 else 1) == 1
+    m = nq.WQLinear_GEMM(4, 128, K, N, DEV, True, dtype)
+    m.qweight.zero_(); m.qzeros.zero_(); m.qscales.fill_(1.0)
+    gates = torch.arange(-2 ** 15, 2 ** 15, device=DEV, dtype=torch.int32).to(torch.int16).view(dtype)
+    x = torch.zeros(M, K, device=DEV, dtype=dtype)
+    for up in (1.0, -0.7):
+        m.bias.copy_(torch.cat([gates, torch.full_like(gates, up)]))
+        want = fused.silu_mul(m(x))
+        assert torch.equal(m.forward_silu_mul(x).view(torch.int16), want.view(torch.int16))
     _lib.check_workspaces()
