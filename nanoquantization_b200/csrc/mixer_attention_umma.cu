@@ -1,18 +1,33 @@
 // Chunk-masked attention of prompts on the 5th-generation tensor cores (head sizes 64 and 128, cache pages of a
 // multiple of 128 tokens); what it computes is stated at nqb200_chunk_attention.
 //
-// One CTA takes 256 queries of one head as two tiles of 128 and walks over key tiles of 128.
-//   warp 0        TMA: Q once, then a two-stage ring of K tiles and one of V tiles, straight from the pages.
-//   warp 1        one thread issues tcgen05.mma: S = Q K^T (both operands in shared memory) and O += P V (P in
-//                 tensor memory, V in shared memory as it lies there: the operand's rows are keys).
-//   warps 4-7     softmax of tile 0, a thread per query row; warps 8-11 the same for tile 1.
-// Tensor memory holds S of both tiles (128 columns each) and O of both; P overwrites the first half of its S.  The two
-// tiles take turns on the tensor pipe while the other one's softmax runs.  The running maximum is only moved (and O
-// rescaled) when it falls behind by more than 8 in log2 units: the weights stay below 2^8 and the sums exact enough,
-// and after a row's first tiles it hardly ever happens.  The cap is monotonic, so the maximum is taken over raw scores.
-// For scores well inside the cap tanh is its Taylor series, which costs fused multiply-adds on register pairs only; up to
+// One CTA takes 256 queries of one head as two tiles of 128 and walks over key tiles of 128, each in two halves of 64.
+//   warp 0        TMA: Q once, then two-stage rings of K tiles and of V tiles, straight from the pages.
+//   warps 1, 2    one lane of each issues tcgen05.mma for a query tile: S = Q K^T of a half (both operands in shared memory)
+//                 and O += P V (P in tensor memory, V in shared memory as it lies there: the operand's rows are keys).
+//   warps 4-19    softmax: four warps for each half of each query tile, a thread per row and half.
+// Tensor memory holds S of both tiles (two halves of 64 columns each) and O of both; P overwrites the first half of its own S.
+// So four chains S -> weights -> O += P V -> next S run beside each other, and a scheduler has a warp of each.  What bounds it:
+// per 256 x 128 scores the tensor pipe needs 2560 cycles (S 48 per MMA of N = 64, which shared memory sets, O 64), the
+// exponentials 2048, and about 4200 pass, because the chains meet at the pipes.  8192 tokens of 32 heads, chunks of 4096, and in one chunk:
+// 545 -> 352 us and 929 -> 586; sigmoid weights in one chunk 883 -> 596 (before: whole tiles, one softmax thread per row, one
+// polling issuer).  The steps on the way, one chunk: rows halved among twice the warps 866, an issuer per query tile 824,
+// S and P by halves 621, the short series 578, its coefficients in terms of s 567, sums of the rounded weights 576, a row's own
+// reference 586 (these two for the error, see below).  An own
+// warp for S beside the two for O (592), polling instead of suspended softmax waits (579) and query tiles started apart (with whole
+// tiles, 849 against 824) gained nothing.
+//
+// The weights are 2^(score - m).  A cap bounds the scores, and up to kBound in log2 units m is the maximum of the
+// first tile with a key of the row's chunk (the row's two threads exchange theirs), or the sink, or kSpan below the cap, whichever is the largest: no weight is above 2^kSpan
+// and those that vanish are below 2^-126 of one that is there.  (A fixed m, the same for all rows, is 1 % faster and has
+// up to 25 % more error in the mean: the largest weight of a short row should be a power of two, so that its rounding to bf16
+// costs nothing.)  Without a cap, or with a wider one, m follows the running maximum when it falls behind by more than 8 in
+// log2 units, and O is rescaled: the weights stay below 2^8, and after a row's first tiles it hardly ever happens.  The cap
+// is monotonic, so the maximum is taken over raw scores.
+// For scores well inside the cap tanh is its Taylor series, which costs fused multiply-adds on register pairs only: three terms
+// up to a tenth of the cap, where what they leave out (0.054 y^6) is below float's rounding, five terms beyond; up to
 // twice the cap it is the seventh convergent of Lambert's continued fraction (one reciprocal more per score); a warp
-// whose tile has a larger score, or needs a mask, takes the general path.
+// whose half tile has a larger score, or needs a mask, takes the general path.
 //
 // Sigmoid weights (nqb200_attention.sigmoid) need no maximum and no sum: a weight is 1 / (1 + 2^x), two weights share one
 // reciprocal, 1 / a = b / (a b), with x clamped to 60 so that a b stays finite (weights below 2^-60 are 2^-60).
@@ -22,13 +37,14 @@
 #include "mixers.cuh"
 #include "tma_utils.cuh"
 #include "umma_utils.cuh"
+#include <type_traits>
 
 namespace nqb200 {
 namespace att {
 
-constexpr int kTile = 128, kThreads = 384;
+constexpr int kTile = 128, kThreads = 640;
 constexpr uint32_t kColS = 0, kColO = 256, kTmemCols = 512;
-constexpr float kLog2e = 1.4426950408889634f, kLag = 8.f, kSeriesRange = 0.4f, kFractionRange = 2.f;
+constexpr float kLog2e = 1.4426950408889634f, kLag = 8.f, kSeriesRange = 0.4f, kShortRange = 0.1f, kFractionRange = 2.f, kBound = 80.f, kSpan = 100.f;
 
 struct Params {
   nqb200_batch bt;
@@ -61,7 +77,24 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
 __device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   return __all_sync(0xFFFFFFFFu, wait_bar(bar, parity, abort_flag, status));
 }
-__device__ __forceinline__ bool test_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xFFFFFFFFu, mbar_test_wait(smem_u32(bar), parity)); }
+// The issuers' waits poll: a suspended warp is woken late, and the tensor pipe has nothing queued meanwhile.
+__device__ __forceinline__ bool poll_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  const uint32_t b = smem_u32(bar);
+  unsigned long long t0 = 0;
+  for (uint32_t polls = 0;;) {
+    if (__all_sync(0xFFFFFFFFu, mbar_test_wait(b, parity))) return true;
+    if ((++polls & 255u) == 0) {
+      const unsigned long long t = global_timer_ns();
+      if (!t0) t0 = t;
+      const bool late = t - t0 > kWaitLimitNs;
+      if (late) {
+        *abort_flag = 1;
+        if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
+      }
+      if (__any_sync(0xFFFFFFFFu, late || *abort_flag != 0)) return false;
+    }
+  }
+}
 
 // D[tmem] (+)= A[smem descriptor] * B[smem descriptor]; the descriptors' high halves are the same.
 __device__ __forceinline__ void umma_ss_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
@@ -108,10 +141,20 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 }
 __device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 __device__ __forceinline__ float min3(float a, float b, float c) { float r; asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+__device__ __forceinline__ float max3_abs(float a, float b, float c) { float r; asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 __device__ __forceinline__ float ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// The sum that a row's result is divided by takes the weights as the product does, rounded to bf16: where one stands out its
+// rounding cancels.  Against sums of the unrounded ones the error to float64 is 1 to 8 % smaller in the mean, for every
+// kind of scores that the tests have.
+__device__ __forceinline__ uint64_t add_rounded(uint64_t sum, uint32_t w) {
+  float a, b; unpair2(sum, a, b);
+  asm("{\n .reg .b16 lo, hi;\n mov.b32 {lo, hi}, %2;\n add.f32.bf16 %0, lo, %0;\n add.f32.bf16 %1, hi, %1;\n}" : "+f"(a), "+f"(b) : "r"(w));
+  return pair2(a, b);
 }
 
 template <int D, int V>
@@ -121,7 +164,8 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   constexpr uint32_t kQBytes = kTile * D * 2, kKBytes = kTile * D * 2, kVBytes = kTile * V * 2, kBox = kTile * 128;
   constexpr uint32_t kOffK = 2 * kQBytes, kOffV = kOffK + 2 * kKBytes;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_q, bar_kfull[2], bar_kfree[2], bar_vfull[2], bar_vfree[2], bar_s[2], bar_p[2][2], bar_pv[2], bar_o[2], bar_drain;
+  __shared__ __align__(8) uint64_t bar_q, bar_kfull[2], bar_kfree[2], bar_vfull[2], bar_vfree[2], bar_s[2][2], bar_p[2][2], bar_pv[2][2], bar_o[2], bar_x[2][4], bar_drain;
+  __shared__ float s_x[2][2][2][kTile];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
@@ -144,12 +188,13 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&bar_q), 1);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(smem_u32(&bar_kfull[s]), 1); mbar_init(smem_u32(&bar_kfree[s]), 1);
-      mbar_init(smem_u32(&bar_vfull[s]), 1); mbar_init(smem_u32(&bar_vfree[s]), 1);
-      mbar_init(smem_u32(&bar_s[s]), 1); mbar_init(smem_u32(&bar_p[s][0]), 4); mbar_init(smem_u32(&bar_p[s][1]), 4);
-      mbar_init(smem_u32(&bar_pv[s]), 1); mbar_init(smem_u32(&bar_o[s]), 1);
+      mbar_init(smem_u32(&bar_kfull[s]), 1); mbar_init(smem_u32(&bar_kfree[s]), 2);
+      mbar_init(smem_u32(&bar_vfull[s]), 1); mbar_init(smem_u32(&bar_vfree[s]), 2);
+      mbar_init(smem_u32(&bar_s[s][0]), 1); mbar_init(smem_u32(&bar_s[s][1]), 1); mbar_init(smem_u32(&bar_p[s][0]), 4); mbar_init(smem_u32(&bar_p[s][1]), 4);
+      mbar_init(smem_u32(&bar_pv[s][0]), 1); mbar_init(smem_u32(&bar_pv[s][1]), 1); mbar_init(smem_u32(&bar_o[s]), 1);
     }
-    mbar_init(smem_u32(&bar_drain), 1);
+    for (int s = 0; s < 8; ++s) mbar_init(smem_u32(&bar_x[s >> 2][s & 3]), 2);
+    mbar_init(smem_u32(&bar_drain), 2);
     s_abort_i = 0;
     mbar_fence_init();
   }
@@ -159,6 +204,8 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_after();
   const uint32_t tmem = s_tmem;
 
+  // of the 96 registers a thread that 640 threads can have: 56 x 128 + 104 x 512 <= 96 x 640
+  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA
     const bool el = elect_one();
@@ -196,84 +243,56 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       mbar_wait(smem_u32(&bar_kfull[j & 1]), (j >> 1) & 1);
       mbar_wait(smem_u32(&bar_vfull[j & 1]), (j >> 1) & 1);
     }
-  } else if (warp == 1) {
+  } else if (warp < 3) {
     // ------------------------------------------------------------------ MMA
-    // One warp, of which one lane issues (elect_one: 8192 tokens of 32 heads, chunks of 4096, 647 -> 575 us against a single
-    // thread), runs both tiles as two little state machines and never blocks on one of them: it polls for the first and the
-    // second half of a tile's weights (then issues that half of O += P V) and for that product's end (P has been read: then S
-    // of the next key tile may overwrite it).  A ring stage is handed back by whichever tile uses it second.
+    // A warp per query tile, of which one lane issues (elect_one).  A half's S may overwrite its weights once their product has
+    // completed.  A ring stage is handed back by both warps, by its only user twice.
+    const int q = warp - 1;
     const bool el = elect_one();
-    const uint32_t idesc_s = umma_idesc(1, 128, kTile);
+    const uint32_t idesc_s = umma_idesc(1, 128, kTile / 2);
     const uint32_t idesc_o = umma_idesc(1, 128, V) | (1u << 16);   // B's rows run along k
-    const uint64_t dq = umma_smem_desc_sw128(smem), dk = umma_smem_desc_sw128(smem + kOffK), dv = smem_desc_mn(smem + kOffV, kBox);
+    const uint64_t dq = umma_smem_desc_sw128(smem + q * kQBytes), dk = umma_smem_desc_sw128(smem + kOffK), dv = smem_desc_mn(smem + kOffV, kBox);
     const uint32_t k_hi = (uint32_t)(dq >> 32), v_hi = (uint32_t)(dv >> 32), q_lo = (uint32_t)dq, k_lo = (uint32_t)dk, v_lo = (uint32_t)dv;
-    auto scores = [&](int q, int s) {
-      const uint32_t a = q_lo + q * (kQBytes >> 4), bk = k_lo + s * (kKBytes >> 4), d = tmem + kColS + q * 128;
-      if (el) {
+    const uint32_t tS = tmem + kColS + q * 128, tO = tmem + kColO + q * 128;
+    const int mine = nq[q], others = nq[q ^ 1];
+    bool ok = mine > 0 && poll_bar_warp(&bar_q, 0, s_abort, p.status);
+    for (int j = 0; ok && j <= mine; ++j) {
+      const int i = j - 1, s = j & 1, so = s ^ 1;
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss_lohi(d, a + (ks >> 2) * (kBox >> 4) + (ks & 3) * 2, bk + (ks >> 2) * (kBox >> 4) + (ks & 3) * 2, k_hi, idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit(smem_u32(&bar_s[q]));
-      }
-    };
-    bool ok = wait_bar_warp(&bar_q, 0, s_abort, p.status) && wait_bar_warp(&bar_kfull[0], 0, s_abort, p.status);
-    const int users = nq[1] > 0 ? 2 : 1;
-    // tile of the next product; 0, 1: waits for that half of the weights, 2: for the product; users that have still to
-    // issue on K / V tile j (by j & 1)
-    int jq[2] = {0, 0};
-    int phase[2] = {0, 0};
-    auto users_of = [&](int j) { return users == 2 ? (j < nq[0]) + (j < nq[1]) : 1; };
-    int kleft[2] = {0, users_of(1)}, vleft[2] = {users_of(0), users_of(1)};
-    if (ok) {
-      tc_fence_after();
-      for (int q = 0; q < users; ++q) scores(q, 0);
-      if (el) umma_commit(smem_u32(&bar_kfree[0]));
-      kleft[0] = users_of(2);
-    }
-    unsigned long long t_last = global_timer_ns();
-    uint32_t polls = 0;
-    while (ok && (jq[0] < nq[0] || jq[1] < nq[1])) {
-      bool moved = false;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int j = jq[q], s = j & 1, sn = s ^ 1;
-        if (j >= nq[q]) continue;
-        if (phase[q] < 2) {
-          const int half = phase[q];
-          if (!test_warp(&bar_p[q][half], s) || !test_warp(&bar_vfull[s], (j >> 1) & 1)) continue;
+      for (int half = 0; half < 2; ++half) {
+        if (j > 0) {      // O += P V of the tile before
+          if (half == 0) ok = poll_bar_warp(&bar_vfull[so], (i >> 1) & 1, s_abort, p.status);
+          ok = ok && poll_bar_warp(&bar_p[q][half], so, s_abort, p.status);
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t d = tmem + kColO + q * 128, pa = tmem + kColS + q * 128 + half * 32, bv = v_lo + s * (kVBytes >> 4) + half * (8192 >> 4);
           if (el) {
 #pragma unroll
             for (int ks = 0; ks < kTile / 32; ++ks)
-              umma_ts_lohi(d, pa + ks * 8, bv + ks * (2048 >> 4), v_hi, idesc_o, (j > 0 || half > 0 || ks > 0) ? 1u : 0u);
+              umma_ts_lohi(tO, tS + half * 64 + ks * 8, v_lo + so * (kVBytes >> 4) + half * (8192 >> 4) + ks * (2048 >> 4), v_hi, idesc_o,
+                           (i > 0 || half > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(smem_u32(j == mine && half == 1 ? &bar_o[q] : &bar_pv[q][half]));
+            if (half == 1) {
+              umma_commit(smem_u32(&bar_vfree[so]));
+              if (i >= others) umma_commit(smem_u32(&bar_vfree[so]));
+            }
           }
-          phase[q] = half + 1;
-          if (half == 1) {
-            if (el) umma_commit(smem_u32(&bar_pv[q]));
-            if (--vleft[s] == 0) { if (el) umma_commit(smem_u32(&bar_vfree[s])); vleft[s] = users_of(j + 2); }
-            if (j == nq[q] - 1) { if (el) umma_commit(smem_u32(&bar_o[q])); jq[q] = j + 1; }
-          }
-        } else {
-          if (!test_warp(&bar_pv[q], s) || !test_warp(&bar_kfull[sn], ((j + 1) >> 1) & 1)) continue;
-          tc_fence_after();
-          scores(q, sn);
-          if (--kleft[sn] == 0) { if (el) umma_commit(smem_u32(&bar_kfree[sn])); kleft[sn] = users_of(j + 3); }
-          jq[q] = j + 1;
-          phase[q] = 0;
         }
-        moved = true;
-      }
-      if (moved) {
-        polls = 0;
-      } else if ((++polls & 63u) == 0) {
-        const unsigned long long now = global_timer_ns();
-        if (polls == 64) t_last = now;
-        if (__any_sync(0xFFFFFFFFu, *s_abort != 0)) ok = false;
-        else if (__any_sync(0xFFFFFFFFu, now - t_last > kWaitLimitNs)) {
-          *s_abort = 1;
-          if (p.status) atomicExch(p.status, NQB200_ERR_WAIT_TIMEOUT);
-          ok = false;
+        if (j < mine) {
+          if (j > 0) ok = poll_bar_warp(&bar_pv[q][half], so, s_abort, p.status);   // the weights have been read: their place takes the next scores
+          if (half == 0) ok = ok && poll_bar_warp(&bar_kfull[s], (j >> 1) & 1, s_abort, p.status);
+          if (!ok) break;
+          tc_fence_after();
+          if (el) {
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks)
+              umma_ss_lohi(tS + half * 64, q_lo + (ks >> 2) * (kBox >> 4) + (ks & 3) * 2,
+                           k_lo + s * (kKBytes >> 4) + half * (8192 >> 4) + (ks >> 2) * (kBox >> 4) + (ks & 3) * 2, k_hi, idesc_s, ks > 0 ? 1u : 0u);
+            umma_commit(smem_u32(&bar_s[q][half]));
+            if (half == 1) {
+              umma_commit(smem_u32(&bar_kfree[s]));
+              if (j >= others) umma_commit(smem_u32(&bar_kfree[s]));
+            }
+          }
         }
       }
     }
@@ -282,53 +301,96 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     mbar_wait(smem_u32(&bar_drain), 0);
   } else if (warp >= 4) {
     // -------------------------------------------------------------- softmax
-    const int q = (warp - 4) >> 2, quarter = warp & 3;
-    const uint32_t tS = tmem + ((uint32_t)(32 * quarter) << 16) + kColS + q * 128, tO = tmem + ((uint32_t)(32 * quarter) << 16) + kColO + q * 128;
-    const int i = i0 + q * kTile + quarter * 32 + lane, pos = pos0 + i, wfirst = pos - lane, wlast = wfirst + 31;
+    const int q = (warp - 4) >> 3, half = ((warp - 4) >> 2) & 1, quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t lanes = (uint32_t)(32 * quarter) << 16, tS = tmem + lanes + kColS + q * 128 + half * 64, tO = tmem + lanes + kColO + q * 128;
+    const int i = i0 + q * kTile + row, pos = pos0 + i, wfirst = pos - lane, wlast = wfirst + 31;
     const int lo = p.chunk > 0 ? pos / p.chunk * p.chunk : 0, lo_last = p.chunk > 0 ? wlast / p.chunk * p.chunk : 0;
-    const bool capped = p.softcap > 0.f;
+    const bool capped = p.softcap > 0.f, bounded = capped && p.softcap * kLog2e <= kBound;
     const float ysc = capped ? p.scale / p.softcap : p.scale, top = capped ? p.softcap * kLog2e : kLog2e;
     auto score = [&](float s) {   // in log2 units
       const float y = s * ysc;
       return top * (capped ? tanh_fast(y) : y);
     };
-    const uint64_t ysc2 = pair2(ysc, ysc), k1 = pair2(top, top), k3 = pair2(-top / 3.f, -top / 3.f), k5 = pair2(top * (2.f / 15.f), top * (2.f / 15.f)),
-                   k7 = pair2(-top * (17.f / 315.f), -top * (17.f / 315.f)), k9 = pair2(top * (62.f / 2835.f), top * (62.f / 2835.f));
-    auto half_done = [&](int half) {   // that half of the weights is in tensor memory
+    auto done = [&]() {           // this half of the weights is in tensor memory
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_p[q][half]));
     };
-    const float sg_scale = -p.scale * (p.temp ? p.temp[h] : 1.f) * kLog2e, sg_shift = p.bias ? -p.bias[h] * kLog2e : 0.f;
-    const uint64_t sg_scale2 = pair2(sg_scale, sg_scale), sg_shift2 = pair2(sg_shift, sg_shift), one2 = pair2(1.f, 1.f);
-    auto sigmoid2 = [&](uint32_t s0, uint32_t s1, float& w0, float& w1) {
-      float x0, x1;
-      unpair2(fma2(pair2(__uint_as_float(s0), __uint_as_float(s1)), sg_scale2, sg_shift2), x0, x1);
-      float d0, d1;
-      unpair2(add2(pair2(ex2(fminf(x0, 60.f)), ex2(fminf(x1, 60.f))), one2), d0, d1);
-      const float r = rcp_fast(d0 * d1);
-      w0 = r * d1;
-      w1 = r * d0;
+    int exchanges = 0;
+    auto exchange = [&](float mine, float& other) {   // with the thread that has the row's other half
+      const int x = exchanges & 1;
+      s_x[q][half][x][row] = mine;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar_x[q][quarter]));
+      const bool got = wait_bar_warp(&bar_x[q][quarter], x, s_abort, p.status);
+      tc_fence_after();
+      other = s_x[q][half ^ 1][x][row];
+      ++exchanges;
+      return got;
     };
+    const float sg_scale = -p.scale * (p.temp ? p.temp[h] : 1.f) * kLog2e, sg_shift = p.bias ? -p.bias[h] * kLog2e : 0.f;
     const float sink = p.sink ? p.sink[h] * kLog2e : -INFINITY;
-    float m = sink, l = 0.f;
+    const float floor = bounded ? top - kSpan : -INFINITY;
+    float m = p.sink ? fmaxf(sink, floor) : sink, l = 0.f;
     uint64_t lsum = pair2(0.f, 0.f);
+    // top tanh(y) by its series, TERMS powers of y^2 beyond the first (0: no cap).  The coefficients carry the powers of y / s.
+    const bool folded = ysc >= 1.f / 4096.f && ysc <= 4096.f;      // and none of them leaves the range of normal numbers
+    auto weights = [&](auto terms, const uint32_t (&r)[2][32], uint64_t nm2) {
+      constexpr int TERMS = decltype(terms)::value;
+      const float z = ysc * ysc, c1 = top * ysc, c3 = -c1 / 3.f * z, c5 = c1 * (2.f / 15.f) * z * z, c7 = -c1 * (17.f / 315.f) * z * z * z,
+                  c9 = c1 * (62.f / 2835.f) * z * z * z * z;
+      const uint64_t k1 = pair2(c1, c1), k3 = pair2(c3, c3), k5 = pair2(c5, c5), k7 = pair2(c7, c7), k9 = pair2(c9, c9);
+      uint64_t ls[2] = {lsum, 0};
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t w[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const uint64_t t = pair2(__uint_as_float(r[c][2 * e]), __uint_as_float(r[c][2 * e + 1]));
+          uint64_t f = k1;
+          if (TERMS) {
+            const uint64_t t2 = mul2(t, t);
+            f = TERMS == 4 ? fma2(fma2(k9, t2, k7), t2, k5) : k5;
+            f = fma2(fma2(f, t2, k3), t2, k1);
+          }
+          float x0, x1;
+          unpair2(fma2(t, f, nm2), x0, x1);
+          x0 = ex2(x0);
+          x1 = ex2(x1);
+          w[e] = pack_bf16(x0, x1);
+          ls[e & 1] = add_rounded(ls[e & 1], w[e]);
+        }
+        tmem_st16(tS + c * 16, w);
+      }
+      lsum = add2(ls[0], ls[1]);
+    };
     bool ok = true;
     for (int j = 0; j < nq[q]; ++j) {
-      ok = wait_bar(&bar_s[q], j & 1, s_abort, p.status);
-      if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+      ok = wait_bar_warp(&bar_s[q][half], j & 1, s_abort, p.status);
+      if (!ok) break;
       tc_fence_after();
-      const int key0 = kstart + j * kTile;
-      const bool masked = key0 + kTile - 1 > wfirst || key0 < lo_last;     // for any row of the warp
-      uint32_t r[4][32];     // the row's scores, all of them
+      const int key0 = kstart + j * kTile + half * 64;
+      const bool masked = key0 + 63 > wfirst || key0 < lo_last;     // for any row of the warp
+      uint32_t r[2][32];     // the row's scores, all of this half
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, r[c]);
+      for (int c = 0; c < 2; ++c) tmem_ld32(tS + c * 32, r[c]);
       tc_wait_ld();
       if (p.sigmoid) {
+        const uint64_t sg_scale2 = pair2(sg_scale, sg_scale), sg_shift2 = pair2(sg_shift, sg_shift), one2 = pair2(1.f, 1.f);
+        auto sigmoid2 = [&](uint32_t s0, uint32_t s1, float& w0, float& w1) {
+          float x0, x1;
+          unpair2(fma2(pair2(__uint_as_float(s0), __uint_as_float(s1)), sg_scale2, sg_shift2), x0, x1);
+          float d0, d1;
+          unpair2(add2(pair2(ex2(fminf(x0, 60.f)), ex2(fminf(x1, 60.f))), one2), d0, d1);
+          const float r = rcp_fast(d0 * d1);
+          w0 = r * d1;
+          w1 = r * d0;
+        };
         if (!masked) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < 2; ++c) {
             uint32_t w[16];
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
@@ -337,11 +399,10 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               w[e] = pack_bf16(x0, x1);
             }
             tmem_st16(tS + c * 16, w);
-            if (c == 1) half_done(0);
           }
         } else {
 #pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < 4; ++c) {
             uint32_t v[16], w[8];
             tmem_ld_32x32b_x16(tS + c * 16, v);
             tc_wait_ld();
@@ -353,68 +414,85 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               w[e] = pack_bf16(key <= pos && key >= lo ? x0 : 0.f, key + 1 <= pos && key + 1 >= lo ? x1 : 0.f);
             }
             tmem_st8(tS + c * 8, w);      // lies behind what has been read of S
-            if (c == 3) half_done(0);
           }
         }
-        half_done(1);
+        done();
         continue;
       }
-      float mx = -INFINITY, ab = 0.f;
-      if (!masked) {
-        float hi[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, lw[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+      float ab = 0.f;
+      if (bounded && j > 0 && !__any_sync(0xFFFFFFFFu, m == -INFINITY)) {
+        if (!masked) {
+          float hi[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const int k = (e >> 1) & 3;
-            hi[k] = max3(hi[k], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-            lw[k] = min3(lw[k], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-          }
-        mx = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
-        ab = fmaxf(mx, -fminf(fminf(lw[0], lw[1]), fminf(lw[2], lw[3])));
+            for (int e = 0; e < 32; e += 2) hi[(e >> 1) & 3] = max3_abs(hi[(e >> 1) & 3], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+          ab = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
+        }
       } else {
+        float mx = -INFINITY;
+        if (!masked) {
+          float hi[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, lw[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int key = key0 + c * 32 + e;
-            mx = (key <= pos && key >= lo) ? fmaxf(mx, __uint_as_float(r[c][e])) : mx;
-          }
-      }
-      const float mt = mx == -INFINITY ? mx : score(mx), mn = fmaxf(m, mt);
-      if (j == 0) {
-        l = p.sink ? ex2(sink - mn) : 0.f;
-        m = mn;
-      } else {
-        const bool move = mn > m + kLag;      // also from -inf
-        if (__any_sync(0xFFFFFFFFu, move)) {
-          const float f = move ? ex2(m - mn) : 1.f;
-          m = move ? mn : m;
-          l *= f;
-          float a, c2;
-          unpair2(lsum, a, c2);
-          lsum = pair2(a * f, c2 * f);
+            for (int e = 0; e < 32; e += 2) {
+              const int k = (e >> 1) & 3;
+              hi[k] = max3(hi[k], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+              lw[k] = min3(lw[k], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+            }
+          mx = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
+          ab = fmaxf(mx, -fminf(fminf(lw[0], lw[1]), fminf(lw[2], lw[3])));
+        } else {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              const int key = key0 + c * 32 + e;
+              mx = (key <= pos && key >= lo) ? fmaxf(mx, __uint_as_float(r[c][e])) : mx;
+            }
+        }
+        float mo;
+        if (!(ok = exchange(mx, mo))) break;
+        mx = fmaxf(mx, mo);
+        const float mt = mx == -INFINITY ? mx : fmaxf(score(mx), floor), mn = fmaxf(m, mt);
+        if (j == 0) {
+          l = p.sink && half == 0 ? ex2(sink - mn) : 0.f;
+          m = mn;
+        } else {
+          const bool move = mn > m + kLag;      // also from -inf
+          if (__any_sync(0xFFFFFFFFu, move)) {
+            const float f = move ? ex2(m - mn) : 1.f;
+            m = move ? mn : m;
+            l *= f;
+            float a, c2;
+            unpair2(lsum, a, c2);
+            lsum = pair2(a * f, c2 * f);
+            if (half == 0) {      // before its weights are reported, which both products of the tile wait for
 #pragma unroll 1
-          for (int c = 0; c < V / 8; ++c) {   // rare: small pieces, few registers
-            uint32_t o[8];
-            tmem_ld_32x32b_x8(tO + c * 8, o);
-            tc_wait_ld();
+              for (int c = 0; c < V / 8; ++c) {   // rare: small pieces, few registers
+                uint32_t o[8];
+                tmem_ld_32x32b_x8(tO + c * 8, o);
+                tc_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-            tmem_st8(tO + c * 8, o);
+                for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+                tmem_st8(tO + c * 8, o);
+              }
+              tc_wait_st();
+            }
           }
-          tc_wait_st();
         }
       }
       const float mu = m == -INFINITY ? 0.f : m;
-      const int range = masked ? 2 : !capped || __all_sync(0xFFFFFFFFu, ab * ysc <= kSeriesRange) ? 0 : __all_sync(0xFFFFFFFFu, ab * ysc <= kFractionRange) ? 1 : 2;
+      const uint64_t ysc2 = pair2(ysc, ysc), nm2 = pair2(-mu, -mu), k1 = pair2(top, top);
+      auto within = [&](float y) { return __all_sync(0xFFFFFFFFu, ab * ysc <= y); };      // for every score of the warp's
+      const int range = masked ? 2 : !capped || (folded && within(kSeriesRange)) ? 0 : within(kFractionRange) ? 1 : 2;
       if (range == 1) {
         // tanh y = y (10395 + 1260 y^2 + 21 y^4) / (10395 + 4725 y^2 + 210 y^4 + y^6)
-        const uint64_t n0 = pair2(10395.f, 10395.f), n1 = pair2(1260.f, 1260.f), n2 = pair2(21.f, 21.f), d1 = pair2(4725.f, 4725.f), d2 = pair2(210.f, 210.f),
-                       nm2 = pair2(-mu, -mu);
+        const uint64_t n0 = pair2(10395.f, 10395.f), n1 = pair2(1260.f, 1260.f), n2 = pair2(21.f, 21.f), d1 = pair2(4725.f, 4725.f), d2 = pair2(210.f, 210.f);
         uint64_t ls[2] = {lsum, 0};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2; ++c) {
           uint32_t w[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
@@ -425,44 +503,20 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             unpair2(fma2(num, pair2(rcp_fast(a), rcp_fast(c2)), nm2), x0, x1);
             x0 = ex2(x0);
             x1 = ex2(x1);
-            ls[e & 1] = add2(ls[e & 1], pair2(x0, x1));
             w[e] = pack_bf16(x0, x1);
+            ls[e & 1] = add_rounded(ls[e & 1], w[e]);
           }
           tmem_st16(tS + c * 16, w);
-          if (c == 1) half_done(0);
         }
         lsum = add2(ls[0], ls[1]);
       } else if (range == 0) {
-        const uint64_t nm2 = pair2(-mu, -mu);
-        uint64_t ls[4] = {lsum, 0, 0, 0};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t w[16];
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const uint64_t y = mul2(pair2(__uint_as_float(r[c][2 * e]), __uint_as_float(r[c][2 * e + 1])), ysc2);
-            uint64_t arg;
-            if (capped) {
-              const uint64_t y2 = mul2(y, y);
-              arg = fma2(y, fma2(fma2(fma2(fma2(k9, y2, k7), y2, k5), y2, k3), y2, k1), nm2);
-            } else {
-              arg = fma2(y, k1, nm2);
-            }
-            float x0, x1;
-            unpair2(arg, x0, x1);
-            x0 = ex2(x0);
-            x1 = ex2(x1);
-            ls[e & 3] = add2(ls[e & 3], pair2(x0, x1));
-            w[e] = pack_bf16(x0, x1);
-          }
-          tmem_st16(tS + c * 16, w);
-          if (c == 1) half_done(0);
-        }
-        lsum = add2(add2(ls[0], ls[1]), add2(ls[2], ls[3]));
+        if (!capped) weights(std::integral_constant<int, 0>(), r, nm2);
+        else if (within(kShortRange)) weights(std::integral_constant<int, 2>(), r, nm2);
+        else weights(std::integral_constant<int, 4>(), r, nm2);
       } else {
         // from tensor memory again, a piece at a time: compact code for the few tiles at the edges
 #pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 4; ++c) {
           uint32_t v[16], w[8];
           tmem_ld_32x32b_x16(tS + c * 16, v);
           tc_wait_ld();
@@ -474,27 +528,31 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               const int key = key0 + c * 16 + 2 * e + u;
               x[u] = (key <= pos && key >= lo) ? ex2(score(__uint_as_float(v[2 * e + u])) - mu) : 0.f;
             }
-            lsum = add2(lsum, pair2(x[0], x[1]));
             w[e] = pack_bf16(x[0], x[1]);
+            lsum = add_rounded(lsum, w[e]);
           }
           tmem_st8(tS + c * 8, w);      // lies behind what has been read of S
-          if (c == 3) half_done(0);
         }
       }
-      half_done(1);
+      done();
     }
     if (ok && nq[q] > 0) {
-      ok = wait_bar(&bar_o[q], 0, s_abort, p.status);
-      if (__all_sync(0xFFFFFFFFu, ok)) {
-        tc_fence_after();
-        float a, c2;
+      ok = wait_bar_warp(&bar_o[q], 0, s_abort, p.status);
+      float f = p.out_scale;
+      if (ok && !p.sigmoid) {
+        float a, c2, other;
         unpair2(lsum, a, c2);
-        const float f = p.sigmoid ? p.out_scale : p.out_scale / (l + a + c2);
-        bf16* dst = p.out + (size_t)(t0 + i) * p.out_stride + (size_t)h * V;
+        l += a + c2;
+        ok = exchange(l, other);
+        f /= l + other;
+      }
+      if (ok) {
+        tc_fence_after();
+        bf16* dst = p.out + (size_t)(t0 + i) * p.out_stride + (size_t)h * V + half * (V / 2);
 #pragma unroll
-        for (int c = 0; c < V / 32; ++c) {
+        for (int c = 0; c < V / 64; ++c) {
           uint32_t r[32];
-          tmem_ld32(tO + c * 32, r);
+          tmem_ld32(tO + half * (V / 2) + c * 32, r);
           tc_wait_ld();
           if (i < n) {
 #pragma unroll

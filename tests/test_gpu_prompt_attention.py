@@ -1,0 +1,64 @@
+"""Attention of prompts on the tcgen05 kernel, against float64: each way it takes a score (no cap, the cap's short and long series,
+the fraction, the exponential), with and without a running maximum, at the edges of its tiles and of chunks."""
+import math
+
+import pytest
+import torch
+
+from nanoquantization_b200 import _lib
+from nanoquantization_b200.engine.batch import StepBatch
+from nanoquantization_b200.layers import mixers as ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+H, G, BS = 4, 2, 128
+
+
+@pytest.mark.parametrize("D,V,chunk", [(128, 128, 0), (64, 128, 512), (128, 64, 700)])
+@pytest.mark.parametrize("softcap,spread,sink", [
+    (50.0, 1.0, None),          # scores a tenth of the cap at most: the short series; the cap bounds them, no running maximum
+    (50.0, 4.0, -3.0),          # the series
+    (50.0, 20.0, 0.5),          # the fraction
+    (20.0, 40.0, 45.0),         # beyond; a sink above every score
+    (50.0, 1.0, 100.0),         # a sink so far above that hardly anything is left
+    (120.0, 1.0, None),         # a cap too far for a fixed reference
+    (120.0, 60.0, 3.0),
+    (0.0, 1.0, None),           # no cap
+    (0.0, 30.0, 2.0),           # no cap and a maximum that moves
+    (400.0, 1.0, None),         # a cap so wide that its series' coefficients are not taken (some would leave the range of float)
+])
+def test_scores_of_every_range(D, V, chunk, softcap, spread, sink):
+    g = torch.Generator(device=DEV).manual_seed(D + V + chunk + int(softcap + spread))
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)  # noqa: E731
+    lengths, starts = [1000, 129, 257], [0, 640, 0]
+    total = [n + s for n, s in zip(lengths, starts)]
+    blocks = [-(-t // BS) for t in total]
+    first = [sum(blocks[:i]) + 1 for i in range(3)]
+    step = StepBatch.host([[0] * n for n in lengths], starts, [list(range(f, f + b)) for f, b in zip(first, blocks)], [0, 1, 2], max(blocks), BS).to(DEV)
+    kc, vc = rnd(sum(blocks) + 1, BS, G, D), rnd(sum(blocks) + 1, BS, G, V)
+    q = (rnd(sum(lengths), H * D).float() * spread).to(torch.bfloat16)
+    sinks = None if sink is None else torch.full((H,), sink, device=DEV)
+    desc = _lib.AttentionDesc(H, G, D, V, chunk, D ** -0.5, softcap, None if sinks is None else sinks.data_ptr(), 1.5)
+    out = torch.full((sum(lengths) + 1, H * V), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.chunk_attention(q, kc, vc, out[:-1], desc, step)
+    torch.cuda.synchronize()
+    assert bool((out[-1] == 7).all())
+    row = 0
+    for n, start, f, t in zip(lengths, starts, first, total):
+        k, v = (c[f:f + -(-t // BS)].reshape(-1, G, c.shape[-1])[:t].double().repeat_interleave(H // G, 1) for c in (kc, vc))
+        s = torch.einsum("ihd,jhd->hij", q[row:row + n].reshape(n, H, D).double(), k) * D ** -0.5
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        i, j = torch.arange(start, t, device=DEV)[:, None], torch.arange(t, device=DEV)[None, :]
+        s = s.masked_fill((j > i) | ((i // chunk != j // chunk) if chunk else False), -math.inf)
+        m = s.amax(-1, keepdim=True)
+        m = m if sink is None else m.clamp(min=sink)
+        p = (s - m).exp()
+        w = 1.5 * p / (p.sum(-1, keepdim=True) + (0.0 if sink is None else (sink - m).exp()))
+        ref, size = torch.einsum("hij,jhd->ihd", w, v), torch.einsum("hij,jhd->ihd", w, v.abs())
+        got = out[row:row + n].reshape(n, H, V).double()
+        # the result and every weight rounded to bf16 (2^-8 of each); a score's error of up to 2e-4 (float arithmetic on scores of up to 2^8, the
+        # series where they end)
+        bound = 2.0 ** -8 * ref.abs() + (2.0 ** -8 + 2e-4) * size + 1e-37
+        assert bool(((got - ref).abs() <= bound).all()), float(((got - ref).abs() / bound).max())
+        row += n
