@@ -13,7 +13,7 @@
 //                   sizes.  It reads nothing another kernel writes, so under
 //                   programmatic stream serialisation it starts before the
 //                   kernel ahead of it has finished.
-//   activation warp : the group's 128 k of every token by plain loads into the
+//   activation warp, or two : the group's 128 k of every token by plain loads into the
 //                   stage (swizzled like a TMA tile), and their sum per token
 //                   (the tensor pipe is this kernel's scarce resource, so the sum
 //                   is not done with an all-ones mma).
@@ -45,12 +45,15 @@ constexpr int kOffW0 = 0, kOffW1 = 16384, kOffX0 = 32768;
 // Sixteen consumer warps share an SM's issue slots.  Up to 8 tokens (MT = 1): in two CTAs with three stages each, a warp
 // taking two chunks of 32 columns.  Up to 16 tokens (MT = 2): in one CTA with five stages, a warp taking one chunk
 // (before, eight warps of two chunks, rows paired by byte permutations and, in bf16, masks as immediates:
-// 5120 x 25600 in bf16 30.2 -> 24.3 us at 16 tokens and 23.0 -> 18.1 at 8, in fp16 25.6 -> 23.3 and 17.7 -> 16.0).  More
-// activation warps, or their loads a unit ahead: no change.
+// 5120 x 25600 in bf16 30.2 -> 24.3 us at 16 tokens and 23.0 -> 18.1 at 8, in fp16 25.6 -> 23.3 and 17.7 -> 16.0).
+// Beside so many consumers an activation warp gets few issue slots, and with the norm's arithmetic for 16 tokens the
+// others waited for it: one such linear of a 4096-wide block took 19.6 us.  Two warps with eight tokens each and packed
+// roundings: 13.0 (14.6 with one, 13.4 with four), and 2 to 5 % off the linears without a norm.  For 8 tokens a second
+// warp costs more than it brings (10.9 -> 12.0), as does leaving out the rows beyond M (branches between loads: 9 % at 12 tokens).
 template <int MT> struct StreamCfg {
   static constexpr int kCtasPerSm = MT == 1 ? 2 : 1;
   static constexpr int kChunks = MT == 1 ? 2 : 1, kConsumerWarps = kUnitN / 32 / kChunks;
-  static constexpr int kThreads = (kConsumerWarps + 2) * 32;   // consumers, TMA producer, activation warp
+  static constexpr int kActWarps = MT, kThreads = (kConsumerWarps + 1 + kActWarps) * 32;   // consumers, TMA producer, activation warps
   static constexpr int kStages = MT == 1 ? 3 : 5;
   static constexpr int kXBox = 8 * MT * 128;                 // bytes of one activation box
   static constexpr int kOffX1 = kOffX0 + kXBox;
@@ -135,7 +138,7 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&bar_full[s]), 1); mbar_init(smem_u32(&bar_empty[s]), kConsumerWarps); mbar_init(smem_u32(&bar_xs[s]), 1);
+      mbar_init(smem_u32(&bar_full[s]), 1); mbar_init(smem_u32(&bar_empty[s]), kConsumerWarps); mbar_init(smem_u32(&bar_xs[s]), Cfg::kActWarps);
     }
     mbar_fence_init();
   }
@@ -180,14 +183,15 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       mbar_wait(smem_u32(&bar_full[i % kStages]), (i / kStages) & 1);
     return;
   }
-  if (warp == kConsumerWarps + 1) {
-    // --------------------------------------------------------- activation warp
-    // Brings the group's 128 k of every token from global memory with plain loads (they are small,
+  if (warp > kConsumerWarps) {
+    // -------------------------------------------------------- activation warps
+    // Each brings the group's 128 k of its eight tokens from global memory with plain loads (they are small,
     // L2-resident and must not queue behind the weight boxes), stores them in the layout of a
     // 128-byte-swizzled tile (16-byte chunk c of row m at chunk c ^ (m & 7)), and leaves each
     // token's sum over the group beside them.  Lanes 0-15 hold one token's 256 bytes, lanes 16-31
     // the next token's.
-    const int cc = lane & 15, half = lane >> 4;
+    constexpr int kMine = 4 * MT / Cfg::kActWarps;                 // pairs of tokens that are this warp's: 2 kMine tokens from m0 on
+    const int cc = lane & 15, half = lane >> 4, m0 = 2 * kMine * (warp - kConsumerWarps - 1);
     int grp = (int)(u_begin % G);
     // With the RMSNorm prologue: 1 / rms of token `lane` from the per-tile sums of squares (added
     // in tile order), handed to the lanes that need it by shuffles.
@@ -197,9 +201,9 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       for (int tl = 0; tl < p.norm_tiles; ++tl) tot += __ldcg(p.norm_ssq + (size_t)lane * p.norm_tiles + tl);
       inv_mine = rsqrtf(tot / (float)p.K + p.norm_eps);
     }
-    float inv_tok[4 * MT];
+    float inv_tok[kMine];
 #pragma unroll
-    for (int j = 0; j < 4 * MT; ++j) inv_tok[j] = __shfl_sync(0xFFFFFFFFu, inv_mine, (2 * j + half) & 31);
+    for (int j = 0; j < kMine; ++j) inv_tok[j] = __shfl_sync(0xFFFFFFFFu, inv_mine, (m0 + 2 * j + half) & 31);
     for (int i = 0; i < nunits; ++i) {
       const int s = i % kStages;
       if (i >= kStages && !mbar_wait(smem_u32(&bar_empty[s]), ((i / kStages) - 1) & 1)) {
@@ -207,27 +211,25 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
         break;
       }
       uint8_t* st = const_cast<uint8_t*>(smem_gen) + s * kStageBytes;
-      uint4 v[4 * MT];
+      uint4 v[kMine];
 #pragma unroll
-      for (int j = 0; j < 4 * MT; ++j) {
-        const int m = 2 * j + half;
+      for (int j = 0; j < kMine; ++j) {
+        const int m = m0 + 2 * j + half;
         v[j] = m < p.M ? __ldcg(reinterpret_cast<const uint4*>(p.x + (size_t)m * p.K + grp * kUnitK) + cc) : make_uint4(0u, 0u, 0u, 0u);
       }
       uint4 nw = make_uint4(0u, 0u, 0u, 0u);
       if (NORM) nw = __ldg(reinterpret_cast<const uint4*>(p.norm_weight + grp * kUnitK) + cc);
 #pragma unroll
-      for (int j = 0; j < 4 * MT; ++j) {
-        const int m = 2 * j + half;
+      for (int j = 0; j < kMine; ++j) {
+        const int m = m0 + 2 * j + half;
         if (NORM) {
           // 16-bit(16-bit(h * inv) * w), the roundings of the norm as a kernel of its own
           const uint32_t hw[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, ww[4] = {nw.x, nw.y, nw.z, nw.w};
           uint32_t o[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float a0 = raw16_to_float<BF16>(float_to_raw16<BF16>(raw16_to_float<BF16>((uint16_t)(hw[e] & 0xFFFF)) * inv_tok[j]));
-            const float a1 = raw16_to_float<BF16>(float_to_raw16<BF16>(raw16_to_float<BF16>((uint16_t)(hw[e] >> 16)) * inv_tok[j]));
-            o[e] = (uint32_t)float_to_raw16<BF16>(a0 * raw16_to_float<BF16>((uint16_t)(ww[e] & 0xFFFF))) |
-                   ((uint32_t)float_to_raw16<BF16>(a1 * raw16_to_float<BF16>((uint16_t)(ww[e] >> 16))) << 16);
+          for (int e = 0; e < 4; ++e) {      // (the product of two 16-bit numbers has one rounding either way)
+            const float a0 = raw16_to_float<BF16>((uint16_t)hw[e]) * inv_tok[j], a1 = raw16_to_float<BF16>((uint16_t)(hw[e] >> 16)) * inv_tok[j];
+            o[e] = mul2<BF16>(round2<BF16>(a0, a1), ww[e]);
           }
           v[j] = make_uint4(o[0], o[1], o[2], o[3]);
         }

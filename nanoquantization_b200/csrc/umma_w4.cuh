@@ -43,6 +43,12 @@ template <bool BF16> __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32
   else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
+template <bool BF16> __device__ __forceinline__ uint32_t round2(float lo, float hi) {
+  uint32_t r;
+  if (BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
 __device__ __forceinline__ uint32_t fma2_f16(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t r;
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
@@ -85,10 +91,7 @@ template <bool BF16> __device__ __forceinline__ uint32_t silu_mul2(uint32_t gw, 
   asm("mov.b64 {%0, %1}, %2;" : "=f"(q0), "=f"(q1) : "l"(q));
   asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(p));
   const float s0 = p0 == p0 ? p0 : q0, s1 = p1 == p1 ? p1 : q1;   // (an infinite gate or divisor has no remainder)
-  uint32_t s;
-  if (BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(s) : "f"(s1), "f"(s0));
-  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(s) : "f"(s1), "f"(s0));
-  return mul2<BF16>(s, uw);
+  return mul2<BF16>(round2<BF16>(s0, s1), uw);
 }
 
 // The column of an A block's 128 that lane `l` of tensor memory holds (the order the dequantisers' stores give).
