@@ -99,7 +99,9 @@ class StepBatch:
 
     def to(self, device) -> "StepBatch":
         n, m = self.i64.numel() * 8, self.i32.numel() * 4
-        if torch.device(device).type != "cuda" or self.i64.is_cuda:
+        if torch.device(device).type != "cuda" or self.i64.is_cuda or self.max_len <= 1:
+            # a decode step has few integers, and is moved ahead of a graph's capture, which empties the pinned allocator's
+            # cache: a new block each time (1.2 to 3 ms) against 0.05 ms for two copies from pageable memory
             i64, i32 = self.i64.to(device), self.i32.to(device)
         else:        # both buffers in one copy
             both = _pinned(n + m)
