@@ -60,8 +60,8 @@ __device__ __forceinline__ void umma_commit_pair_both(uint32_t bar, uint16_t mas
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"(mask) : "memory");
 }
-// Arrival on a barrier of a CTA of this cluster that also publishes this thread's writes to shared memory to that CTA, and the
-// wait that takes them over.
+// Arrival on a barrier of a CTA of this cluster that also orders what this warp did to shared memory before it, for that CTA: its
+// writes there, and its reads of that CTA's memory; and the fence behind the wait on it that takes them over.
 __device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -400,7 +400,10 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         // The tile leaves through shared memory: [token][column] in 16 bits, written by one TMA store that clips
         // at M and N.  The accumulator is handed back as soon as it has been read.
         if (ow > 0 && !wait_bar(&bar_ofree, (ow - 1) & 1, s_abort, status)) break;   // the previous store has read the staging area
-        if (SILU && ow > 0 && !wait_bar(&bar_oread, (ow - 1) & 1, s_abort, status)) break;   // and so has the other CTA
+        if (SILU && ow > 0) {
+          if (!wait_bar(&bar_oread, (ow - 1) & 1, s_abort, status)) break;                   // and so has the other CTA:
+          acquire_cluster();                                                                 // its reads come before this tile's writes
+        }
         uint8_t* stage = smem_raw + (smem_base - smem_u32(smem_raw)) + kOffOut + n_local * 2;
         // The accumulator is handed back right after the last read, before the last values are converted:
         // the tensor pipe idles from the tile's last MMA until then.
@@ -456,7 +459,8 @@ umma_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             }
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bar_oread), rank ^ 1u));
+          // (release: plain reads of the other CTA's shared memory are what this reports, and nothing else orders them)
+          if (lane == 0) mbar_arrive_cluster_release(map_to_cta(smem_u32(&bar_oread), rank ^ 1u));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the writes, before the TMA engine reads them
         __syncwarp();

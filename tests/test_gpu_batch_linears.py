@@ -56,6 +56,7 @@ def test_dealings_and_edges(M, K, N, launches, dtype, bias):
 
 @pytest.mark.parametrize("M,K,N", [
     (512, 256, 51200),        # several tiles a cluster: the staging area is handed back and forth
+    (2048, 256, 51200),       # the same twenty times over, with little work between
     (2049, 256, 24576),       # a last tile of one token: one SM has tokens to finish, the other none
     (700, 4096, 24576),       # tokens beyond the input within a tile
     (1000, 1024, 19200),      # the columns of one half end inside what the plain call takes as a tile
