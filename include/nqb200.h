@@ -90,9 +90,11 @@ int nqb200_gemm(const void* x, const void* qweight, const void* qscales, const v
  * nqb200_gemm_gate_up_silu_supported() says 1 (group 128; either M <= 16, N a multiple of twice
  * nqb200_decode_tile_columns() and K long enough that every column tile is split across CTAs, or N a multiple of 256
  * and an M that the two-SM kernel takes in whole tiles); elsewhere it
- * returns NQB200_ERR_BAD_SHAPE and the caller runs nqb200_gemm + nqb200_silu_mul.  Workspace as
- * for nqb200_gemm with the same M, N, K. */
+ * returns NQB200_ERR_BAD_SHAPE and the caller runs nqb200_gemm + nqb200_silu_mul, which gives the same bits and for some
+ * prompts is the faster way: nqb200_gemm_gate_up_silu_faster() says 1 where the one call is supported and not slower.
+ * Workspace as for nqb200_gemm with the same M, N, K. */
 int nqb200_gemm_gate_up_silu_supported(int64_t M, int64_t N, int64_t K, int64_t group_size, int dtype);
+int nqb200_gemm_gate_up_silu_faster(int64_t M, int64_t N, int64_t K, int64_t group_size, int dtype);
 int nqb200_gemm_gate_up_silu(const void* x, const void* qweight, const void* qscales, const void* qzeros,
                              const void* bias, int bias_dtype, void* out, int64_t M, int64_t N, int64_t K,
                              int64_t group_size, int dtype, void* workspace, size_t workspace_bytes, void* stream);

@@ -98,6 +98,11 @@ extern "C" int nqb200_gemm_gate_up_silu_supported(int64_t M, int64_t N, int64_t 
   return umma_prefill_supports(M, N, K, g) ? umma_pair_silu_supports(M, N, K, g) : stream_silu_supported(M, N, K, g);
 }
 
+extern "C" int nqb200_gemm_gate_up_silu_faster(int64_t M, int64_t N, int64_t K, int64_t g, int dtype) {
+  if (!nqb200_gemm_gate_up_silu_supported(M, N, K, g, dtype)) return 0;
+  return !umma_prefill_supports(M, N, K, g) || umma_pair_silu_faster(M, N, K);
+}
+
 extern "C" int nqb200_gemm_gate_up_silu(const void* x, const void* qweight, const void* qscales, const void* qzeros,
                                         const void* bias, int bias_dtype, void* out, int64_t M, int64_t N, int64_t K,
                                         int64_t g, int dtype, void* workspace, size_t workspace_bytes, void* stream) {

@@ -104,6 +104,7 @@ int launch_umma_pair(const GemmArgs& a);
 bool umma_pair_supports(int64_t M, int64_t N, int64_t K, int64_t g);
 size_t umma_pair_workspace_bytes(int64_t M, int64_t N, int64_t K);
 bool umma_pair_silu_supports(int64_t M, int64_t N, int64_t K, int64_t g);
+bool umma_pair_silu_faster(int64_t M, int64_t N, int64_t K);
 int umma_pair_launches(int64_t M, int64_t N, int64_t K);
 bool decode_mma_supports(int64_t M, int64_t N, int64_t K, int64_t g);
 

@@ -681,13 +681,19 @@ bool umma_pair_supports(int64_t M, int64_t N, int64_t K, int64_t g) {
 }
 
 // Gate and up projections merged, silu(gate) * up as the result: tiles of 128 columns of each, whole (so that every sum is the one
-// that the plain call forms).  The activation is left to the epilogue wherever such tiles are dealt, since a launch of its own is
-// never the faster: K x N of 1024 x 6144, 4096 x 24576 and 5120 x 51200 at 200, 777, 1777, 3000 and 8192 tokens, bf16, us for the
-// two launches -> one: 54.2 -> 50.2, 451.6 -> 425.0 and 1236 -> 1242 at 3000, 29.6 -> 29.6, 148.5 -> 144.4 and 499 -> 482 at
-// 777, and the same within 0.2 % at 200, where tiles of few tokens leave through the same steps.
+// that the plain call forms).
 bool umma_pair_silu_supports(int64_t M, int64_t N, int64_t K, int64_t g) {
   return N % (2 * pair::kCols) == 0 && umma_pair_supports(M, N, K, g) && pair::make_plan(M, N, K).quantum != 1;
 }
+
+// Where that is faster than the plain call and a launch for the activation.  Nine layers, K x N, by 200 to 6000 tokens, in turns, bf16,
+// us for two launches -> one: 2048 x 12288 at 3000 tokens 135.5 -> 123.6, 2560 x 19456 246.0 -> 227.4, 4096 x 24576 452.7 -> 439.8,
+// 5120 x 25600 607.1 -> 605.0.  With little work for the tensor pipe behind it the epilogue shows (1 to 3 % lost at 200 and 400 tokens and,
+// in fp16, with K = 1024 at 777 and 1777; even from 777 x 2560 on).  Weights that fill the L2 cache are lost to it: a pair fetches 64
+// bytes of a row here and 64 there, and what comes along with them is gone before its turn (the same with requests of 64
+// bytes: 5120 x 51200 at 777 tokens 360 -> 346, two launches 329).  5120 x 34816, 89 MB: 454.8 -> 474.4 at 1777 tokens; 4096 x 49152, 101 MB:
+// 916.6 -> 974.9 at 3000; 5120 x 51200, 131 MB: 674.3 -> 708.9 at 1777; 66 MB (5120 x 25600) is the largest that gains.
+bool umma_pair_silu_faster(int64_t M, int64_t N, int64_t K) { return M * K >= (1 << 21) && K * N / 2 <= 72000000; }
 
 int umma_pair_launches(int64_t M, int64_t N, int64_t K) { return pair::make_plan(M, N, K).fixup ? 2 : 1; }
 

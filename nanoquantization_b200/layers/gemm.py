@@ -318,14 +318,14 @@ class WQLinear_GEMM(nn.Module):
     @torch.no_grad()
     def forward_silu_mul(self, x: torch.Tensor) -> torch.Tensor:
         """For a merged gate|up projection: ``silu(y[..., :N/2]) * y[..., N/2:]`` with ``y = forward(x)``,
-        bit-identical to running the three steps one after the other.  For decode-sized inputs and for prompts the
-        activation runs inside the kernel that finishes the GEMM; otherwise as a launch of its own."""
+        bit-identical to running the three steps one after the other.  For decode-sized inputs, and for prompts
+        where that is faster, the activation runs inside the kernel that finishes the GEMM; otherwise as a launch of its own."""
         from . import fused
         x2 = x.reshape(-1, x.shape[-1])
         M, K = x2.shape
         lib = _lib.load()
-        if x2.is_cuda and M > 0 and lib.nqb200_gemm_gate_up_silu_supported(M, self.out_features, K, self.group_size,
-                                                                             _lib.dtype_code(self.qscales.dtype)):
+        if x2.is_cuda and M > 0 and lib.nqb200_gemm_gate_up_silu_faster(M, self.out_features, K, self.group_size,
+                                                                          _lib.dtype_code(self.qscales.dtype)):
             out = _w4a16(x2, self.qweight, self.qscales, self.qzeros, self.bias, None, silu_mul=True)
         else:
             out = fused.silu_mul(_w4a16(x2, self.qweight, self.qscales, self.qzeros, self.bias, None))

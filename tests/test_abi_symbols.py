@@ -96,3 +96,19 @@ def test_library_is_not_older_than_its_sources():
     from nanoquantization_b200.csrc import build
     for path in build.LIBRARIES:
         assert not build._stale(path), f"{path} is older than csrc/: rebuild with python -m nanoquantization_b200.csrc.build"
+
+
+def test_where_the_activation_is_left_to_the_linear():
+    """One call for gate, up and activation is taken only where it is supported, and not where two launches are faster."""
+    lib = _lib.load()
+    sup, faster = lib.nqb200_gemm_gate_up_silu_supported, lib.nqb200_gemm_gate_up_silu_faster
+    for code in (0, 1):
+        for M, K, N, want in ((1, 4096, 24576, 1), (16, 5120, 51200, 1), (3000, 4096, 24576, 1), (3000, 5120, 25600, 1),
+                              (1777, 5120, 51200, 0), (1777, 5120, 34816, 0),     # weights that fill the L2 cache
+                              (200, 4096, 24576, 0), (777, 1024, 6144, 0)):       # little work behind the epilogue
+            assert sup(M, N, K, 128, code) == 1
+            assert faster(M, N, K, 128, code) == want
+        for M in (1, 8, 16, 17, 64, 129, 300, 777, 3000):
+            for K in (128, 1000, 1024, 4096):
+                for N in (6400, 6144, 24576, 24584):
+                    assert faster(M, N, K, 128, code) <= sup(M, N, K, 128, code)

@@ -6,6 +6,7 @@ import torch
 import nanoquantization_b200 as nq
 from nanoquantization_b200 import _lib
 from nanoquantization_b200.layers import fused
+from nanoquantization_b200.layers.gemm import _w4a16
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -54,6 +55,10 @@ def test_dealings_and_edges(M, K, N, launches, dtype, bias):
     _lib.check_workspaces()
 
 
+def in_one_call(m, x):
+    return _w4a16(x, m.qweight, m.qscales, m.qzeros, m.bias, None, silu_mul=True)
+
+
 @pytest.mark.parametrize("M,K,N", [
     (512, 256, 51200),        # several tiles a cluster: the staging area is handed back and forth
     (2048, 256, 51200),       # the same twenty times over, with little work between
@@ -77,7 +82,8 @@ def test_gate_up_silu_of_prompts_is_the_separate_steps(M, K, N, dtype, bias):
     x[0] *= 100.0                                                     # gates at both ends of the sigmoid
     want = fused.silu_mul(m(x))
     for _ in range(2):
-        assert torch.equal(m.forward_silu_mul(x), want)               # every rounding is the same
+        assert torch.equal(in_one_call(m, x), want)                   # every rounding is the same
+    assert torch.equal(m.forward_silu_mul(x), want)                   # whichever way it takes
     _lib.check_workspaces()
 
 
@@ -93,5 +99,5 @@ def test_gate_up_silu_of_every_gate(dtype):
     for up in (1.0, -0.7):
         m.bias.copy_(torch.cat([gates, torch.full_like(gates, up)]))
         want = fused.silu_mul(m(x))
-        assert torch.equal(m.forward_silu_mul(x).view(torch.int16), want.view(torch.int16))
+        assert torch.equal(in_one_call(m, x).view(torch.int16), want.view(torch.int16))
     _lib.check_workspaces()
