@@ -75,7 +75,13 @@ size_t nqb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int64_t grou
  * awq_gemm (gemm.py:329-379, M < 256) and awq_dequantize + torch.matmul
  * (gemm.py:560-561, M >= 256), and the bias add gemm.py:565-566.
  * `bias` may be NULL; `bias_dtype` is NQB200_F16 or NQB200_BF16 (the reference
- * module stores its bias in bf16, gemm.py:435-443). */
+ * module stores its bias in bf16, gemm.py:435-443).
+ *
+ * Order: a call comes after everything ahead of it on the stream, with one exception.  Calls that the streaming kernel takes
+ * (nqb200_gemm_kernel_name() "decode_stream": up to 16 tokens; also nqb200_gemm_decode_noalloc and the fused and all-reducing
+ * entries at such sizes) fetch qweight, qscales and qzeros while the kernel ahead may still run.  A kernel that writes these must
+ * not be one that lets its successors start before it has written (griddepcontrol.launch_dependents,
+ * cudaTriggerProgrammaticLaunchCompletion).  nqb200_quantize_pack, copies, and torch's kernels are not of that kind. */
 int nqb200_gemm(const void* x, const void* qweight, const void* qscales, const void* qzeros,
                 const void* bias, int bias_dtype, void* out,
                 int64_t M, int64_t N, int64_t K, int64_t group_size, int dtype,

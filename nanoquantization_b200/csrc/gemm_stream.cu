@@ -157,9 +157,10 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
     int issued = 0, s = 0;
     uint32_t phase = 1;      // parity of the phase in which the stage was last given back
     bool ok = true;
-    // Everything this warp requests (packed weights, scales, zero-points) is read-only, so it
-    // does not wait for the kernel ahead of this one on the stream; the activations come through
-    // the activation warp, which does.
+    // What this warp requests (packed weights, scales, zero-points) is settled before the kernel ahead of this one on the
+    // stream starts its successors, which nqb200.h asks of callers, so it does not wait for that kernel; the activations come
+    // through the activation warps, which do.  (Prefetches into L2 ahead of a wait, which would need no such rule, cost 5 % over 42
+    // calls of up to 16 tokens: 4096 -> 6144, one token, bf16 8.1 -> 9.1 us.)
     for (int i = 0; i < nunits; ++i) {
       if (i >= kStages) {
         ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&bar_empty[s]), phase));
