@@ -364,24 +364,40 @@ stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
       float* slot = p.slots + ((size_t)blockIdx.x * 2 + (tile == first_tile ? 0 : 1)) * kSlotFloats;
 #pragma unroll
       for (int ch = 0; ch < kChunks; ++ch) {
-        const int col = 32 * (kChunks * warp + ch) + 8 * (gq >> 1), n0 = tile * kUnitN + col + odd;
+        const int col = 32 * (kChunks * warp + ch) + 8 * (gq >> 1), n0 = tile * kUnitN + col;
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+        for (int mt = 0; mt < MT; ++mt) {
+          if (whole) {
+            // lanes l and l ^ 4 hold the even and the odd columns of eight, for the same two tokens: each takes one token
+            uint32_t w[2][2];
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const int m = 8 * mt + 2 * tig + t;
-            if (m >= p.M) continue;        // rows beyond M are never read
-            if (!whole) {
-              // a slot holds, of every eight columns, the even ones first
-              __stcg(reinterpret_cast<float4*>(slot + m * kUnitN + col + 4 * odd),
-                     make_float4(total[ch][mt][0][t], total[ch][mt][1][t], total[ch][mt][2][t], total[ch][mt][3][t]));
-            } else if (n0 < p.N) {
+            for (int t = 0; t < 2; ++t)
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                p.out[(size_t)m * p.N + n0 + 2 * j] =
-                    float_to_raw16<BF16>(p.bias ? total[ch][mt][j][t] + bias_to_float(p.bias, p.bias_dtype, n0 + 2 * j) : total[ch][mt][j][t]);
+              for (int k = 0; k < 2; ++k) {
+                float v0 = total[ch][mt][2 * k][t], v1 = total[ch][mt][2 * k + 1][t];
+                if (p.bias && n0 < p.N) { v0 += bias_to_float(p.bias, p.bias_dtype, n0 + 4 * k + odd); v1 += bias_to_float(p.bias, p.bias_dtype, n0 + 4 * k + 2 + odd); }
+                w[t][k] = round2<BF16>(v0, v1);
+              }
+            uint32_t e[2], o[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const uint32_t own = odd ? w[1][k] : w[0][k], got = __shfl_xor_sync(0xFFFFFFFFu, odd ? w[0][k] : w[1][k], 4);
+              e[k] = odd ? got : own; o[k] = odd ? own : got;
+            }
+            const int m = 8 * mt + 2 * tig + odd;
+            if (m < p.M && n0 < p.N)
+              *reinterpret_cast<uint4*>(p.out + (size_t)m * p.N + n0) =
+                  make_uint4(__byte_perm(e[0], o[0], 0x5410), __byte_perm(e[0], o[0], 0x7632), __byte_perm(e[1], o[1], 0x5410), __byte_perm(e[1], o[1], 0x7632));
+          } else {
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              const int m = 8 * mt + 2 * tig + t;
+              if (m < p.M)                 // rows beyond M are never read; a slot holds, of every eight columns, the even ones first
+                __stcg(reinterpret_cast<float4*>(slot + m * kUnitN + col + 4 * odd),
+                       make_float4(total[ch][mt][0][t], total[ch][mt][1][t], total[ch][mt][2][t], total[ch][mt][3][t]));
             }
           }
+        }
       }
 #pragma unroll
       for (int q = 0; q < kChunks * MT * 8; ++q) (&total[0][0][0][0])[q] = 0.f;

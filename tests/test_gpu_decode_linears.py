@@ -1,8 +1,10 @@
 """The linears and recurrent states of decode steps on both sides of the sizes at which their kernels change how much a thread has
-under way, against float64."""
+under way, or who writes the output, against float64."""
 import pytest
 import torch
 
+import nanoquantization_b200 as nq
+from nanoquantization_b200 import _lib
 from nanoquantization_b200.engine.batch import StepBatch
 from nanoquantization_b200.layers import mixers as ops
 from nanoquantization_b200.layers.sequence_mixers import RetentionMixer
@@ -78,3 +80,34 @@ def test_retention_step(batch, heads, dim, vdim, rot):
     # a float product and sum (angles of 11 radians are good to 7e-7); one rounding to bfloat16
     _close(state, S, 2e-6)
     _close(act[:, 8:], want.flatten(1), 2.0 ** -8)
+
+
+@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("K,N", [(128, 32), (128, 544), (128, 51200), (256, 96256), (256, 102400)])
+@pytest.mark.parametrize("dtype,bias", [(torch.float16, True), (torch.bfloat16, False)])
+@torch.no_grad()
+def test_packed_linears_whose_tiles_are_whole(M, K, N, dtype, bias):
+    """A block that has a tile's whole K writes the output itself: tiles of 512 columns, the last ones of 32, 64 and 512; one tile a block
+    and several."""
+    lib, code = _lib.load(), 0 if dtype == torch.float16 else 1
+    assert lib.nqb200_gemm_kernel_name(M, N, K, 128, code) == b"decode_stream"
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    m = nq.WQLinear_GEMM(4, 128, K, N, DEV, bias, dtype)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, device=DEV, dtype=torch.int64).to(torch.int32)  # noqa: E731
+    m.qweight.copy_(words(K, N // 8)); m.qzeros.copy_(words(K // 128, N // 8))
+    m.qscales.copy_((torch.rand(K // 128, N, generator=g, device=DEV) * 9e-3 + 1e-3).to(dtype))
+    if bias:
+        m.bias.copy_(torch.randn(N, generator=g, device=DEV))
+    x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
+    buf = torch.full((M + 2, N), -7.25, dtype=dtype, device=DEV)      # sentinel rows: a store past the tokens would change them
+    m(x, out=buf[1:M + 1])
+    torch.cuda.synchronize()
+    assert bool((buf[0] == -7.25).all()) and bool((buf[M + 1] == -7.25).all())
+    q, z = nq.unpack_int4(m.qweight).double(), nq.unpack_int4(m.qzeros).double()
+    W = (q - z.repeat_interleave(128, 0)) * m.qscales.double().repeat_interleave(128, 0)
+    ref = x.double() @ W + (m.bias.double() if bias else 0.0)
+    # half a unit of the result's last place, and float32 sums of K products of x with q and with the zero-point (and 128 in bfloat16)
+    size = x.double().abs() @ ((q + z.repeat_interleave(128, 0) + 256.0) * m.qscales.double().repeat_interleave(128, 0))
+    bound = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) * ref.abs() + K * 2.0 ** -24 * size + 2.0 ** -24
+    assert bool(((buf[1:M + 1].double() - ref).abs() <= bound).all())
+    _lib.check_workspaces()
