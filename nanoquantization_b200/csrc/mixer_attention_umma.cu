@@ -12,8 +12,8 @@
 // exponentials 2048, and about 4200 pass, because the chains meet at the pipes.  8192 tokens of 32 heads, chunks of 4096, and in one chunk:
 // 545 -> 352 us and 929 -> 586; sigmoid weights in one chunk 883 -> 596 (before: whole tiles, one softmax thread per row, one
 // polling issuer).  The steps on the way, one chunk: rows halved among twice the warps 866, an issuer per query tile 824,
-// S and P by halves 621, the short series 578, its coefficients in terms of s 567, sums of the rounded weights 576, a row's own
-// reference 586 (these two for the error, see below).  An own
+// S and P by halves 621, the short series 578, its coefficients in terms of s 567, a row's own
+// reference 577 (for the error, see below).  An own
 // warp for S beside the two for O (592), polling instead of suspended softmax waits (579) and query tiles started apart (with whole
 // tiles, 849 against 824) gained nothing.
 //
@@ -28,6 +28,8 @@
 // up to a tenth of the cap, where what they leave out (0.054 y^6) is below float's rounding, five terms beyond; up to
 // twice the cap it is the seventh convergent of Lambert's continued fraction (one reciprocal more per score); a warp
 // whose half tile has a larger score, or needs a mask, takes the general path.
+//
+// The sum that a row is divided by takes the weights in float32, before the product's rounding to bf16.
 //
 // Sigmoid weights (nqb200_attention.sigmoid) need no maximum and no sum: a weight is 1 / (1 + 2^x), two weights share one
 // reciprocal, 1 / a = b / (a b), with x clamped to 60 so that a b stays finite (weights below 2^-60 are 2^-60).
@@ -146,15 +148,6 @@ __device__ __forceinline__ float ex2(float x) { float r; asm("ex2.approx.ftz.f32
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-// The sum that a row's result is divided by takes the weights as the product does, rounded to bf16: where one stands out its
-// rounding cancels.  Against sums of the unrounded ones the error to float64 is 1 to 8 % smaller in the mean, for every
-// kind of scores that the tests have.
-__device__ __forceinline__ uint64_t add_rounded(uint64_t sum, uint32_t w) {
-  float a, b; unpair2(sum, a, b);
-  asm("{\n .reg .b16 lo, hi;\n mov.b32 {lo, hi}, %2;\n add.f32.bf16 %0, lo, %0;\n add.f32.bf16 %1, hi, %1;\n}" : "+f"(a), "+f"(b) : "r"(w));
-  return pair2(a, b);
 }
 
 template <int D, int V>
@@ -360,7 +353,7 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           x0 = ex2(x0);
           x1 = ex2(x1);
           w[e] = pack_bf16(x0, x1);
-          ls[e & 1] = add_rounded(ls[e & 1], w[e]);
+          ls[e & 1] = add2(ls[e & 1], pair2(x0, x1));
         }
         tmem_st16(tS + c * 16, w);
       }
@@ -504,7 +497,7 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             x0 = ex2(x0);
             x1 = ex2(x1);
             w[e] = pack_bf16(x0, x1);
-            ls[e & 1] = add_rounded(ls[e & 1], w[e]);
+            ls[e & 1] = add2(ls[e & 1], pair2(x0, x1));
           }
           tmem_st16(tS + c * 16, w);
         }
@@ -529,7 +522,7 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               x[u] = (key <= pos && key >= lo) ? ex2(score(__uint_as_float(v[2 * e + u])) - mu) : 0.f;
             }
             w[e] = pack_bf16(x[0], x[1]);
-            lsum = add_rounded(lsum, w[e]);
+            lsum = add2(lsum, pair2(x[0], x[1]));
           }
           tmem_st8(tS + c * 8, w);      // lies behind what has been read of S
         }

@@ -62,3 +62,33 @@ def test_scores_of_every_range(D, V, chunk, softcap, spread, sink):
         bound = 2.0 ** -8 * ref.abs() + (2.0 ** -8 + 2e-4) * size + 1e-37
         assert bool(((got - ref).abs() <= bound).all()), float(((got - ref).abs() / bound).max())
         row += n
+
+
+@pytest.mark.parametrize("softcap,low", [(0.0, None), (50.0, None), (50.0, -10.0), (50.0, -60.0), (50.0, -150.0), (120.0, None)])
+def test_the_sum_takes_unrounded_weights(softcap, low):
+    """Every path a score can take.  One key has weight 1 and is the only one with a value; the others weigh half of 1 + 2^-8 + 2^-12, which bf16
+    rounds up by nearly 2^-8.  With the exact result at 1 a sum of rounded weights is 2^-8 too large, the next bf16 number below."""
+    D, T = 64, 256
+    weight = 0.5 * (1 + 2.0 ** -8 + 2.0 ** -12)
+    raw = torch.full((T,), math.log(weight), dtype=torch.float64)
+    if softcap:
+        raw = softcap * torch.atanh(raw / softcap)
+    raw[0] = 0.0
+    if low is not None:
+        raw[[1, 65, 129]] = low           # decides the path of the halves of tiles that the last rows see whole
+    k = torch.zeros(T, G, D, dtype=torch.float64)
+    for c in range(3):                    # scores exact to 2^-24: three bf16 numbers each
+        k[:, :, c] = (raw - k[:, 0].sum(-1)).to(torch.bfloat16).double()[:, None]
+    s = k[:, 0].sum(-1)
+    s = softcap * torch.tanh(s / softcap) if softcap else s
+    p = s.exp()
+    kc, vc = torch.zeros(3, BS, G, D, dtype=torch.bfloat16, device=DEV), torch.zeros(3, BS, G, D, dtype=torch.bfloat16, device=DEV)
+    kc[1:] = k.to(torch.bfloat16).view(2, BS, G, D).to(DEV)
+    vc[1, 0] = 1.0
+    step = StepBatch.host([[0] * T], [0], [[1, 2]], [0], 2, BS).to(DEV)
+    q = torch.zeros(T, H, D, dtype=torch.bfloat16, device=DEV)
+    q[:, :, :3] = 1.0
+    out = torch.empty(T, H * D, dtype=torch.bfloat16, device=DEV)
+    desc = _lib.AttentionDesc(heads=H, kv_heads=G, dim=D, vdim=D, chunk=0, scale=1.0, softcap=softcap, sink=None, out_scale=float(p.sum()))
+    ops.chunk_attention(q.view(T, H * D), kc, vc, out, desc, step)
+    assert bool((out[-1].float() == 1.0).all()), out[-1].float().unique()
