@@ -9,21 +9,21 @@
 // Tensor memory holds S of both tiles (two halves of 64 columns each) and O of both; P overwrites the first half of its own S.
 // So four chains S -> weights -> O += P V -> next S run beside each other, and a scheduler has a warp of each.  What bounds it:
 // per 256 x 128 scores the tensor pipe needs 2560 cycles (S 48 per MMA of N = 64, which shared memory sets, O 64), the
-// exponentials 2048, and about 4200 pass, because the chains meet at the pipes.  8192 tokens of 32 heads, chunks of 4096, and in one chunk:
-// 545 -> 352 us and 929 -> 586; sigmoid weights in one chunk 883 -> 596 (before: whole tiles, one softmax thread per row, one
-// polling issuer).  The steps on the way, one chunk: rows halved among twice the warps 866, an issuer per query tile 824,
-// S and P by halves 621, the short series 578, its coefficients in terms of s 567, a row's own
-// reference 577 (for the error, see below).  An own
-// warp for S beside the two for O (592), polling instead of suspended softmax waits (579) and query tiles started apart (with whole
-// tiles, 849 against 824) gained nothing.
+// exponentials 2048, and about 4600 pass, because the chains meet at the pipes.  8192 tokens of 32 heads of 128, us, in turns against
+// whole tiles with one softmax thread per row and one polling issuer: chunks of 4096 626 -> 406, one chunk 1087 -> 679, scores beyond
+// the cap 2667 -> 1678, no cap 931 -> 611, sigmoid weights 959 -> 624.  An own warp for S beside the two for O, polling instead of
+// suspended softmax waits and query tiles started apart gained nothing.
 //
-// The weights are 2^(score - m).  A cap bounds the scores, and up to kBound in log2 units m is the maximum of the
-// first tile with a key of the row's chunk (the row's two threads exchange theirs), or the sink, or kSpan below the cap, whichever is the largest: no weight is above 2^kSpan
-// and those that vanish are below 2^-126 of one that is there.  (A fixed m, the same for all rows, is 1 % faster and has
-// up to 25 % more error in the mean: the largest weight of a short row should be a power of two, so that its rounding to bf16
-// costs nothing.)  Without a cap, or with a wider one, m follows the running maximum when it falls behind by more than 8 in
-// log2 units, and O is rescaled: the weights stay below 2^8, and after a row's first tiles it hardly ever happens.  The cap
-// is monotonic, so the maximum is taken over raw scores.
+// The weights are 2^(score - m).  m is the largest score of the tile that a row begins in, or the sink, and follows the largest score
+// when it falls behind by more than kLag in log2 units; O and the sums are then rescaled: no weight is above 2^kLag, whatever the
+// scores do, and after a row's first tiles it hardly ever happens.  (With 7 the error to float64 is for every kind of scores measured at most
+// what whole tiles with a lag of 8 had; smaller lags take off up to 5 % more of it and cost 2 to 3 % each where scores spread by 6 log2 units.)
+// A half finds out by itself that its scores ask for no move, from the largest magnitude, which the choice below needs as well; that
+// the other half has not moved it learns from what that one hands on, in the order of the products, and does not wait for the other's
+// scores: 940 -> 679 us with a cap of 120, against halves that compare their maxima in every tile.  Of the 679 the hand-over takes 65.
+// (A reference that never moves, which a cap of 50 allows, needs neither, but its weights reach 2^100 and more values overflow, and the
+// largest weight of a row is rounded where it could be a power of two: up to 11 % more error.)  The cap is monotonic, so the
+// maximum is taken over raw scores.
 // For scores well inside the cap tanh is its Taylor series, which costs fused multiply-adds on register pairs only: three terms
 // up to a tenth of the cap, where what they leave out (0.054 y^6) is below float's rounding, five terms beyond; up to
 // twice the cap it is the seventh convergent of Lambert's continued fraction (one reciprocal more per score); a warp
@@ -46,15 +46,18 @@ namespace att {
 
 constexpr int kTile = 128, kThreads = 640;
 constexpr uint32_t kColS = 0, kColO = 256, kTmemCols = 512;
-constexpr float kLog2e = 1.4426950408889634f, kLag = 8.f, kSeriesRange = 0.4f, kShortRange = 0.1f, kFractionRange = 2.f, kBound = 80.f, kSpan = 100.f;
+constexpr float kLog2e = 1.4426950408889634f, kLag = 7.f, kSeriesRange = 0.4f, kShortRange = 0.1f, kFractionRange = 2.f;
 
 struct Params {
   nqb200_batch bt;
   bf16* out; int64_t out_stride;
   int heads, kv_heads, chunk;
   float scale, softcap, out_scale;
+  // a raw score s in log2 units: top tanh(ysc s), or s ysc_top without a cap; and tanh's series in s, with the powers of ysc and top in them
+  float ysc, top, ysc_top, c3, c5, c7, c9;
+  int folded;          // none of the coefficients leaves the range of normal numbers
   const float* sink;
-  int sigmoid; const float* temp; const float* bias;
+  const float* temp; const float* bias;      // of sigmoid weights
   int* status;
 };
 
@@ -133,6 +136,14 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
                  "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
+               "%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+                 "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+                 "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
 // pairs of floats in one 64-bit register
 __device__ __forceinline__ uint64_t pair2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ void unpair2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
@@ -142,7 +153,6 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r;
 }
 __device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
-__device__ __forceinline__ float min3(float a, float b, float c) { float r; asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 __device__ __forceinline__ float max3_abs(float a, float b, float c) { float r; asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 __device__ __forceinline__ float ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -150,15 +160,15 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <int D, int V>
+template <int D, int V, bool SIGMOID>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const Params p) {
   constexpr uint32_t kQBytes = kTile * D * 2, kKBytes = kTile * D * 2, kVBytes = kTile * V * 2, kBox = kTile * 128;
   constexpr uint32_t kOffK = 2 * kQBytes, kOffV = kOffK + 2 * kKBytes;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_q, bar_kfull[2], bar_kfree[2], bar_vfull[2], bar_vfree[2], bar_s[2][2], bar_p[2][2], bar_pv[2][2], bar_o[2], bar_x[2][4], bar_drain;
-  __shared__ float s_x[2][2][2][kTile];
+  __shared__ __align__(8) uint64_t bar_q, bar_kfull[2], bar_kfree[2], bar_vfull[2], bar_vfree[2], bar_s[2][2], bar_p[2][2], bar_pv[2][2], bar_o[2], bar_x[2][4], bar_m[2][2][4], bar_drain;
+  __shared__ float s_x[2][2][2][kTile], s_m[2][2][kTile];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort_i;
   volatile int* s_abort = &s_abort_i;
@@ -186,7 +196,10 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       mbar_init(smem_u32(&bar_s[s][0]), 1); mbar_init(smem_u32(&bar_s[s][1]), 1); mbar_init(smem_u32(&bar_p[s][0]), 4); mbar_init(smem_u32(&bar_p[s][1]), 4);
       mbar_init(smem_u32(&bar_pv[s][0]), 1); mbar_init(smem_u32(&bar_pv[s][1]), 1); mbar_init(smem_u32(&bar_o[s]), 1);
     }
-    for (int s = 0; s < 8; ++s) mbar_init(smem_u32(&bar_x[s >> 2][s & 3]), 2);
+    for (int s = 0; s < 8; ++s) {
+      mbar_init(smem_u32(&bar_x[s >> 2][s & 3]), 2);
+      mbar_init(smem_u32(&bar_m[s >> 2][0][s & 3]), 32); mbar_init(smem_u32(&bar_m[s >> 2][1][s & 3]), 32);
+    }
     mbar_init(smem_u32(&bar_drain), 2);
     s_abort_i = 0;
     mbar_fence_init();
@@ -197,8 +210,8 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_after();
   const uint32_t tmem = s_tmem;
 
-  // of the 96 registers a thread that 640 threads can have: 56 x 128 + 104 x 512 <= 96 x 640
-  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+  // of the 96 registers a thread that 640 threads can have: 32 x 128 + 112 x 512 = 96 x 640
+  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;"); else asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA
     const bool el = elect_one();
@@ -298,11 +311,10 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t lanes = (uint32_t)(32 * quarter) << 16, tS = tmem + lanes + kColS + q * 128 + half * 64, tO = tmem + lanes + kColO + q * 128;
     const int i = i0 + q * kTile + row, pos = pos0 + i, wfirst = pos - lane, wlast = wfirst + 31;
     const int lo = p.chunk > 0 ? pos / p.chunk * p.chunk : 0, lo_last = p.chunk > 0 ? wlast / p.chunk * p.chunk : 0;
-    const bool capped = p.softcap > 0.f, bounded = capped && p.softcap * kLog2e <= kBound;
-    const float ysc = capped ? p.scale / p.softcap : p.scale, top = capped ? p.softcap * kLog2e : kLog2e;
+    const bool capped = p.softcap > 0.f;
     auto score = [&](float s) {   // in log2 units
-      const float y = s * ysc;
-      return top * (capped ? tanh_fast(y) : y);
+      const float y = s * p.ysc;
+      return p.top * (capped ? tanh_fast(y) : y);
     };
     auto done = [&]() {           // this half of the weights is in tensor memory
       tc_wait_st();
@@ -325,16 +337,34 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     };
     const float sg_scale = -p.scale * (p.temp ? p.temp[h] : 1.f) * kLog2e, sg_shift = p.bias ? -p.bias[h] * kLog2e : 0.f;
     const float sink = p.sink ? p.sink[h] * kLog2e : -INFINITY;
-    const float floor = bounded ? top - kSpan : -INFINITY;
-    float m = p.sink ? fmaxf(sink, floor) : sink, l = 0.f;
+    float m = sink;
     uint64_t lsum = pair2(0.f, 0.f);
-    // top tanh(y) by its series, TERMS powers of y^2 beyond the first (0: no cap).  The coefficients carry the powers of y / s.
-    const bool folded = ysc >= 1.f / 4096.f && ysc <= 4096.f;      // and none of them leaves the range of normal numbers
+    // A row's reference goes from half to half in the order of their products: 0 and 1 of the first tile, 0 and 1 of the next, and so on,
+    // except in the tiles where rows begin (the first, and the one of the last row's chunk), where both agree on it.
+    const int second = (lo_last - kstart) / kTile;
+    auto pass = [&](float mine) {    // (every lane arrives: a branch for one of them cost 2 % of the kernel)
+      s_m[q][half][row] = mine;
+      mbar_arrive(smem_u32(&bar_m[q][half][quarter]));
+    };
+    auto take = [&](int n) {       // what the other half passed on, its n-th
+      if (!wait_bar_warp(&bar_m[q][half ^ 1][quarter], (n - 1) & 1, s_abort, p.status)) return false;
+      const float got = s_m[q][half ^ 1][row];
+      if (__any_sync(0xFFFFFFFFu, got != m)) {
+        const float f = got != m ? ex2(m - got) : 1.f;
+        lsum = mul2(lsum, pair2(f, f));
+        m = got;
+      }
+      return true;
+    };
+    auto catch_up = [&](int j, bool joint) {      // with what came before this half of tile j
+      const int n = j - 1 - (second > 0 && j > second ? 1 : 0);      // tiles before it in which it was passed on
+      if (half == 1) return joint || take(n + 1);
+      return j == 0 || j == 1 || j - 1 == second || take(n);
+    };
+    // top tanh(y) by its series, TERMS powers of y^2 beyond the first (0: no cap)
     auto weights = [&](auto terms, const uint32_t (&r)[2][32], uint64_t nm2) {
       constexpr int TERMS = decltype(terms)::value;
-      const float z = ysc * ysc, c1 = top * ysc, c3 = -c1 / 3.f * z, c5 = c1 * (2.f / 15.f) * z * z, c7 = -c1 * (17.f / 315.f) * z * z * z,
-                  c9 = c1 * (62.f / 2835.f) * z * z * z * z;
-      const uint64_t k1 = pair2(c1, c1), k3 = pair2(c3, c3), k5 = pair2(c5, c5), k7 = pair2(c7, c7), k9 = pair2(c9, c9);
+      const uint64_t k1 = pair2(p.ysc_top, p.ysc_top), k3 = pair2(p.c3, p.c3), k5 = pair2(p.c5, p.c5), k7 = pair2(p.c7, p.c7), k9 = pair2(p.c9, p.c9);
       uint64_t ls[2] = {lsum, 0};
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -361,7 +391,9 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     };
     bool ok = true;
     for (int j = 0; j < nq[q]; ++j) {
-      ok = wait_bar_warp(&bar_s[q][half], j & 1, s_abort, p.status);
+      // where rows of this warp begin both halves agree on a reference, the largest score of the two
+      const bool joint = j == 0 || j == second;
+      ok = (SIGMOID || catch_up(j, joint)) && wait_bar_warp(&bar_s[q][half], j & 1, s_abort, p.status);
       if (!ok) break;
       tc_fence_after();
       const int key0 = kstart + j * kTile + half * 64;
@@ -370,7 +402,7 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
       for (int c = 0; c < 2; ++c) tmem_ld32(tS + c * 32, r[c]);
       tc_wait_ld();
-      if (p.sigmoid) {
+      if constexpr (SIGMOID) {
         const uint64_t sg_scale2 = pair2(sg_scale, sg_scale), sg_shift2 = pair2(sg_shift, sg_shift), one2 = pair2(1.f, 1.f);
         auto sigmoid2 = [&](uint32_t s0, uint32_t s1, float& w0, float& w1) {
           float x0, x1;
@@ -412,74 +444,75 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         done();
         continue;
       }
-      float ab = 0.f;
-      if (bounded && j > 0 && !__any_sync(0xFFFFFFFFu, m == -INFINITY)) {
+      float ab = 0.f, mx = -INFINITY;     // the largest magnitude and, where it is asked for, the largest score
+      if (!masked) {
+        float hi[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) hi[(e >> 1) & 3] = max3_abs(hi[(e >> 1) & 3], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+        ab = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
+      }
+      const float lag = m + kLag;
+      // (|score| <= |y top|: at most this, so that most tiles need neither the cap nor the sign)
+      if (joint || masked || !__all_sync(0xFFFFFFFFu, ab * p.ysc_top <= lag)) {
         if (!masked) {
-          float hi[4] = {0.f, 0.f, 0.f, 0.f};
+          float hi[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
           for (int c = 0; c < 2; ++c)
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) hi[(e >> 1) & 3] = max3_abs(hi[(e >> 1) & 3], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-          ab = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
-        }
-      } else {
-        float mx = -INFINITY;
-        if (!masked) {
-          float hi[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, lw[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-              const int k = (e >> 1) & 3;
-              hi[k] = max3(hi[k], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-              lw[k] = min3(lw[k], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-            }
+            for (int e = 0; e < 32; e += 2) hi[(e >> 1) & 3] = max3(hi[(e >> 1) & 3], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
           mx = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
-          ab = fmaxf(mx, -fminf(fminf(lw[0], lw[1]), fminf(lw[2], lw[3])));
         } else {
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const int key = key0 + c * 32 + e;
-              mx = (key <= pos && key >= lo) ? fmaxf(mx, __uint_as_float(r[c][e])) : mx;
-            }
-        }
-        float mo;
-        if (!(ok = exchange(mx, mo))) break;
-        mx = fmaxf(mx, mo);
-        const float mt = mx == -INFINITY ? mx : fmaxf(score(mx), floor), mn = fmaxf(m, mt);
-        if (j == 0) {
-          l = p.sink && half == 0 ? ex2(sink - mn) : 0.f;
-          m = mn;
-        } else {
-          const bool move = mn > m + kLag;      // also from -inf
-          if (__any_sync(0xFFFFFFFFu, move)) {
-            const float f = move ? ex2(m - mn) : 1.f;
-            m = move ? mn : m;
-            l *= f;
-            float a, c2;
-            unpair2(lsum, a, c2);
-            lsum = pair2(a * f, c2 * f);
-            if (half == 0) {      // before its weights are reported, which both products of the tile wait for
 #pragma unroll 1
-              for (int c = 0; c < V / 8; ++c) {   // rare: small pieces, few registers
-                uint32_t o[8];
-                tmem_ld_32x32b_x8(tO + c * 8, o);
-                tc_wait_ld();
+          for (int c = 0; c < 4; ++c) {
+            uint32_t v[16];
+            tmem_ld_32x32b_x16(tS + c * 16, v);
+            tc_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-                tmem_st8(tO + c * 8, o);
-              }
-              tc_wait_st();
+            for (int e = 0; e < 16; ++e) {
+              const int key = key0 + c * 16 + e;
+              mx = (key <= pos && key >= lo) ? fmaxf(mx, __uint_as_float(v[e])) : mx;
             }
           }
         }
+        if (joint) {
+          float mo;
+          if (!(ok = exchange(mx, mo))) break;
+          mx = fmaxf(mx, mo);
+        }
+        mx = mx == -INFINITY ? mx : score(mx);
+      }
+      const bool move = mx > lag;      // also from -inf
+      if (!joint) pass(move ? mx : m);
+      if (j == 0) {
+        m = fmaxf(m, mx);
+        lsum = pair2(p.sink && half == 0 ? ex2(sink - m) : 0.f, 0.f);
+      } else if (__any_sync(0xFFFFFFFFu, move)) {
+        const float f = move ? ex2(m - mx) : 1.f;
+        lsum = mul2(lsum, pair2(f, f));
+        m = move ? mx : m;
+        if (half == 0 || !joint) {
+          // O has the products of all halves before this one, and no other until this one's weights are reported
+          if (!(ok = wait_bar_warp(&bar_pv[q][half ^ 1], (j - 1 + half) & 1, s_abort, p.status))) break;
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < V / 32; ++c) {
+            tmem_ld32(tO + c * 32, r[0]);
+            tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r[0][e] = __float_as_uint(__uint_as_float(r[0][e]) * f);
+            tmem_st32(tO + c * 32, r[0]);
+          }
+          tc_wait_st();
+          tmem_ld32(tS, r[0]);      // the scores again
+          tc_wait_ld();
+        }
       }
       const float mu = m == -INFINITY ? 0.f : m;
-      const uint64_t ysc2 = pair2(ysc, ysc), nm2 = pair2(-mu, -mu), k1 = pair2(top, top);
-      auto within = [&](float y) { return __all_sync(0xFFFFFFFFu, ab * ysc <= y); };      // for every score of the warp's
-      const int range = masked ? 2 : !capped || (folded && within(kSeriesRange)) ? 0 : within(kFractionRange) ? 1 : 2;
+      const uint64_t ysc2 = pair2(p.ysc, p.ysc), nm2 = pair2(-mu, -mu), k1 = pair2(p.top, p.top);
+      auto within = [&](float y) { return __all_sync(0xFFFFFFFFu, ab * p.ysc <= y); };      // for every score of the warp's
+      const int range = masked ? 2 : !capped || (p.folded && within(kSeriesRange)) ? 0 : within(kFractionRange) ? 1 : 2;
       if (range == 1) {
         // tanh y = y (10395 + 1260 y^2 + 21 y^4) / (10395 + 4725 y^2 + 210 y^4 + y^6)
         const uint64_t n0 = pair2(10395.f, 10395.f), n1 = pair2(1260.f, 1260.f), n2 = pair2(21.f, 21.f), d1 = pair2(4725.f, 4725.f), d2 = pair2(210.f, 210.f);
@@ -530,12 +563,12 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       done();
     }
     if (ok && nq[q] > 0) {
-      ok = wait_bar_warp(&bar_o[q], 0, s_abort, p.status);
+      ok = (SIGMOID || catch_up(nq[q], true)) && wait_bar_warp(&bar_o[q], 0, s_abort, p.status);
       float f = p.out_scale;
-      if (ok && !p.sigmoid) {
+      if (ok && !SIGMOID) {
         float a, c2, other;
         unpair2(lsum, a, c2);
-        l += a + c2;
+        const float l = a + c2;
         ok = exchange(l, other);
         f /= l + other;
       }
@@ -579,16 +612,20 @@ static bool encode_rows(CUtensorMap* m, const void* base, uint64_t rows, uint64_
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int D, int V>
-static int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Params& p, cudaStream_t st) {
+template <int D, int V, bool SIGMOID>
+static int launch_t(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Params& p, cudaStream_t st) {
   // at least 120 KB, whatever the sizes: one CTA per SM, because a CTA takes all of the SM's tensor memory
   const size_t need = (size_t)kTile * (2 * D + 2 * D + 2 * V) * 2 + 1024, smem = need > 120 * 1024 ? need : 120 * 1024;
-  if (cudaFuncSetAttribute(attention_umma_kernel<D, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  if (cudaFuncSetAttribute(attention_umma_kernel<D, V, SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     return NQB200_ERR_LAUNCH;
   }
   const dim3 grid((unsigned)((p.bt.max_len + 2 * kTile - 1) / (2 * kTile)), (unsigned)p.heads, (unsigned)p.bt.batch);
-  return launch_overlapped(attention_umma_kernel<D, V>, grid, dim3(kThreads), smem, st, q, k, v, p);
+  return launch_overlapped(attention_umma_kernel<D, V, SIGMOID>, grid, dim3(kThreads), smem, st, q, k, v, p);
+}
+template <int D, int V>
+static int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Params& p, bool sigmoid, cudaStream_t st) {
+  return sigmoid ? launch_t<D, V, true>(q, k, v, p, st) : launch_t<D, V, false>(q, k, v, p, st);
 }
 
 }  // namespace att
@@ -609,10 +646,17 @@ int attention_umma(const void* q, int64_t q_stride, const void* k_cache, const v
     return NQB200_ERR_LAUNCH;
   att::Params p = {};
   p.bt = *b; p.out = (bf16*)out; p.out_stride = out_stride; p.heads = a->heads; p.kv_heads = a->kv_heads; p.chunk = a->chunk;
-  p.scale = a->scale; p.softcap = a->softcap; p.out_scale = a->out_scale; p.sink = a->sink; p.sigmoid = a->sigmoid; p.temp = a->temp; p.bias = a->bias;
+  p.scale = a->scale; p.softcap = a->softcap; p.out_scale = a->out_scale; p.sink = a->sink; p.temp = a->temp; p.bias = a->bias;
   p.status = status;
-  if (a->dim == 64) return a->vdim == 64 ? att::launch<64, 64>(tq, tk, tv, p, st) : att::launch<64, 128>(tq, tk, tv, p, st);
-  return a->vdim == 64 ? att::launch<128, 64>(tq, tk, tv, p, st) : att::launch<128, 128>(tq, tk, tv, p, st);
+  p.ysc = p.softcap > 0.f ? p.scale / p.softcap : p.scale;
+  p.top = p.softcap > 0.f ? p.softcap * att::kLog2e : att::kLog2e;
+  p.ysc_top = p.top * p.ysc;
+  const float z = p.ysc * p.ysc;
+  p.c3 = -p.ysc_top / 3.f * z; p.c5 = p.ysc_top * (2.f / 15.f) * z * z; p.c7 = -p.ysc_top * (17.f / 315.f) * z * z * z;
+  p.c9 = p.ysc_top * (62.f / 2835.f) * z * z * z * z;
+  p.folded = p.ysc >= 1.f / 4096.f && p.ysc <= 4096.f;
+  if (a->dim == 64) return a->vdim == 64 ? att::launch<64, 64>(tq, tk, tv, p, a->sigmoid, st) : att::launch<64, 128>(tq, tk, tv, p, a->sigmoid, st);
+  return a->vdim == 64 ? att::launch<128, 64>(tq, tk, tv, p, a->sigmoid, st) : att::launch<128, 128>(tq, tk, tv, p, a->sigmoid, st);
 }
 
 }  // namespace nqb200

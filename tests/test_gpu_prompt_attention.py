@@ -92,3 +92,51 @@ def test_the_sum_takes_unrounded_weights(softcap, low):
     desc = _lib.AttentionDesc(heads=H, kv_heads=G, dim=D, vdim=D, chunk=0, scale=1.0, softcap=softcap, sink=None, out_scale=float(p.sum()))
     ops.chunk_attention(q.view(T, H * D), kc, vc, out, desc, step)
     assert bool((out[-1].float() == 1.0).all()), out[-1].float().unique()
+
+
+@pytest.mark.parametrize("chunk", [0, 639])         # 639: the second chunk has a single key in its first tile
+@pytest.mark.parametrize("softcap,sink,kind", [
+    (50.0, None, "jump"),         # a first tile near minus the cap, later keys near the cap
+    (50.0, -45.0, "jump"),
+    (50.0, 20.0, "jump"),
+    (0.0, None, "jump"),
+    (0.0, None, "stairs"),        # every half tile above the one before, for some rows; below, for others
+    (120.0, -100.0, "stairs"),
+    (50.0, None, "stairs"),
+])
+def test_references_that_move_far(softcap, sink, kind, chunk):
+    """Scores that leave what came before far behind, with values of 2^40: a weight may be large against what is kept of a row, but not so large."""
+    D, T = 64, 1000
+    g = torch.Generator().manual_seed(chunk + int(softcap) + len(kind))
+    key = torch.arange(T) % (chunk or T)
+    lead = torch.where(key < 128 if not chunk else key < 1, -150.0, 150.0) if kind == "jump" else -130.0 + 20.0 * (torch.arange(T) // 64)
+    k = torch.randn(T, G, D, generator=g)
+    k[:, :, 0] = lead[:, None]
+    v = torch.randn(T, G, D, generator=g) * 2.0 ** 40
+    q = torch.randn(T, H, D, generator=g)
+    q[:, :, 0] = 8.0 * (0.5 + torch.rand(T, H, generator=g)) * torch.where(torch.rand(T, H, generator=g) < 0.25, -1.0, 1.0)
+    k, v, q = (t.to(torch.bfloat16) for t in (k, v, q))
+    nb = -(-T // BS)
+    kc, vc = (torch.zeros(nb + 1, BS, G, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    kc[1:].view(-1, G, D)[:T] = k.to(DEV)
+    vc[1:].view(-1, G, D)[:T] = v.to(DEV)
+    step = StepBatch.host([[0] * T], [0], [list(range(1, nb + 1))], [0], nb, BS).to(DEV)
+    sinks = None if sink is None else torch.full((H,), sink, device=DEV)
+    desc = _lib.AttentionDesc(heads=H, kv_heads=G, dim=D, vdim=D, chunk=chunk, scale=D ** -0.5, softcap=softcap,
+                              sink=None if sinks is None else sinks.data_ptr(), out_scale=1.0)
+    out = torch.empty(T, H * D, dtype=torch.bfloat16, device=DEV)
+    ops.chunk_attention(q.to(DEV).view(T, H * D), kc, vc, out, desc, step)
+    k, v, q = (t.to(DEV).double() for t in (k, v, q))
+    s = torch.einsum("ihd,jhd->hij", q, k.repeat_interleave(H // G, 1)) * D ** -0.5
+    s = softcap * torch.tanh(s / softcap) if softcap else s
+    i, j = torch.arange(T, device=DEV)[:, None], torch.arange(T, device=DEV)[None, :]
+    s = s.masked_fill((j > i) | ((i // chunk != j // chunk) if chunk else False), -math.inf)
+    m = s.amax(-1, keepdim=True)
+    m = m if sink is None else m.clamp(min=sink)
+    p = (s - m).exp()
+    w = p / (p.sum(-1, keepdim=True) + (0.0 if sink is None else (sink - m).exp()))
+    ref, size = (torch.einsum("hij,jhd->ihd", w, t.repeat_interleave(H // G, 1)) for t in (v, v.abs()))
+    got = out.view(T, H, D).double()
+    # as above; beside a sink far above them all weights may vanish
+    bound = 2.0 ** -8 * ref.abs() + (2.0 ** -8 + 2e-4) * size + 2.0 ** 40 * 1e-37
+    assert bool(((got - ref).abs() <= bound).all()), float(((got - ref).abs() / bound).nan_to_num(math.inf).max())
