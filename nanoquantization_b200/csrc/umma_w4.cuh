@@ -90,7 +90,8 @@ template <bool BF16> __device__ __forceinline__ uint32_t silu_mul2(uint32_t gw, 
   const uint64_t p = fma_f2(fma_f2(q, pack_f2(-d0, -d1), g), r, q);
   asm("mov.b64 {%0, %1}, %2;" : "=f"(q0), "=f"(q1) : "l"(q));
   asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(p));
-  const float s0 = p0 == p0 ? p0 : q0, s1 = p1 == p1 ? p1 : q1;   // (an infinite gate or divisor has no remainder)
+  // an infinite gate or divisor has no remainder, and that of -0 would take its sign
+  const float s0 = p0 == p0 && q0 != 0.f ? p0 : q0, s1 = p1 == p1 && q1 != 0.f ? p1 : q1;
   return mul2<BF16>(round2<BF16>(s0, s1), uw);
 }
 

@@ -89,7 +89,7 @@ def test_gate_up_silu_of_prompts_is_the_separate_steps(M, K, N, dtype, bias):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_gate_up_silu_of_every_gate(dtype):
-    """All 65536 patterns of a gate, as the bias of columns whose weights are zero."""
+    """Every gate but -0, as the bias of columns whose weights are zero."""
     M, K, N = 512, 256, 131072
     assert _lib.load().nqb200_gemm_gate_up_silu_supported(M, N, K, 128, 0 if dtype == torch.float16 else 1) == 1
     m = nq.WQLinear_GEMM(4, 128, K, N, DEV, True, dtype)
@@ -100,4 +100,24 @@ def test_gate_up_silu_of_every_gate(dtype):
         m.bias.copy_(torch.cat([gates, torch.full_like(gates, up)]))
         want = fused.silu_mul(m(x))
         assert torch.equal(in_one_call(m, x).view(torch.int16), want.view(torch.int16))
+    _lib.check_workspaces()
+
+
+@pytest.mark.parametrize("dtype,scale,x_value", [(torch.float16, 2.0 ** -24, 2.0 ** -12), (torch.bfloat16, 2.0 ** -60, 2.0 ** -86)])
+def test_gate_up_silu_of_minus_zero(dtype, scale, x_value):
+    """Negative sums that vanish when they are rounded: the gate is -0, and so is what comes of it."""
+    M, K, N = 512, 256, 51200
+    assert _lib.load().nqb200_gemm_gate_up_silu_supported(M, N, K, 128, 0 if dtype == torch.float16 else 1) == 1
+    m = nq.WQLinear_GEMM(4, 128, K, N, DEV, False, dtype)
+    half = N // 2
+    m.qzeros[:, :half // 8] = 0x11111111                               # weights of the gate: 0 - 1
+    m.qweight[:, half // 8:] = 0x11111111                              # of the other half: 1 - 0
+    m.qscales[:, :half] = scale
+    m.qscales[:, half:] = 1.0
+    x = torch.full((M, K), x_value, device=DEV, dtype=dtype)
+    y = m(x)
+    assert bool((y[:, :half].view(torch.int16) == -2 ** 15).all()) and bool((y[:, half:] > 0).all())
+    got, want = in_one_call(m, x), fused.silu_mul(y)
+    assert bool((want.view(torch.int16) == -2 ** 15).all())
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     _lib.check_workspaces()
