@@ -61,27 +61,6 @@ struct Params {
   int* status;
 };
 
-constexpr uint32_t kSuspendNs = 20000;
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  const uint32_t b = smem_u32(bar);
-  if (mbar_test_wait(b, parity)) return true;
-  unsigned long long t0 = 0;      // the clock is read only after a suspension that ran out
-  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
-    if (*abort_flag) return false;
-    const unsigned long long t = global_timer_ns();
-    if (!t0) t0 = t;
-    if (t - t0 > kWaitLimitNs) {
-      *abort_flag = 1;
-      if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
-      return false;
-    }
-  }
-  return true;
-}
-// The same, and a test, for a whole warp whose lanes go on together (the votes keep its control flow uniform, see elect_one).
-__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  return __all_sync(0xFFFFFFFFu, wait_bar(bar, parity, abort_flag, status));
-}
 // The issuers' waits poll: a suspended warp is woken late, and the tensor pipe has nothing queued meanwhile.
 __device__ __forceinline__ bool poll_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   const uint32_t b = smem_u32(bar);

@@ -42,27 +42,6 @@ struct Params {
   int* status;
 };
 
-constexpr uint32_t kSuspendNs = 20000;
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  const uint32_t b = smem_u32(bar);
-  if (mbar_test_wait(b, parity)) return true;
-  unsigned long long t0 = 0;      // the clock is read only after a suspension that ran out
-  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
-    if (*abort_flag) return false;
-    const unsigned long long t = global_timer_ns();
-    if (!t0) t0 = t;
-    if (t - t0 > kWaitLimitNs) {
-      *abort_flag = 1;
-      if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
-      return false;
-    }
-  }
-  return true;
-}
-// The same for a whole warp, whose lanes go on together (the vote keeps its control flow uniform, see elect_one).
-__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  return __all_sync(0xFFFFFFFFu, wait_bar(bar, parity, abort_flag, status));
-}
 // One arrival on the barrier at this offset in both CTAs when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void commit_both(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"

@@ -1,7 +1,9 @@
 // tcgen05 / tensor-memory helpers (sm_100a): allocation, register<->TMEM moves,
-// the MMA itself, commit and the fences that order them against mbarriers.
+// the MMA itself, commit, the fences that order them against mbarriers, and the bounded waits of the kernels' roles.
 #pragma once
 #include <stdint.h>
+#include "nqb200.h"
+#include "tma_utils.cuh"
 
 namespace nqb200 {
 
@@ -59,6 +61,30 @@ __device__ __forceinline__ bool elect_one() {
 }
 // The warp's index, known to be the same in all its lanes.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// A wait suspends in hardware for up to kSuspendNs at a time (woken at once when the phase completes), so that warps which
+// wait most of the time hardly issue; the clock is read only after a suspension that ran out.
+constexpr uint32_t kSuspendNs = 20000;
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  const uint32_t b = smem_u32(bar);
+  if (mbar_test_wait(b, parity)) return true;
+  unsigned long long t0 = 0;
+  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
+    if (*abort_flag) return false;
+    const unsigned long long t = global_timer_ns();
+    if (!t0) t0 = t;
+    if (t - t0 > kWaitLimitNs) {
+      *abort_flag = 1;
+      if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
+      return false;
+    }
+  }
+  return true;
+}
+// The same for a whole warp, whose lanes go on together (the vote keeps its control flow uniform, see elect_one).
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status));
+}
 
 // 16 lanes x 128 bits, twice: thread (g = lane/4, t = lane%4) supplies
 //   r0 -> (lane g, column t)   r1 -> (lane g+8, column t)   r2 -> (lane g, column t+4)   r3 -> (lane g+8, column t+4)

@@ -7,30 +7,6 @@
 
 namespace nqb200 {
 
-// A wait suspends in hardware for up to kSuspendNs at a time (woken at once when the phase completes), so that warps which
-// wait most of the time hardly issue; the clock is read only after a suspension that ran out.
-constexpr uint32_t kSuspendNs = 20000;
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  const uint32_t b = smem_u32(bar);
-  if (mbar_test_wait(b, parity)) return true;
-  unsigned long long t0 = 0;
-  while (!mbar_try_wait_suspend(b, parity, kSuspendNs)) {
-    if (*abort_flag) return false;
-    const unsigned long long t = global_timer_ns();
-    if (!t0) t0 = t;
-    if (t - t0 > kWaitLimitNs) {
-      *abort_flag = 1;
-      if (status) atomicExch(status, NQB200_ERR_WAIT_TIMEOUT);
-      return false;
-    }
-  }
-  return true;
-}
-// The same for a whole warp, whose lanes go on together (the vote keeps its control flow uniform, see elect_one).
-__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status));
-}
-
 template <bool BF16> __device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
   uint32_t r;
   if (BF16) asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
