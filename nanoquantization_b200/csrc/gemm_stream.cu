@@ -10,9 +10,9 @@
 //                   128-byte swizzle, the group's scales and zero-points),
 //                   completion on an mbarrier.  About 190 KB per SM is in flight
 //                   from the first cycle, which is what keeps HBM busy at these
-//                   sizes.  It reads nothing another kernel writes, so under
-//                   programmatic stream serialisation it starts before the
-//                   kernel ahead of it has finished.
+//                   sizes.  What it reads is settled by then (nqb200.h asks
+//                   callers for that), so under programmatic stream serialisation
+//                   it starts before the kernel ahead of it has finished.
 //   activation warp, or two : the group's 128 k of every token by plain loads into the
 //                   stage (swizzled like a TMA tile), and their sum per token
 //                   (the tensor pipe is this kernel's scarce resource, so the sum

@@ -672,9 +672,10 @@ static int launch_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensor
 
 bool umma_pair_supports(int64_t M, int64_t N, int64_t K, int64_t g) {
   if (!(M > 128 && g == 128 && K % 128 == 0 && N % 32 == 0)) return false;
-  // Against the single-CTA kernel: its own cost model's estimate for the shape, less the 10 us by which this
-  // kernel's fixed cost (cluster launch, tensor-memory allocation for a pair, a deeper pipeline to fill) exceeds
-  // that kernel's.  Fitted with tiles of 256 tokens on M in 192..4096 x the sweep's five shapes.
+  // Against the single-CTA kernel: an estimate made for an earlier form of it, less the 10 us by which this
+  // kernel's fixed cost (cluster launch, tensor-memory allocation for a pair, a deeper pipeline to fill) exceeded
+  // that one's.  Fitted with tiles of 256 tokens on M in 192..4096 x the sweep's five shapes; both kernels have become faster since, and
+  // where between 129 and about 400 tokens the line lies now has not been measured.
   const pair::Plan pl = pair::make_plan(M, N, K);
   if ((pl.U + 1) * pl.nclusters >= (1ll << 31)) return false;   // the kernel's 32-bit unit arithmetic
   return pl.est_us <= umma_prefill_estimate_us(M, N, K) - 10.0;

@@ -39,12 +39,6 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// D[tmem] (+)= A[tmem] * B[smem descriptor]; one thread issues it for the CTA.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-               " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-               ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // The mbarrier receives one arrival when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -52,8 +46,8 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 
 // True in one lane of a converged warp.  What issues tensor-core and TMA instructions runs as a whole warp through control flow
 // that is the same for all lanes (warp_index(), votes on the waits) and puts only the instruction itself under this: its operands
-// then live in uniform registers.  Under "if (lane == 0)" the compiler has to move every operand there for every instruction:
-// measured 46 to 98 cycles from one 128 x 48 x 16 MMA to the next instead of the tensor pipe's 24, and 370 between TMA instructions.
+// then live in uniform registers, where under "if (lane == 0)" every operand has to be moved there for every instruction.  Two-SM
+// prefill kernel, 777 tokens of 12288 -> 4096 79 -> 68 us; experts' grouped GEMM 497 -> 447; prompt attention 647 -> 575.
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
@@ -123,19 +117,14 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// M = 256: 128 rows of A and D in each CTA's tensor memory; B is N x K with N/2 rows in each CTA's shared memory.
-__device__ __forceinline__ void umma_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-               " tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}"
-               ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // `bar` is a shared::cluster address: the barrier may live in either CTA of the pair.
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// The MMAs with the 64-bit shared-memory descriptor given as its two halves (the high half is constant for
-// a kernel, the low half is a base plus an offset: one 32-bit add per MMA for the issuing thread).
+// D[tmem] (+)= A[tmem] * B[smem descriptor], issued by one thread for the CTA, or for a pair: M = 256, 128 rows of A and D in each
+// CTA's tensor memory, B is N x K with N/2 rows in each CTA's shared memory.  The 64-bit shared-memory descriptor comes as its two halves
+// (the high half is constant for a kernel, the low half is a base plus an offset: one 32-bit add per MMA for the issuing thread).
 __device__ __forceinline__ void umma_ts_lohi(uint32_t d_tmem, uint32_t a_tmem, uint32_t desc_lo, uint32_t desc_hi, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile("{\n .reg .pred p;\n .reg .b64 d;\n setp.ne.b32 p, %5, 0;\n mov.b64 d, {%2, %3};\n"

@@ -1,5 +1,5 @@
-// What the tcgen05 kernels of the packed linears share: bounded waits, the arithmetic that turns packed words into 16-bit
-// weights, and the dealing of units to CTAs.
+// Arithmetic that the kernels of the packed linears share: packed words to 16-bit weights, pairs of 16-bit numbers, silu(gate) * up,
+// and the order of columns in tensor memory.
 #pragma once
 #include "common.cuh"
 #include "tma_utils.cuh"
@@ -30,8 +30,8 @@ __device__ __forceinline__ uint32_t fma2_f16(uint32_t a, uint32_t b, uint32_t c)
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
   return r;
 }
-// (a & mask) | bits as one instruction: with mask and bits in registers.  (The instruction has room for one immediate, and
-// with both as constants the compiler makes two of it.)
+// (a & mask) | bits, with mask and bits in registers: one instruction.  (Written with both as constants 777 tokens of 12288 -> 4096 took 101.9
+// us instead of 100.5, and 4096 of 5120 -> 25600 829 instead of 825.)
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
   uint32_t r;
   asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
