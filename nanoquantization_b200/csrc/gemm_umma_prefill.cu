@@ -21,7 +21,9 @@
 //
 //   warp 0        TMA of the packed weights: 128 x 128 bytes per unit.  Before the wait for the kernel ahead on the stream the
 //                 first ones are brought into the L2 cache, which is all that may be done then: that kernel may have written them.
-//                 (42 calls of 17 to 128 tokens in chains: 0.976 of the time that copies into shared memory at that point take.)
+//                 Up to 64 tokens a tile the whole ring, beyond it four units: 42 calls of 17 to 128 tokens in chains take 0.98 of the
+//                 time that copies into shared memory at that point took (1.006 without any, 0.994 with two, 0.986 with four).  The whole
+//                 ring also beyond 64 would keep a call's first copies waiting on an idle stream: 100 tokens of 4096 -> 12288 20.0 -> 20.3 us.
 //   warp 2        TMA of the activations: one box of both 64-k halves per unit.
 //   warp 1        MMA issuer: per half unit and k-step two MMAs (one per A block) of M 128, N tokens, K 16.
 //   warps 3-18    dequantisers, two sets of 8 taking alternate units; a slot of the A operand holds half a unit.  Scales and
@@ -41,6 +43,7 @@ constexpr int kDequantWarps = 16, kEpiWarps = 8, kFirstDequant = 3, kFirstEpi = 
 constexpr int kThreads = (kFirstEpi + kEpiWarps) * 32;
 constexpr int kWStageBytes = 16384;
 constexpr int kMaxW = 8, kMaxX = 4, kMaxA = 6;
+constexpr int kAhead = 4;        // units whose weights are brought into L2 ahead of the dependency wait, beyond 64 tokens a tile
 constexpr int kSmemBudget = 220 * 1024;
 constexpr int kTmemCols = 512;
 
@@ -166,7 +169,7 @@ umma_prefill_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     }
     __syncwarp();
     Place ahead = at;
-    for (int i = 0; i < p.sw && i < nunits; ++i) {
+    for (int i = 0; i < (p.nt <= 64 ? p.sw : kAhead) && i < nunits; ++i) {
       if (el) tma_prefetch_2d(&tm_w, ahead.tn * 32, ahead.g * kUnitK);
       ahead.next(p);
     }
