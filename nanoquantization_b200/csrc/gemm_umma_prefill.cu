@@ -6,9 +6,9 @@
 // Measured in chains of calls (bf16, microseconds): 4096 x 24576 34.9 -> 25.2 at 48 tokens and 38.2 -> 34.7 at 128, 12288 x 4096
 // 19.7 -> 17.1 at 48, against the form before this one (issuing threads of their own, whole tiles or an even
 // split of K, the epilogue's stores two bytes wide); 1.21 in the mean over 91 calls of 17 to 400 tokens, before the prefetch at
-// warp 0.  A unit takes 0.71 us at 17 tokens, 0.73 at 48 and 0.87 at 128, where memory needs 0.39: what bounds it hardly depends on the
-// tokens, which leaves the dequantisers (not shown by counters).  Two blocks per SM, each half as
-// large, reach the same rate.  Clusters that add their parts through distributed shared memory instead of a second kernel were
+// warp 0.  A unit takes 0.71 us at 17 tokens, 0.73 at 48 and 0.87 at 128, where memory needs 0.39.  No pipe is full (ncu,
+// 48 tokens of 4096 x 24576: issue slots 53 % of active cycles, ALU 35, FMA 33, tensor 21, DRAM 25): it is the chain from weights to
+// MMAs with its fill and drain.  Two blocks per SM, each half as large, reach the same rate.  Clusters that add their parts through distributed shared memory instead of a second kernel were
 // slower (48 tokens, 4096 x 6144 13.1, 4096 x 24576 29.0): fewer of them fit, and the exchange took 2 us.
 //
 // The weights are the 128-row A operand, dequantised to their true 16-bit values (q - z) * s -- the integer difference first,
