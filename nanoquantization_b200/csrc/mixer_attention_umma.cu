@@ -9,9 +9,9 @@
 // Tensor memory holds S of both tiles (two halves of 64 columns each) and O of both; P overwrites the first half of its own S.
 // So four chains S -> weights -> O += P V -> next S run beside each other, and a scheduler has a warp of each.  What bounds it:
 // per 256 x 128 scores the tensor pipe needs 2560 cycles (S 48 per MMA of N = 64, which shared memory sets, O 64), the
-// exponentials 2048, and about 4600 pass, because the chains meet at the pipes.  8192 tokens of 32 heads of 128, us, in turns against
-// whole tiles with one softmax thread per row and one polling issuer: chunks of 4096 626 -> 406, one chunk 1087 -> 679, scores beyond
-// the cap 2667 -> 1678, no cap 931 -> 611, sigmoid weights 959 -> 624.  An own warp for S beside the two for O, polling instead of
+// exponentials 2048, and about 4500 pass, because the chains meet at the pipes.  8192 tokens of 32 heads of 128, us, in turns against
+// whole tiles with one softmax thread per row and one polling issuer: chunks of 4096 645 -> 400, one chunk 1093 -> 673, scores beyond
+// the cap 2673 -> 1590, no cap 932 -> 589, sigmoid weights 963 -> 624.  An own warp for S beside the two for O, polling instead of
 // suspended softmax waits and query tiles started apart gained nothing.
 //
 // The weights are 2^(score - m).  m is the largest score of the tile that a row begins in, or the sink, and follows the largest score
@@ -20,14 +20,15 @@
 // what whole tiles with a lag of 8 had; smaller lags take off up to 5 % more of it and cost 2 to 3 % each where scores spread by 6 log2 units.)
 // A half finds out by itself that its scores ask for no move, from the largest magnitude, which the choice below needs as well; that
 // the other half has not moved it learns from what that one hands on, in the order of the products, and does not wait for the other's
-// scores: 940 -> 679 us with a cap of 120, against halves that compare their maxima in every tile.  Of the 679 the hand-over takes 65.
+// scores: 955 -> 671 us with a cap of 120, against halves that compare their maxima in every tile.  Of the 673 the hand-over takes 65.
 // (A reference that never moves, which a cap of 50 allows, needs neither, but its weights reach 2^100 and more values overflow, and the
 // largest weight of a row is rounded where it could be a power of two: up to 11 % more error.)  The cap is monotonic, so the
 // maximum is taken over raw scores.
 // For scores well inside the cap tanh is its Taylor series, which costs fused multiply-adds on register pairs only: three terms
 // up to a tenth of the cap, where what they leave out (0.054 y^6) is below float's rounding, five terms beyond; up to
 // twice the cap it is the seventh convergent of Lambert's continued fraction (one reciprocal more per score); a warp
-// whose half tile has a larger score, or needs a mask, takes the general path.
+// whose half tile has a larger score, or needs a mask, takes the general path, of which there is one with and one without a cap (as one,
+// the cap's exponential and reciprocal are computed either way: 128 tokens without a cap 9.7 us instead of 8.3, 600 19.4 instead of 17.7).
 //
 // The sum that a row is divided by takes the weights in float32, before the product's rounding to bf16.
 //
@@ -443,17 +444,13 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             for (int e = 0; e < 32; e += 2) hi[(e >> 1) & 3] = max3(hi[(e >> 1) & 3], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
           mx = fmaxf(fmaxf(hi[0], hi[1]), fmaxf(hi[2], hi[3]));
         } else {
-#pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t v[16];
-            tmem_ld_32x32b_x16(tS + c * 16, v);
-            tc_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int key = key0 + c * 16 + e;
-              mx = (key <= pos && key >= lo) ? fmaxf(mx, __uint_as_float(v[e])) : mx;
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              const int key = key0 + c * 32 + e;
+              mx = (key <= pos && key >= lo) ? fmaxf(mx, __uint_as_float(r[c][e])) : mx;
             }
-          }
         }
         if (joint) {
           float mo;
@@ -520,24 +517,28 @@ attention_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         else weights(std::integral_constant<int, 4>(), r, nm2);
       } else {
         // from tensor memory again, a piece at a time: compact code for the few tiles at the edges
+        auto general = [&](auto cap) {
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t v[16], w[8];
-          tmem_ld_32x32b_x16(tS + c * 16, v);
-          tc_wait_ld();
+          for (int c = 0; c < 4; ++c) {
+            uint32_t v[16], w[8];
+            tmem_ld_32x32b_x16(tS + c * 16, v);
+            tc_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            float x[2];
+            for (int e = 0; e < 8; ++e) {
+              float x[2];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int key = key0 + c * 16 + 2 * e + u;
-              x[u] = (key <= pos && key >= lo) ? ex2(score(__uint_as_float(v[2 * e + u])) - mu) : 0.f;
+              for (int u = 0; u < 2; ++u) {
+                const int key = key0 + c * 16 + 2 * e + u;
+                const float s = __uint_as_float(v[2 * e + u]) * p.ysc;
+                x[u] = (key <= pos && key >= lo) ? ex2(p.top * (decltype(cap)::value ? tanh_fast(s) : s) - mu) : 0.f;
+              }
+              w[e] = pack_bf16(x[0], x[1]);
+              lsum = add2(lsum, pair2(x[0], x[1]));
             }
-            w[e] = pack_bf16(x[0], x[1]);
-            lsum = add2(lsum, pair2(x[0], x[1]));
+            tmem_st8(tS + c * 8, w);      // lies behind what has been read of S
           }
-          tmem_st8(tS + c * 8, w);      // lies behind what has been read of S
-        }
+        };
+        if (capped) general(std::true_type()); else general(std::false_type());
       }
       done();
     }
